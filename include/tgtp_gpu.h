@@ -239,7 +239,8 @@ tgtp_status saba_count_static(const uint32_t* device_idx, const uint32_t* device
  * every slot iterates until its residual norm is at most tol * ||e_u - e_v|| (TGTP_ERR_TIMEOUT when
  * max_iter iterations do not get there).  host_iterations (may be NULL) receives the iteration count
  * of each batch of 32 slots (ceil(count / 32) entries).  Synchronous; scratch is allocated per call
- * (5 blocks of n x 32 doubles). */
+ * (four blocks of n x 32 doubles per batch;
+ * several batches run side by side while their blocks stay within 80 MB). */
 tgtp_status tgtp_exact_sc_slots(tgtp_graph* g, const uint32_t* host_slots, uint32_t count,
                                 double tol, uint32_t max_iter, double* host_resistance,
                                 uint32_t* host_iterations);

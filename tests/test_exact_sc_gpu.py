@@ -71,6 +71,34 @@ def test_exact_sc_of_a_self_loop_slot_is_zero_and_repeats_count_once(cuda_device
     assert got[10] == 0.0 and got[11] == 0.0
 
 
+@pytest.mark.parametrize("hub", [63, 64, 65, 128, 129, 700])
+def test_exact_sc_of_rows_at_the_edges_of_a_segment(cuda_device, hub):
+    """Rows of more than 64 slots are added up in segments of 64: a hub joined to every vertex of
+    a ring, the edges to ring vertices 61 .. 64 listed twice (so one repeat lies on slots 63 and 64
+    of the hub's row), a count that is no multiple of the 32 slots of a batch.  The dense oracle solves
+    the same systems in FP64; both are within the conjugate gradients' tolerance (1e-12 of
+    sqrt(2)) times the condition number of the ring with a hub (below 10^3)."""
+    from oracle import exact_sc
+    from tgtp_b200.aesc import AESCGraph, exact_sc_slots
+
+    ring = np.arange(hub)
+    twice = ring[61:65]
+    u = np.concatenate([ring, ring, twice])
+    v = np.concatenate([(ring + 1) % hub, np.full(hub, hub), np.full(len(twice), hub)])
+    src, dst = np.concatenate([u, v]), np.concatenate([v, u])
+    order = np.lexsort((dst, src))
+    idx = np.zeros(hub + 2, np.uint32)
+    idx[1:] = np.cumsum(np.bincount(src, minlength=hub + 1))
+    adj = dst[order].astype(np.uint32)
+    want = exact_sc.exact_scores(idx, adj)
+    slots = np.arange(0, len(adj), 3, dtype=np.uint32)
+    g = AESCGraph.from_csr(idx, adj)
+    got, iters = exact_sc_slots(g, slots, tol=1e-12)
+    g.free()
+    assert np.max(np.abs(got - want[slots])) < 1e-9
+    assert len(iters) == -(-len(slots) // 32) and np.all(iters % 8 == 0)
+
+
 def _within_eps_fractions(g, eps, slots, exact):
     """Fraction of the sampled slots within eps of the exact value, FP64 and mixed (BF16) forms."""
     from tgtp_b200 import eigenprep_gpu
