@@ -3372,8 +3372,8 @@ void launch(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, 
     TGTP_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
 }
 
-// Resident blocks per SM of a kernel at a block size and dynamic shared memory, cached; the kernel's
-// dynamic shared-memory limit is raised to the largest size asked for so far.
+}  // namespace
+
 int blocks_per_sm(const void* kern, int threads, size_t smem) {
     static std::mutex mu;
     static std::map<std::tuple<const void*, int, size_t, int>, int> cache;
@@ -3393,6 +3393,8 @@ int blocks_per_sm(const void* kern, int threads, size_t smem) {
     cache[key] = per_sm;
     return per_sm;
 }
+
+namespace {
 
 // Symmetrisation of one run (stage 3) on the graph's stream.
 template <class Real, class Acc>

@@ -649,9 +649,7 @@ tgtp_status saba_count(tgtp_graph* g, uint32_t depth, uint32_t n_walks, uint32_t
         auto* c = g->counters.as<uint32_t>();
         saba_run(g, depth, n_walks, c);
         uint64_t sums[3];
-        saba_summarize(g, c, sums);
-        if (host_counters)
-            TGTP_CUDA(cudaMemcpy(host_counters, c, sizeof(uint32_t) * g->n, cudaMemcpyDeviceToHost));
+        saba_summarize(g, c, host_counters, sums);
         if (out) {
             out->visit_count = sums[0];
             out->checksum = sums[1];
@@ -673,9 +671,7 @@ tgtp_status mt_walk_count(tgtp_graph* g, uint32_t depth, uint32_t n_walks, int32
         auto* c = g->counters.as<uint32_t>();
         mt_walk_run(g, depth, n_walks, simd != 0, c);
         uint64_t sums[3];
-        saba_summarize(g, c, sums);
-        if (host_counters)
-            TGTP_CUDA(cudaMemcpy(host_counters, c, sizeof(uint32_t) * g->n, cudaMemcpyDeviceToHost));
+        saba_summarize(g, c, host_counters, sums);
         if (out) {
             out->visit_count = sums[0];
             out->checksum = sums[1];

@@ -200,15 +200,15 @@ struct tgtp_graph {
     tgtp::DeviceBuffer block_bits;   // the block push's row masks when they do not fit in smem
     tgtp::DeviceBuffer block_lists;  // the block push's row lists (four of n entries per CTA)
     tgtp::DeviceBuffer walk_queue, walk_ctl;  // the block push's walk items; per wave length, claim
-    // walk copy of the graph renumbered by degree (built on the first saba_count)
-    tgtp::DeviceBuffer saba_info, saba_adj, saba_cnt;
-    bool saba_ready = false;
-    // the same copy with each slot holding its target's row record (16 bytes per slot; built on
-    // the first saba_count that walks the inlined copy)
-    tgtp::DeviceBuffer saba_adj16;
-    bool saba_inline_ready = false;
+    // walk copies of the graph renumbered by degree (built on the first walk that needs them): the
+    // row records, the inverse numbering, the degree class of every number and the class table;
+    // the plain adjacency; the packed one (8 bytes per slot)
+    tgtp::DeviceBuffer saba_info, saba_inv, saba_cls, saba_classes, saba_adj, saba_packed;
+    uint32_t saba_ncls = 0;
+    tgtp::DeviceBuffer mt_seeds;  // per warp of the MT19937 walks: the states of its next sources
+    bool saba_ready = false, saba_plain_ready = false, saba_packed_ready = false;
     // the walk layout saba_tune chose: walkers per lane (low byte: 1, 2 or 4, so 4, 8 or 16
-    // bouquets per warp) and 0x100 for the inlined copy; 0 = not tuned
+    // bouquets per warp) and 0x100 for the packed copy; 0 = not tuned
     uint16_t saba_choice = 0;
     int32_t last_precision = -1;
     bool have_run = false;
@@ -220,10 +220,44 @@ struct tgtp_graph {
 
 namespace tgtp {
 void saba_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, uint32_t* device_counters);
-// Times the walk layouts (walkers per lane 1 / 2 / 4, plain or inlined copy) for this graph and
+// Times the walk layouts (walkers per lane 1 / 2 / 4, plain or packed copy) for this graph and
 // walk configuration, `trials` runs each after a warm-up, and keeps the fastest on the handle.
 int saba_tune(tgtp_graph* g, uint32_t depth, uint32_t n_walks, int trials);
-void saba_summarize(tgtp_graph* g, const uint32_t* device_counters, uint64_t* host_sums3);
+// The packed walk copy (saba.cu): slot q of the degree-renumbered adjacency holds
+// (p | class(p) << pbits, fmix32(original id of p)); row p starts at class.x + p * class.y and has
+// class.y slots.
+struct PackedWalk {
+    const uint2* slots;    // m
+    const uint2* classes;  // ncls
+    const uint4* info;     // row records: (row start, degree, original id, 0)
+    uint32_t ncls, pbits;
+};
+constexpr uint32_t kMaxClasses = 4096;
+void saba_prepare(tgtp_graph* g);
+void saba_prepare_plain(tgtp_graph* g);
+bool saba_packable(const tgtp_graph* g);
+PackedWalk saba_prepare_packed(tgtp_graph* g);
+// Visit counters of the renumbered vertices in global memory.  Numbers are in order of degree, so
+// neighbouring numbers take visits at similar rates and the first ones the most: sectors of eight
+// counters are dealt out to 64 runs of the array, so that the busy ones spread over the L2 slices.
+struct WalkCounters {
+    uint32_t* words;  // 64 * len
+    uint32_t len;     // words per run: 8 * ceil(n / 512)
+    __device__ __forceinline__ uint32_t* at(uint32_t p) const {
+        return words + size_t((p >> 3) & 63u) * len + ((p >> 9) << 3) + (p & 7u);
+    }
+};
+// Zeroed counters (and the sums saba_summarize reads); then, back to the original ids, into
+// device_counters.
+WalkCounters walk_counters(tgtp_graph* g);
+void scatter_counters(tgtp_graph* g, WalkCounters cnt, uint32_t* device_counters);
+// The run's sums (visit count, checksum, fallback bouquets) and, if asked, its counters on the
+// host; synchronises the stream.
+void saba_summarize(tgtp_graph* g, const uint32_t* device_counters, uint32_t* host_counters,
+                    uint64_t* host_sums3);
+// Resident blocks per SM of a kernel at a block size and dynamic shared memory, cached; the kernel's
+// dynamic shared-memory limit is raised to the largest size asked for so far.
+int blocks_per_sm(const void* kern, int threads, size_t smem);
 // The reference's MT19937 walk baselines (scalar or 8-lane bouquet draw order) into
 // device_counters (n uint32), asynchronous; the sums of saba_summarize then describe them.
 void mt_walk_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, bool simd, uint32_t* device_counters);

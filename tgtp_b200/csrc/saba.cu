@@ -28,6 +28,14 @@ namespace tgtp {
 namespace {
 
 constexpr int kSabaThreads = 512;
+// Walk over the packed copy: one block of 1,024 threads shares one set of counters.  What a walk is
+// short of is L1 lines for its loads in flight (L1 and shared memory share 256 KB per SM) and L2
+// atomics for the counters outside shared memory, so the counters take what leaves L1 about 100 KB.
+// R-MAT scale 18, D 10, W 2,048: 12,288 counters per 512-thread block 20.6 ms; per 1,024-thread block
+// 24,576 / 32,768 / 36,864 / 40,960 / 49,152 counters 15.8 / 14.9 / 14.6 / 14.8 / 25 ms (the last
+// leaves L1 too small); Chung-Lu n = 10^6, D 10, W 256: 28.3 / 26.9 / 26.6 / 29.4 / 58 ms.
+constexpr int kPackedThreads = 1024;
+constexpr uint32_t kPackedHotCap = 36864;
 constexpr uint32_t kSabaHotCap = 12288;  // 48 KiB of shared counters per block
 
 __global__ void __launch_bounds__(kSabaThreads)
@@ -123,12 +131,14 @@ __global__ void saba_iota_kernel(uint32_t* __restrict__ ids, uint64_t n) {
 
 __global__ void saba_info_kernel(const uint32_t* __restrict__ order, const uint32_t* __restrict__ sdeg,
                                  const uint32_t* __restrict__ beg, uint64_t n,
-                                 uint4* __restrict__ info, uint32_t* __restrict__ inv) {
+                                 uint4* __restrict__ info, uint32_t* __restrict__ inv,
+                                 uint32_t* __restrict__ flag) {
     for (uint64_t p = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
          p += uint64_t(gridDim.x) * blockDim.x) {
         const uint32_t old = order[p];
         info[p] = make_uint4(beg[p], sdeg[p], old, 0u);
         inv[old] = uint32_t(p);
+        flag[p] = p > 0 && sdeg[p] != sdeg[p - 1];  // a new degree class starts here
     }
 }
 
@@ -144,11 +154,28 @@ __global__ void saba_adj_kernel(const uint32_t* __restrict__ idx, const uint32_t
     }
 }
 
-__global__ void saba_scatter_kernel(const uint32_t* __restrict__ cnt, const uint4* __restrict__ info,
-                                    uint64_t n, uint32_t* __restrict__ counters) {
+// Counters back to the original ids, with visit_count = sum c[v] and checksum = sum (v + 1) c[v]
+// (both exact in 64 bits) added up on the way.
+__global__ void saba_scatter_kernel(const WalkCounters cnt, const uint4* __restrict__ info,
+                                    uint64_t n, uint32_t* __restrict__ counters,
+                                    unsigned long long* __restrict__ sums) {
+    unsigned long long s0 = 0, s1 = 0;
     for (uint64_t p = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
-         p += uint64_t(gridDim.x) * blockDim.x)
-        counters[info[p].z] = cnt[p];
+         p += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t v = info[p].z, c = *cnt.at(uint32_t(p));
+        counters[v] = c;
+        s0 += c;
+        s1 += uint64_t(c) * (uint64_t(v) + 1);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        s0 += __shfl_xor_sync(kFullMask, s0, o);
+        s1 += __shfl_xor_sync(kFullMask, s1, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(sums + 0, s0);
+        atomicAdd(sums + 1, s1);
+    }
 }
 
 // The walk on the renumbered graph.  Each lane carries WPL walkers (bouquets 4w + g of the warp's
@@ -163,7 +190,7 @@ template <int WPL>
 __global__ void __launch_bounds__(kSabaThreads)
 saba_walk_perm_kernel(const uint4* __restrict__ info, const uint32_t* __restrict__ adjp,
                       uint32_t depth, uint32_t bouquets_per_src, uint32_t grid_step,
-                      uint64_t total_bouquets, uint32_t* __restrict__ cnt, uint32_t hot,
+                      uint64_t total_bouquets, WalkCounters cnt, uint32_t hot,
                       uint32_t hot_rec, unsigned long long* __restrict__ fallback_total) {
     // the records as three arrays (row start, degree, original id: 12 bytes a vertex), then the
     // counters
@@ -251,7 +278,7 @@ saba_walk_perm_kernel(const uint4* __restrict__ info, const uint32_t* __restrict
                         orig[w] = r.z;
                     }
                     if (nxt[w] < hot) atomicAdd(s_cnt + nxt[w], 1u);
-                    else atomicAdd(cnt + nxt[w], 1u);
+                    else atomicAdd(cnt.at(nxt[w]), 1u);
                 }
             }
         }
@@ -269,7 +296,7 @@ saba_walk_perm_kernel(const uint4* __restrict__ info, const uint32_t* __restrict
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < hot; i += blockDim.x) {
         const uint32_t c = s_cnt[i];
-        if (c) atomicAdd(cnt + i, c);
+        if (c) atomicAdd(cnt.at(i), c);
     }
     uint32_t f = fallbacks;
 #pragma unroll
@@ -277,31 +304,58 @@ saba_walk_perm_kernel(const uint4* __restrict__ info, const uint32_t* __restrict
     if (lane == 0 && f) atomicAdd(fallback_total, (unsigned long long)f);
 }
 
-// ---- walk copy with the next row inlined in each slot ------------------------------------------------
+// ---- packed walk copy -----------------------------------------------------------------------------
 // A hop of saba_walk_perm_kernel makes two dependent random loads: the chosen slot (the next vertex
-// p) and then p's 16-byte row record.  In this copy, slot q of the renumbered adjacency holds the
-// record of the vertex it points to: (row start, degree, fmix32(original id), p).  A hop is then one
-// dependent 16-byte load; the counter update (p) stays off the dependent chain.  The copy takes
-// 16 bytes per slot (4 x the plain renumbered adjacency).
-__global__ void saba_adj16_kernel(const uint32_t* __restrict__ adjp, const uint4* __restrict__ info,
-                                  uint64_t m, uint4* __restrict__ adj16) {
-    for (uint64_t q = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < m;
-         q += uint64_t(gridDim.x) * blockDim.x) {
-        const uint32_t p = adjp[q];
-        const uint4 r = info[p];
-        adj16[q] = make_uint4(r.x, r.y, fmix32(r.z), p);
+// p) and then p's 16-byte row record.  In the packed copy a hop makes one, of 8 bytes: slot q holds
+// (p | class(p) << pbits, fmix32(original id of p)).  The row record follows from the class: numbers
+// are in order of degree, so the numbers of one degree D are consecutive, P, P + 1, ..., and so are
+// their rows, of D slots each from slot B on; row p starts at B + (p - P) D.  The class table holds
+// (B - P D mod 2^32, D), 8 bytes per distinct degree (607 of them on R-MAT scale 18, 4.9 KB), in
+// shared memory.  The random load is what bounds the walk (a 32-byte sector from L2 per hop; 65-80 %
+// of the L1 pipe busy), so the bytes per slot decide how much of the copy L2 holds.  Against the
+// plain copy (4 + 16 bytes in two dependent loads) and an earlier one of 16 bytes per slot, walk
+// kernel, ms: R-MAT scale 18 (61 MB packed), D 10, W 2,048 25.8 -> 14.6; Chung-Lu n = 10^6, D 10,
+// W 256 34.7 -> 26.6; R-MAT n = 60,000, D 10, W 512 1.35 -> 1.16; the 4,039-vertex graph 0.116 ->
+// 0.117 (all L2-resident before too).
+// cls[p] = number of degree changes up to p = class of p.  The first number of each class writes
+// its entry while the table has room (kMaxClasses); *ncls counts all of them.
+__global__ void saba_class_table_kernel(const uint32_t* __restrict__ cls,
+                                        const uint32_t* __restrict__ sdeg,
+                                        const uint32_t* __restrict__ beg, uint64_t n,
+                                        uint2* __restrict__ classes, uint32_t* __restrict__ ncls) {
+    for (uint64_t p = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < n;
+         p += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t c = cls[p];
+        if ((p == 0 || cls[p - 1] != c) && c < kMaxClasses)
+            classes[c] = make_uint2(beg[p] - uint32_t(p) * sdeg[p], sdeg[p]);
+        if (p + 1 == n) *ncls = c + 1;
     }
 }
 
-// The walk over the inlined copy: trajectories, hashes and fallbacks exactly as
-// saba_walk_perm_kernel (the hash of the primary phase is read precomputed from the slot).
+__global__ void saba_packed_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ adj,
+                                   const uint32_t* __restrict__ row_of,
+                                   const uint32_t* __restrict__ inv, const uint4* __restrict__ info,
+                                   const uint32_t* __restrict__ cls, uint32_t pbits, uint64_t m,
+                                   uint2* __restrict__ slots) {
+    for (uint64_t q = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < m;
+         q += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t old = row_of[q], to = adj[q], p = inv[to];
+        slots[info[inv[old]].x + (uint32_t(q) - idx[old])] =
+            make_uint2(p | (cls[p] << pbits), fmix32(to));
+    }
+}
+
+// The walk over the packed copy: trajectories, hashes and fallbacks exactly as
+// saba_walk_perm_kernel.  Shared memory: the class table, then `hot` counters.
 template <int WPL>
-__global__ void __launch_bounds__(kSabaThreads)
-saba_walk_inline_kernel(const uint4* __restrict__ info, const uint4* __restrict__ adj16,
-                        uint32_t depth, uint32_t bouquets_per_src, uint32_t grid_step,
-                        uint64_t total_bouquets, uint32_t* __restrict__ cnt, uint32_t hot,
-                        unsigned long long* __restrict__ fallback_total) {
-    extern __shared__ uint32_t s_cnt[];
+__global__ void __launch_bounds__(kPackedThreads)
+saba_walk_packed_kernel(const PackedWalk g, uint32_t depth, uint32_t bouquets_per_src,
+                        uint32_t grid_step, uint64_t total_bouquets, WalkCounters cnt,
+                        uint32_t hot, unsigned long long* __restrict__ fallback_total) {
+    extern __shared__ __align__(8) uint32_t s_words[];
+    uint2* s_cls = reinterpret_cast<uint2*>(s_words);
+    uint32_t* s_cnt = s_words + 2 * g.ncls;
+    for (uint32_t i = threadIdx.x; i < g.ncls; i += blockDim.x) s_cls[i] = __ldg(g.classes + i);
     for (uint32_t i = threadIdx.x; i < hot; i += blockDim.x) s_cnt[i] = 0;
     __syncthreads();
 
@@ -311,6 +365,7 @@ saba_walk_inline_kernel(const uint4* __restrict__ info, const uint4* __restrict_
     constexpr uint32_t SB = 4 * WPL;  // bouquets per warp step
     const uint64_t steps = (total_bouquets + SB - 1) / SB;
     const uint64_t s_lo = steps * warp / nwarps, s_hi = steps * (warp + 1) / nwarps;
+    const uint32_t pmask = (1u << g.pbits) - 1u;
 
     uint32_t src[WPL], bq[WPL];
 #pragma unroll
@@ -329,7 +384,7 @@ saba_walk_inline_kernel(const uint4* __restrict__ info, const uint4* __restrict_
             active[w] = b < total_bouquets;
             beg[w] = d[w] = hsh[w] = 0;
             if (active[w]) {
-                const uint4 r = __ldg(info + src[w]);
+                const uint4 r = __ldg(g.info + src[w]);
                 beg[w] = r.x;
                 d[w] = r.y;
                 hsh[w] = fmix32(r.z);
@@ -340,6 +395,7 @@ saba_walk_inline_kernel(const uint4* __restrict__ info, const uint4* __restrict_
             primary[w] = true;
         }
         for (uint32_t len = 0; len < depth; ++len) {
+            uint2 e[WPL];
 #pragma unroll
             for (int w = 0; w < WPL; ++w) {
                 const unsigned zero =
@@ -348,6 +404,7 @@ saba_walk_inline_kernel(const uint4* __restrict__ info, const uint4* __restrict_
             }
 #pragma unroll
             for (int w = 0; w < WPL; ++w) {
+                e[w] = make_uint2(0u, 0u);
                 if (active[w]) {
                     uint32_t k;
                     if (primary[w]) {
@@ -356,12 +413,21 @@ saba_walk_inline_kernel(const uint4* __restrict__ info, const uint4* __restrict_
                     } else {
                         k = splitmix32(state[w]) % d[w];
                     }
-                    const uint4 e = __ldg(adj16 + beg[w] + k);
-                    beg[w] = e.x;
-                    d[w] = e.y;
-                    hsh[w] = e.z;
-                    if (e.w < hot) atomicAdd(s_cnt + e.w, 1u);
-                    else atomicAdd(cnt + e.w, 1u);
+                    e[w] = __ldg(g.slots + beg[w] + k);
+                }
+            }
+#pragma unroll
+            for (int w = 0; w < WPL; ++w) {
+                if (active[w]) {
+                    const uint32_t p = e[w].x & pmask;
+                    if (len + 1 < depth) {
+                        const uint2 c = s_cls[e[w].x >> g.pbits];
+                        beg[w] = c.x + p * c.y;
+                        d[w] = c.y;
+                        hsh[w] = e[w].y;
+                    }
+                    if (p < hot) atomicAdd(s_cnt + p, 1u);
+                    else atomicAdd(cnt.at(p), 1u);
                 }
             }
         }
@@ -379,7 +445,7 @@ saba_walk_inline_kernel(const uint4* __restrict__ info, const uint4* __restrict_
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < hot; i += blockDim.x) {
         const uint32_t c = s_cnt[i];
-        if (c) atomicAdd(cnt + i, c);
+        if (c) atomicAdd(cnt.at(i), c);
     }
     uint32_t f = fallbacks;
 #pragma unroll
@@ -410,63 +476,117 @@ __global__ void saba_sums_kernel(const uint32_t* __restrict__ c, uint64_t n,
 
 }  // namespace
 
-// Builds the degree-renumbered walk copy of the graph once per handle.
+// Renumbers the graph's vertices by degree, once per handle: the row records, the inverse numbering,
+// the class of every number and the class table.
 void saba_prepare(tgtp_graph* g) {
     if (g->saba_ready) return;
     cudaStream_t s = g->stream;
-    const uint64_t n = g->n, m = g->m;
-    if (n > uint64_t(INT32_MAX) || m > uint64_t(UINT32_MAX))
-        fail(TGTP_ERR_UNSUPPORTED, "graph too large for the walk counter");
+    const uint64_t n = g->n;
     g->saba_info.reserve(sizeof(uint4) * (n + 1));
-    g->saba_adj.reserve(sizeof(uint32_t) * (m + 1));
-    DeviceBuffer ids, order, sdeg, beg, inv, tmp;
-    ids.reserve(sizeof(uint32_t) * (n + 1));
-    order.reserve(sizeof(uint32_t) * (n + 1));
-    sdeg.reserve(sizeof(uint32_t) * (n + 1));
-    beg.reserve(sizeof(uint32_t) * (n + 1));
-    inv.reserve(sizeof(uint32_t) * (n + 1));
-    const unsigned nb = unsigned(std::min<uint64_t>((n + 255) / 256, 8u * g->num_sms));
-    saba_iota_kernel<<<nb ? nb : 1, 256, 0, s>>>(ids.as<uint32_t>(), n);
+    g->saba_inv.reserve(sizeof(uint32_t) * (n + 1));
+    g->saba_cls.reserve(sizeof(uint32_t) * (n + 1));
+    g->saba_classes.reserve(sizeof(uint2) * (kMaxClasses + 1));
+    // temporaries: ids, order, sorted degrees, row starts, class flags, then the number of classes
+    DeviceBuffer rows, tmp;
+    const size_t stride = (n + 63) & ~uint64_t(63);
+    rows.reserve(sizeof(uint32_t) * (5 * stride + 1));
+    uint32_t* ids = rows.as<uint32_t>();
+    uint32_t* order = ids + stride;
+    uint32_t* sdeg = order + stride;
+    uint32_t* beg = sdeg + stride;
+    uint32_t* flag = beg + stride;
+    uint32_t* ncls = flag + stride;
+    auto* inv = g->saba_inv.as<uint32_t>();
+    auto* cls = g->saba_cls.as<uint32_t>();
+    const unsigned nb = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, 8u * g->num_sms)));
+    int bits = 1;
+    while (bits < 32 && (g->max_degree >> bits)) ++bits;
+    saba_iota_kernel<<<nb, 256, 0, s>>>(ids, n);
     TGTP_LAUNCH_CHECK("saba_iota_kernel");
-    size_t t1 = 0, t2 = 0;
-    TGTP_CUDA(cub::DeviceRadixSort::SortPairsDescending(
-        nullptr, t1, g->deg.as<uint32_t>(), sdeg.as<uint32_t>(), ids.as<uint32_t>(),
-        order.as<uint32_t>(), int(n), 0, 32, s));
-    TGTP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t2, sdeg.as<uint32_t>(), beg.as<uint32_t>(),
-                                            int(n), s));
-    tmp.reserve(std::max(t1, t2));
-    TGTP_CUDA(cub::DeviceRadixSort::SortPairsDescending(
-        tmp.ptr, t1, g->deg.as<uint32_t>(), sdeg.as<uint32_t>(), ids.as<uint32_t>(),
-        order.as<uint32_t>(), int(n), 0, 32, s));
-    TGTP_CUDA(cub::DeviceScan::ExclusiveSum(tmp.ptr, t2, sdeg.as<uint32_t>(), beg.as<uint32_t>(),
-                                            int(n), s));
-    saba_info_kernel<<<nb ? nb : 1, 256, 0, s>>>(order.as<uint32_t>(), sdeg.as<uint32_t>(),
-                                                 beg.as<uint32_t>(), n, g->saba_info.as<uint4>(),
-                                                 inv.as<uint32_t>());
+    size_t t1 = 0, t2 = 0, t3 = 0;
+    TGTP_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, t1, g->deg.as<uint32_t>(), sdeg, ids,
+                                                        order, n, 0, bits, s));
+    TGTP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t2, sdeg, beg, n, s));
+    TGTP_CUDA(cub::DeviceScan::InclusiveSum(nullptr, t3, flag, cls, n, s));
+    tmp.reserve(std::max({t1, t2, t3}));
+    TGTP_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp.ptr, t1, g->deg.as<uint32_t>(), sdeg, ids,
+                                                        order, n, 0, bits, s));
+    TGTP_CUDA(cub::DeviceScan::ExclusiveSum(tmp.ptr, t2, sdeg, beg, n, s));
+    saba_info_kernel<<<nb, 256, 0, s>>>(order, sdeg, beg, n, g->saba_info.as<uint4>(), inv, flag);
     TGTP_LAUNCH_CHECK("saba_info_kernel");
-    if (m) {
-        const unsigned mb = unsigned(std::min<uint64_t>((m + 255) / 256, 8u * g->num_sms));
-        saba_adj_kernel<<<mb, 256, 0, s>>>(g->idx.as<uint32_t>(), g->adj.as<uint32_t>(),
-                                           g->row_of.as<uint32_t>(), inv.as<uint32_t>(),
-                                           g->saba_info.as<uint4>(), m, g->saba_adj.as<uint32_t>());
-        TGTP_LAUNCH_CHECK("saba_adj_kernel");
-    }
+    TGTP_CUDA(cub::DeviceScan::InclusiveSum(tmp.ptr, t3, flag, cls, n, s));
+    saba_class_table_kernel<<<nb, 256, 0, s>>>(cls, sdeg, beg, n, g->saba_classes.as<uint2>(), ncls);
+    TGTP_LAUNCH_CHECK("saba_class_table_kernel");
+    uint32_t h = 0;
+    TGTP_CUDA(cudaMemcpyAsync(&h, ncls, sizeof(h), cudaMemcpyDeviceToHost, s));
     TGTP_CUDA(cudaStreamSynchronize(s));  // the temporaries go back to the cache
+    g->saba_ncls = h;
     g->saba_ready = true;
 }
 
-// Whether saba_count walks the inlined copy (one dependent 16-byte load per hop) or the plain
-// renumbered copy (two): the tuned choice (saba_tune), else TGTP_SABA_INLINE=0/1, else the inlined
-// copy while its 16 bytes per slot stay within 48 MB.  Walks are random, so the copies are read
-// from L2: on the 4,039-vertex graph (2.8 MB inlined) the inlined copy measured 1.5x the plain
-// one; on R-MAT scale 18 (122 MB inlined against 33 MB plain, beside a 126 MB L2) it measured
-// 0.8x, the inlined copy no longer fitting.  saba_tune may still try it up to 2 GiB.
-bool saba_inline_fits(const tgtp_graph* g) { return g->m * sizeof(uint4) <= (size_t(2) << 30); }
+// The plain renumbered adjacency, once per handle.
+void saba_prepare_plain(tgtp_graph* g) {
+    if (g->saba_plain_ready) return;
+    saba_prepare(g);
+    g->saba_adj.reserve(sizeof(uint32_t) * (g->m + 1));
+    if (g->m) {
+        const unsigned mb = unsigned(std::min<uint64_t>((g->m + 255) / 256, 8u * g->num_sms));
+        saba_adj_kernel<<<mb, 256, 0, g->stream>>>(g->idx.as<uint32_t>(), g->adj.as<uint32_t>(),
+                                                   g->row_of.as<uint32_t>(), g->saba_inv.as<uint32_t>(),
+                                                   g->saba_info.as<uint4>(), g->m,
+                                                   g->saba_adj.as<uint32_t>());
+        TGTP_LAUNCH_CHECK("saba_adj_kernel");
+    }
+    g->saba_plain_ready = true;
+}
 
-bool saba_use_inline(const tgtp_graph* g) {
+// Bits of a vertex number in a packed slot; the class takes the others.
+uint32_t saba_pbits(const tgtp_graph* g) {
+    uint32_t b = 1;
+    while ((g->n - 1) >> b) ++b;
+    return b;
+}
+
+// Whether the graph's numbers and classes fit in a packed slot's 32 bits and the class table in
+// its shared memory, and the copy takes at most 4 GiB (needs saba_prepare).
+bool saba_packable(const tgtp_graph* g) {
+    return saba_pbits(g) < 32 && g->saba_ncls <= kMaxClasses &&
+           g->saba_ncls <= (uint64_t(1) << (32 - saba_pbits(g))) &&
+           g->m * sizeof(uint2) <= (uint64_t(4) << 30);
+}
+
+// The packed copy, once per handle.
+PackedWalk saba_prepare_packed(tgtp_graph* g) {
+    saba_prepare(g);
+    PackedWalk w;
+    w.ncls = g->saba_ncls;
+    w.pbits = saba_pbits(g);
+    if (!g->saba_packed_ready) {
+        g->saba_packed.reserve(sizeof(uint2) * (g->m + 1));
+        if (g->m) {
+            const unsigned mb = unsigned(std::min<uint64_t>((g->m + 255) / 256, 8u * g->num_sms));
+            saba_packed_kernel<<<mb, 256, 0, g->stream>>>(
+                g->idx.as<uint32_t>(), g->adj.as<uint32_t>(), g->row_of.as<uint32_t>(),
+                g->saba_inv.as<uint32_t>(), g->saba_info.as<uint4>(), g->saba_cls.as<uint32_t>(),
+                w.pbits, g->m, g->saba_packed.as<uint2>());
+            TGTP_LAUNCH_CHECK("saba_packed_kernel");
+        }
+        g->saba_packed_ready = true;
+    }
+    w.slots = g->saba_packed.as<uint2>();
+    w.classes = g->saba_classes.as<uint2>();
+    w.info = g->saba_info.as<uint4>();
+    return w;
+}
+
+// Whether saba_count walks the packed copy (one dependent 8-byte load per hop) or the plain
+// renumbered copy (two): the tuned choice (saba_tune), else TGTP_SABA_INLINE=0/1, else the packed
+// copy where the graph fits one (needs saba_prepare).
+bool saba_use_packed(const tgtp_graph* g) {
+    if (!saba_packable(g)) return false;
     if (g->saba_choice) return (g->saba_choice & 0x100) != 0;
     if (const char* e = std::getenv("TGTP_SABA_INLINE")) return std::atoi(e) != 0;
-    return g->m * sizeof(uint4) <= size_t(48) << 20;
+    return true;
 }
 
 // Row records of the plain walk copy kept in shared memory (the highest-degree numbers): the tuned
@@ -484,47 +604,33 @@ uint32_t saba_hot_records(const tgtp_graph* g) {
     return 4096u;
 }
 
-void saba_prepare_inline(tgtp_graph* g) {
-    if (g->saba_inline_ready) return;
-    saba_prepare(g);
-    cudaStream_t s = g->stream;
-    g->saba_adj16.reserve(sizeof(uint4) * (g->m + 1));
-    if (g->m) {
-        const unsigned mb = unsigned(std::min<uint64_t>((g->m + 255) / 256, 8u * g->num_sms));
-        saba_adj16_kernel<<<mb, 256, 0, s>>>(g->saba_adj.as<uint32_t>(), g->saba_info.as<uint4>(),
-                                             g->m, g->saba_adj16.as<uint4>());
-        TGTP_LAUNCH_CHECK("saba_adj16_kernel");
-    }
-    g->saba_inline_ready = true;
-}
-
 template <int WPL>
 void saba_launch(tgtp_graph* g, uint32_t depth, uint32_t bps, uint32_t grid_step, uint64_t total,
-                 uint32_t* cnt, unsigned long long* fb) {
+                 WalkCounters cnt, unsigned long long* fb) {
     cudaStream_t s = g->stream;
-    uint32_t cap = kSabaHotCap;
+    uint32_t cap = saba_use_packed(g) ? kPackedHotCap : kSabaHotCap;
     if (const char* e = std::getenv("TGTP_SABA_HOT")) cap = uint32_t(std::atoi(e));
     cap = std::max<uint32_t>(1024u, std::min<uint32_t>(cap, 53248u));
+    const bool packed = saba_use_packed(g);
+    if (packed) cap = std::min<uint32_t>(cap, 53248u - 2 * g->saba_ncls);  // beside the class table
     const uint32_t hot = uint32_t(g->n < cap ? g->n : cap);
-    const bool inl = saba_use_inline(g);
-    const uint32_t hot_rec = inl ? 0u : std::min(hot, saba_hot_records(g));
-    const size_t smem = sizeof(uint32_t) * (hot + 3 * size_t(hot_rec));
-    if (inl) saba_prepare_inline(g);
-    const void* kern = inl ? reinterpret_cast<const void*>(saba_walk_inline_kernel<WPL>)
-                           : reinterpret_cast<const void*>(saba_walk_perm_kernel<WPL>);
-    TGTP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int per_sm = 0;
-    TGTP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSabaThreads, smem));
-    if (per_sm < 1) per_sm = 1;
+    const uint32_t hot_rec = packed ? 0u : std::min(hot, saba_hot_records(g));
+    PackedWalk pw{};
+    if (packed) pw = saba_prepare_packed(g);
+    else saba_prepare_plain(g);
+    const size_t smem = sizeof(uint32_t) * (hot + 3 * size_t(hot_rec)) + sizeof(uint2) * pw.ncls;
+    const void* kern = packed ? reinterpret_cast<const void*>(saba_walk_packed_kernel<WPL>)
+                              : reinterpret_cast<const void*>(saba_walk_perm_kernel<WPL>);
+    const int threads = packed ? kPackedThreads : kSabaThreads;
+    const int per_sm = std::max(1, blocks_per_sm(kern, threads, smem));
     uint64_t blocks = uint64_t(g->num_sms) * per_sm;
-    const uint64_t need = (total + 4 * WPL - 1) / (4 * WPL) / (kSabaThreads / 32) + 1;
+    const uint64_t need = (total + 4 * WPL - 1) / (4 * WPL) / (threads / 32) + 1;
     if (blocks > need) blocks = need;
     ScopedKernel k(g->prof, s, "saba_walk");
-    if (inl) {
-        saba_walk_inline_kernel<WPL><<<unsigned(blocks), kSabaThreads, smem, s>>>(
-            g->saba_info.as<uint4>(), g->saba_adj16.as<uint4>(), depth, bps, grid_step, total,
-            cnt, hot, fb);
-        TGTP_LAUNCH_CHECK("saba_walk_inline_kernel");
+    if (packed) {
+        saba_walk_packed_kernel<WPL><<<unsigned(blocks), unsigned(threads), smem, s>>>(
+            pw, depth, bps, grid_step, total, cnt, hot, fb);
+        TGTP_LAUNCH_CHECK("saba_walk_packed_kernel");
     } else {
         saba_walk_perm_kernel<WPL><<<unsigned(blocks), kSabaThreads, smem, s>>>(
             g->saba_info.as<uint4>(), g->saba_adj.as<uint32_t>(), depth, bps, grid_step, total,
@@ -533,23 +639,44 @@ void saba_launch(tgtp_graph* g, uint32_t depth, uint32_t bps, uint32_t grid_step
     }
 }
 
+// One zeroing for the sums (visit count, checksum, fallback bouquets, unused) and the counters of
+// the renumbered vertices behind them.
+WalkCounters walk_counters(tgtp_graph* g) {
+    WalkCounters c;
+    c.len = 8u * uint32_t((g->n + 511) / 512);
+    const size_t bytes = 4 * sizeof(unsigned long long) + sizeof(uint32_t) * 64 * size_t(c.len);
+    g->sums.reserve(bytes);
+    TGTP_CUDA(cudaMemsetAsync(g->sums.ptr, 0, bytes, g->stream));
+    c.words = reinterpret_cast<uint32_t*>(g->sums.as<unsigned long long>() + 4);
+    return c;
+}
+
+void scatter_counters(tgtp_graph* g, WalkCounters cnt, uint32_t* device_counters) {
+    ScopedKernel k(g->prof, g->stream, "saba_scatter");
+    const unsigned nb = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((g->n + 255) / 256, 8u * g->num_sms)));
+    saba_scatter_kernel<<<nb, 256, 0, g->stream>>>(cnt, g->saba_info.as<uint4>(), g->n, device_counters,
+                                                   g->sums.as<unsigned long long>());
+    TGTP_LAUNCH_CHECK("saba_scatter_kernel");
+}
+
 void saba_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, uint32_t* device_counters) {
     cudaStream_t s = g->stream;
-    g->sums.reserve(4 * sizeof(unsigned long long));
-    auto* sums = g->sums.as<unsigned long long>();
-    TGTP_CUDA(cudaMemsetAsync(device_counters, 0, sizeof(uint32_t) * g->n, s));
-    TGTP_CUDA(cudaMemsetAsync(sums, 0, 4 * sizeof(unsigned long long), s));
-    if (n_walks == 0 || depth == 0) return;
+    const WalkCounters cnt = walk_counters(g);
+    if (n_walks == 0 || depth == 0) {
+        TGTP_CUDA(cudaMemsetAsync(device_counters, 0, sizeof(uint32_t) * g->n, s));
+        return;
+    }
+    if (g->n > uint64_t(INT32_MAX))
+        fail(TGTP_ERR_UNSUPPORTED, "graph too large for the walk counter");
     saba_prepare(g);
+    auto* sums = g->sums.as<unsigned long long>();
     const uint32_t bouquets_per_src = n_walks / 8;
     const uint32_t grid_step = UINT32_MAX / n_walks;
     const uint64_t total = g->n * uint64_t(bouquets_per_src);
-    g->saba_cnt.reserve(sizeof(uint32_t) * (g->n + 1));
-    auto* cnt = g->saba_cnt.as<uint32_t>();
-    TGTP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * g->n, s));
-    // walkers per lane: the tuned choice, else TGTP_SABA_WPL, else 1 over the inlined copy and 2
-    // over the plain one (its two dependent loads per hop want more chains in flight)
-    int wpl = saba_use_inline(g) ? 1 : 2;
+    // walkers per lane: the tuned choice, else TGTP_SABA_WPL, else 1 over the packed copy (2: within
+    // 2 % on large graphs, 6 % slower on the 4,039-vertex one) and 2 over the plain one (its two
+    // dependent loads per hop want more chains in flight)
+    int wpl = saba_use_packed(g) ? 1 : 2;
     if (g->saba_choice) wpl = g->saba_choice & 0xff;
     else if (const char* e = std::getenv("TGTP_SABA_WPL")) wpl = std::atoi(e);
     switch (wpl) {
@@ -557,19 +684,14 @@ void saba_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, uint32_t* device_
         case 4: saba_launch<4>(g, depth, bouquets_per_src, grid_step, total, cnt, sums + 2); break;
         default: saba_launch<1>(g, depth, bouquets_per_src, grid_step, total, cnt, sums + 2); break;
     }
-    {
-        ScopedKernel k(g->prof, s, "saba_scatter");
-        const unsigned nb = unsigned(std::min<uint64_t>((g->n + 255) / 256, 8u * g->num_sms));
-        saba_scatter_kernel<<<nb ? nb : 1, 256, 0, s>>>(cnt, g->saba_info.as<uint4>(), g->n,
-                                                        device_counters);
-        TGTP_LAUNCH_CHECK("saba_scatter_kernel");
-    }
+    scatter_counters(g, cnt, device_counters);
 }
 
 int saba_tune(tgtp_graph* g, uint32_t depth, uint32_t n_walks, int trials) {
+    saba_prepare(g);
     std::vector<uint16_t> cand;
     for (int wpl : {1, 2, 4}) {
-        if (saba_inline_fits(g)) cand.push_back(uint16_t(0x100 | wpl));
+        if (saba_packable(g)) cand.push_back(uint16_t(0x100 | wpl));
         // plain copy: no hot records, or 3,072 / 4,096 of them in shared memory
         for (int code : {0, 3, 4}) cand.push_back(uint16_t((code << 12) | wpl));
     }
@@ -615,17 +737,14 @@ int saba_tune(tgtp_graph* g, uint32_t depth, uint32_t n_walks, int trials) {
     return pick;
 }
 
-void saba_summarize(tgtp_graph* g, const uint32_t* device_counters, uint64_t* host_sums3) {
+void saba_summarize(tgtp_graph* g, const uint32_t* device_counters, uint32_t* host_counters,
+                    uint64_t* host_sums3) {
     cudaStream_t s = g->stream;
-    auto* sums = g->sums.as<unsigned long long>();
-    {
-        ScopedKernel k(g->prof, s, "saba_sums");
-        const unsigned blocks = unsigned(std::min<uint64_t>((g->n + 255) / 256, 4u * g->num_sms));
-        saba_sums_kernel<<<blocks ? blocks : 1, 256, 0, s>>>(device_counters, g->n, sums);
-        TGTP_LAUNCH_CHECK("saba_sums_kernel");
-    }
     unsigned long long h[3];
-    TGTP_CUDA(cudaMemcpyAsync(h, sums, sizeof(h), cudaMemcpyDeviceToHost, s));
+    if (host_counters)
+        TGTP_CUDA(cudaMemcpyAsync(host_counters, device_counters, sizeof(uint32_t) * g->n,
+                                  cudaMemcpyDeviceToHost, s));
+    TGTP_CUDA(cudaMemcpyAsync(h, g->sums.ptr, sizeof(h), cudaMemcpyDeviceToHost, s));
     TGTP_CUDA(cudaStreamSynchronize(s));
     host_sums3[0] = h[0];
     host_sums3[1] = h[1];
