@@ -185,10 +185,15 @@ Profiler::~Profiler() {
 // ---- per-slot maps built on the device at upload -----------------------------------------------
 namespace {
 
-__global__ void degree_kernel(const uint32_t* __restrict__ idx, uint64_t n, uint32_t* __restrict__ deg) {
+// Degrees and their reciprocals (infinite for an isolated vertex).
+__global__ void degree_kernel(const uint32_t* __restrict__ idx, uint64_t n, uint32_t* __restrict__ deg,
+                              double* __restrict__ dinv) {
     for (uint64_t v = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < n;
-         v += uint64_t(gridDim.x) * blockDim.x)
-        deg[v] = idx[v + 1] - idx[v];
+         v += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t d = idx[v + 1] - idx[v];
+        deg[v] = d;
+        dinv[v] = __ddiv_rn(1.0, double(d));
+    }
 }
 
 // row_of[pos] = u with idx[u] <= pos < idx[u+1] (rows may be empty: take the last such u).
@@ -404,7 +409,9 @@ void graph_prepare(tgtp_graph* g) {
     unsigned* info = c + n + 1;  // forward total, then {flags, max, min, active}
     const unsigned init[5] = {0u, 0u, 0u, 0xffffffffu, 0u};
     TGTP_CUDA(cudaMemcpyAsync(info, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    degree_kernel<<<grid_for(n, g->num_sms), 256, 0, s>>>(idx, n, g->deg.as<uint32_t>());
+    g->dinv.reserve(sizeof(double) * (n + 1));
+    degree_kernel<<<grid_for(n, g->num_sms), 256, 0, s>>>(idx, n, g->deg.as<uint32_t>(),
+                                                          g->dinv.as<double>());
     TGTP_LAUNCH_CHECK("degree_kernel");
     if (m) {
         row_of_kernel<<<grid_for(m, g->num_sms), 256, 0, s>>>(idx, n, m, g->row_of.as<uint32_t>());

@@ -152,6 +152,7 @@ struct tgtp_graph {
 
     // CSR and derived per-slot maps (device)
     tgtp::DeviceBuffer idx, adj, deg;
+    tgtp::DeviceBuffer dinv;     // 1 / degree (FP64)
     tgtp::DeviceBuffer row_of;   // slot -> its row u
     tgtp::DeviceBuffer rev;      // slot (u,v) -> lower_bound of u in row v
     tgtp::DeviceBuffer sym_src;  // slot q -> 1 + last slot p with rev[p] == q (0: none)
