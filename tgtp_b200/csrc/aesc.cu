@@ -9,9 +9,11 @@
 //   2. the listed sources: push rounds until the push/walk cost test stops them (:456-503), the
 //      top-gamma edge bound (:414-442), the per-edge chi and walk count (:392-412, :508-521) and
 //      the 2-way bouquet walks (:241-391), accumulating each source's CSR row (:524-525).
-//        source_kernel       persistent warps, one source at a time per warp;
-//        push_block_kernel   mixed form on large graphs: the push of 32 sources per CTA as a
-//                            pull product, then source_kernel for the rest (PrePush mode).
+//        source_kernel        FP32 / FP64 forms: persistent warps, one source at a time per warp;
+//        mixed_source_kernel  mixed form: one source at a time per block (mixed_source.cuh);
+//        push_shared_kernel, push_block_kernel  mixed form, deep pushes: the push alone, one source
+//                             per block in shared memory, or 32 sources per CTA as a pull product;
+//                             then mixed_source_kernel for the rest and the walk kernels.
 //   3. finish_kernel: score[q] = row[q] + row[reverse slot] (:532-550), with the rows of unlisted
 //      sources (every tau <= 1: one push round, no walks) in closed form.
 //
@@ -99,6 +101,7 @@ inline int form_key(const tgtp_config& cfg) {
 
 // The run's work words ([0] next list entry, [1] error flags, [2] list length, [3] unused) sit
 // behind the striped counters in the same buffer, and the per-row marks behind them.
+constexpr int kWorkWords = 4;
 inline unsigned* run_work(tgtp_graph* g) {
     return reinterpret_cast<unsigned*>(g->stats.as<unsigned char>() +
                                        sizeof(unsigned long long) * kStCount * kStStripes);
@@ -964,20 +967,19 @@ struct PrePush {
     uint32_t support;  // size of the final frontier
 };
 
-template <class Real, class Acc>
+template <class Real>
 struct SourceParams {
     const uint32_t* idx;
     const uint32_t* adj;
     const uint32_t* deg;
     uint32_t n;
     const int* taus;
-    Acc* preds;           // pre-symmetric row scores (Real in the parity forms, double in MIXED)
+    Real* preds;          // pre-symmetric row scores
     unsigned* work;       // [0] next list entry, [1] error flags, [2] list length
     const uint32_t* rows; // the sources to run (rows with a slot of tau > 1), in any order
     uint32_t* qbuf;       // 2 * n per warp
     WalkItem* items;      // max_degree per warp
     Real* pvec_g;         // n per warp (global tier)
-    unsigned long long* fx_g;  // n per warp: fixed-point accumulators (Jacobi push, global tier)
     unsigned char* wclean;     // per warp: 1 = its HBM vectors are all zero (left so by its last run)
     unsigned char* vis_g; // vis_stride per warp (global tier)
     size_t vis_stride;
@@ -990,32 +992,18 @@ struct SourceParams {
     const uint2* adjd;    // (neighbour, neighbour degree) per slot
     uint64_t budget_ns;   // device time budget; past it every warp stops and flags a timeout
     unsigned* claim;      // the claim counter of this launch
-    uint32_t list_base;   // this launch runs list entries [list_base, list_base + list_cap)
-    uint32_t list_cap;
-    // PrePush mode (mixed form, large graphs): the push ran in push_block_kernel; entry k's final
-    // residual vector is column (k - list_base) % S of its CTA's block
-    const PrePush* pre;
-    const float* pre_cols;
-    const uint32_t* pre_final;
     // The graph has rows that repeat a neighbour or hold their own vertex (the reference's loader
     // keeps duplicate edges and self-loops, src/graph.h:63-66, 75-78): the first round takes the
-    // general path and the push serialises each run of a repeated neighbour (parity forms only).
+    // general path and the push serialises each run of a repeated neighbour.
     bool multi;
     // Vertex count the per-warp scratch is laid out for (the graph's n, or the largest n of a
     // batch whose graphs share the scratch of one persistent launch).
     uint32_t scratch_n;
-    bool gs_window;  // parity forms: the windowed sequential push (else one vertex at a time)
+    bool gs_window;  // the windowed sequential push (else one vertex at a time)
     // Optional run trace (null when off): the walk count nr of every walking slot, and the rounds
     // pushed (ell) of every listed row.
     uint32_t* trace_nr;
     uint32_t* trace_ell;
-    // PrePush mode: when set, a source's walking slots (with their nr) are appended to this queue
-    // instead of being walked by the warp here: light items from the front (walk_count[0] counts
-    // them; walk_queue_kernel walks them), heavy ones (many walks of few hops) from the back
-    // (walk_count[2]; heavy_walk_kernel).  walk_cap entries.
-    WalkItem* walk_queue;
-    unsigned* walk_count;
-    uint32_t walk_cap;
 };
 
 // The source kernel's parameters: one graph (N = 1), or up to N graphs whose listed rows one
@@ -1023,11 +1011,11 @@ struct SourceParams {
 // first entry's per-warp scratch (qbuf, items, residual vectors, flags, claim counter).  The pack
 // travels in the kernel's parameter space, so a warp reads its graph's fields from the constant
 // bank with a warp-uniform index.
-template <class Real, class Acc, int N>
+template <class Real, int N>
 struct SourcePack {
     static constexpr int kMax = N;
     uint32_t count;
-    SourceParams<Real, Acc> g[N];
+    SourceParams<Real> g[N];
 };
 constexpr int kBatchPack = 64;  // graphs per persistent batch launch
 
@@ -1171,119 +1159,6 @@ __device__ void kth_largest(const uint32_t* q, uint32_t qs, const Real* pvec, in
         }
         remaining -= int(c);
         thr = mx;
-    }
-}
-
-// kth_largest over the positive entries of a dense vector (the residual column the block push
-// leaves, whose positive entries are exactly the final frontier, in vertex order): the same
-// selection without the frontier list, as contiguous pipelined loads.
-template <class Real>
-__device__ void kth_largest_col(const Real* col, uint32_t n, int rg, Real& t, int& n_eq_taken,
-                                uint32_t* cand = nullptr, uint32_t* ncand = nullptr) {
-    const uint32_t lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    auto load_v = [&](uint32_t i0, Real* r) {
-#pragma unroll
-        for (int b = 0; b < kB; ++b) {
-            const uint32_t i = i0 + 32 * b + lane;
-            const Real x = i < n ? col[i] : Real(0);
-            r[b] = x > Real(0) ? x : Real(-INFINITY);
-        }
-    };
-    if (rg <= kTopK) {
-        Real L[kTopK];
-#pragma unroll
-        for (int j = 0; j < kTopK; ++j) L[j] = Real(-INFINITY);
-        // With cand: every positive entry that reaches its lane's top kTopK so far (x >= the
-        // lane's current kTopK-th value) is listed, in index order.  An entry not listed had
-        // kTopK >= rg larger ones before it, so it is below the rg-th largest value; every entry
-        // at or above that value has fewer than rg larger ones and is listed.
-        uint32_t nc = 0;
-        pipelined<Real>(n, load_v, [&](uint32_t i0, const Real* r) {
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                const Real x = r[b];
-                if (cand) {
-                    const bool rec = x > Real(-INFINITY) && x >= L[kTopK - 1];
-                    const unsigned bal = __ballot_sync(kFullMask, rec);
-                    if (rec) cand[nc + __popc(bal & below)] = i0 + 32 * b + lane;
-                    nc += __popc(bal);
-                }
-                if (x > L[kTopK - 1]) {
-#pragma unroll
-                    for (int j = kTopK - 1; j > 0; --j) {
-                        const Real prev = L[j - 1];
-                        L[j] = x > prev ? prev : (x > L[j] ? x : L[j]);
-                    }
-                    L[0] = x > L[0] ? x : L[0];
-                }
-            }
-        });
-        Real last = Real(-INFINITY);
-        int run = 0;
-        for (int r = 0; r < rg; ++r) {
-            const Real mx = warp_max(L[0]);
-            const unsigned who = __ballot_sync(kFullMask, L[0] == mx);
-            if (lane == uint32_t(__ffs(who) - 1)) {
-#pragma unroll
-                for (int j = 0; j < kTopK - 1; ++j) L[j] = L[j + 1];
-                L[kTopK - 1] = Real(-INFINITY);
-            }
-            run = (r > 0 && mx == last) ? run + 1 : 1;
-            last = mx;
-        }
-        t = last;
-        n_eq_taken = run;
-        if (ncand) *ncand = nc;
-        return;
-    }
-    Real thr = Real(INFINITY);
-    int remaining = rg;
-    while (true) {
-        Real best = Real(-INFINITY);
-        unsigned cnt = 0;
-        pipelined<Real>(n, load_v, [&](uint32_t, const Real* r) {
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                const Real x = r[b];
-                if (x < thr && x > Real(-INFINITY)) {
-                    if (x > best) {
-                        best = x;
-                        cnt = 1;
-                    } else if (x == best) {
-                        ++cnt;
-                    }
-                }
-            }
-        });
-        const Real mx = warp_max(best);
-        unsigned c = best == mx ? cnt : 0;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(kFullMask, c, o);
-        if (int(c) >= remaining) {
-            t = mx;
-            n_eq_taken = remaining;
-            return;
-        }
-        remaining -= int(c);
-        thr = mx;
-    }
-}
-
-// Segmented max / min over lanes whose segment ids are non-decreasing: after the shuffles, the
-// last lane of each segment holds the segment's extremum.
-template <class Real>
-__device__ __forceinline__ void seg_maxmin(uint32_t seg, Real& mx, Real& mn) {
-    const uint32_t lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const Real ymx = __shfl_up_sync(kFullMask, mx, o);
-        const Real ymn = __shfl_up_sync(kFullMask, mn, o);
-        const uint32_t ys = __shfl_up_sync(kFullMask, seg, o);
-        if (lane >= uint32_t(o) && ys == seg) {
-            mx = std_max(mx, ymx);
-            mn = std_min(mn, ymn);
-        }
     }
 }
 
@@ -1793,10 +1668,9 @@ __global__ void row_key_kernel(const uint32_t* __restrict__ idx, const int* __re
 }
 
 // The HBM-tier variants with FP32 residuals keep at least three 128-thread blocks per SM (at most
-// 168 registers, the occupancy they had before the windowed push and the column edge bound were
-// added): their phases are latency-bound on HBM and need the warps.  The FP64 variant compiled to
-// about 240 registers (two blocks per SM) without spills before and is left so.
-template <class Real, class Acc, bool SMEM, bool JACOBI, class Pack>
+// 168 registers): their phases are latency-bound on HBM and need the warps.  The FP64 variant
+// compiled to about 240 registers (two blocks per SM) without spills before and is left so.
+template <class Real, bool SMEM, class Pack>
 __global__ void __launch_bounds__(kSrcMaxThreads, (!SMEM && sizeof(Real) == 4) ? 3 : 1)
 source_kernel(Pack pk) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1806,31 +1680,23 @@ source_kernel(Pack pk) {
     const uint32_t wpb = blockDim.x >> 5;
     const uint64_t gw = uint64_t(blockIdx.x) * wpb + wib;
     // the per-warp scratch (shared by every graph of the pack) comes from the first entry
-    const SourceParams<Real, Acc>& p0 = pk.g[0];
+    const SourceParams<Real>& p0 = pk.g[0];
     const uint32_t sn = p0.scratch_n;
     const unsigned lt = (1u << lane) - 1u;
     constexpr uint32_t NONE = 0xffffffffu;
     Real* pvec;
     unsigned char* vis;       // per vertex: 1 = discovered this round, 2 = in the top-gamma set
     unsigned long long* acc;  // 64 per warp: per-slot neighbourhood max (0..31) / min (32..63)
-    unsigned long long* fx;   // Jacobi push: per-vertex fixed-point accumulators (all zero between rounds)
     if (SMEM) {
         unsigned char* base = smem + size_t(wib) * p0.smem_per_warp;
         pvec = reinterpret_cast<Real*>(base);
         const size_t pv = (size_t(sn) * sizeof(Real) + 15) & ~size_t(15);
         vis = base + pv;
         const size_t vb = (size_t(sn) + 15) & ~size_t(15);
-        // the fixed-point accumulators live in shared memory when they fit beside the residual
-        // vector, else in HBM (p0.fx_g)
-        const bool fx_here = JACOBI && p0.fx_g == nullptr;
-        fx = fx_here ? reinterpret_cast<unsigned long long*>(base + pv + vb)
-                     : (JACOBI ? p0.fx_g + gw * size_t(sn) : nullptr);
-        acc = reinterpret_cast<unsigned long long*>(base + pv + vb +
-                                                    (fx_here ? sizeof(unsigned long long) * sn : 0));
+        acc = reinterpret_cast<unsigned long long*>(base + pv + vb);
     } else {
         pvec = p0.pvec_g + gw * size_t(sn);
         vis = p0.vis_g + gw * p0.vis_stride;
-        fx = JACOBI ? p0.fx_g + gw * size_t(sn) : nullptr;
         acc = reinterpret_cast<unsigned long long*>(smem + size_t(wib) * kAccBytes);
     }
     // pvec and flags are zeroed once, before the warp's first source, unless the warp's last run
@@ -1887,9 +1753,7 @@ source_kernel(Pack pk) {
         uint32_t acc_items = 0;
         s_pre[0] = 0;
         for (uint32_t i = 0; i < pk.count; ++i) {
-            const SourceParams<Real, Acc>& gp = pk.g[i];
-            const unsigned total = gp.work[2];
-            acc_items += total > gp.list_base ? min(total - gp.list_base, gp.list_cap) : 0u;
+            acc_items += pk.g[i].work[2];
             s_pre[i + 1] = acc_items;
         }
     }
@@ -1911,16 +1775,12 @@ source_kernel(Pack pk) {
         if (k >= nrows) break;
         // the item's graph: the last list whose prefix is at most k (warp-uniform)
         uint32_t gi = 0;
-        if (Pack::kMax > 1) {
-            uint32_t lo = 0, hi = pk.count;
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (s_pre[mid] <= k) lo = mid;
-                else hi = mid;
-            }
-            gi = lo;
+        for (uint32_t hi = pk.count; hi - gi > 1;) {
+            const uint32_t mid = (gi + hi) >> 1;
+            if (s_pre[mid] <= k) gi = mid;
+            else hi = mid;
         }
-        const SourceParams<Real, Acc>& p = pk.g[gi];
+        const SourceParams<Real>& p = pk.g[gi];
         if (gi != last_gi) {
             if (last_gi != 0xffffffffu) flush_stats(pk.g[last_gi].stats);
             last_gi = gi;
@@ -1933,13 +1793,11 @@ source_kernel(Pack pk) {
         const uint32_t* __restrict__ idx = p.idx;
         const uint32_t* __restrict__ adj = p.adj;
         const int* __restrict__ taus = p.taus;
-        const uint32_t entry = p.list_base + uint32_t(k - s_pre[gi]);
-        const uint32_t src = __ldg(p.rows + entry);
+        const uint32_t src = __ldg(p.rows + uint32_t(k - s_pre[gi]));
         if (!cleared) {
             for (uint32_t i = lane; i < sn; i += 32) {
                 pvec[i] = Real(0);
                 vis[i] = 0;
-                if (JACOBI) fx[i] = 0ull;
             }
             cleared = true;
             __syncwarp();
@@ -1950,7 +1808,7 @@ source_kernel(Pack pk) {
         const uint32_t dsi = re - rb;
         const Real ds = from_u64<Real>(dsi);
         // preds = 1.0 / ds (:468-470); stored together with the first round's update below
-        const Acc pinit = from_f64<Acc>(__ddiv_rn(1.0, double(ds)));
+        const Real pinit = from_f64<Real>(__ddiv_rn(1.0, double(ds)));
         uint32_t qs = 0;
         int ell = 0;
         Real gmin, gmax;
@@ -1973,46 +1831,7 @@ source_kernel(Pack pk) {
             }
         };
         lap(0);
-        if (p.pre) {
-            // The push ran in push_block_kernel, which left the source's final residual vector as
-            // n contiguous floats (its column, transposed into the CTA's other block buffer).  The
-            // HBM tier reads it in place; the shared-memory tier copies it.  The final frontier
-            // (the support) is rebuilt in vertex order.
-            const PrePush pr = p.pre[entry];
-            const float* cb = pre_column(p.pre_cols, p.pre_final, entry - p.list_base, n);
-            if constexpr (!SMEM && std::is_same<Real, float>::value) pvec = const_cast<Real*>(cb);
-            uint32_t cq = 0;
-            // HBM tier: the column is read in place and the edge bound selects from it directly
-            // (its positive entries are the frontier, in vertex order), so no frontier list is
-            // built; the shared-memory tier copies the column and lists the frontier.  The scan
-            // keeps 2 x kB coalesced 128-byte loads in flight (pipelined).
-            if (!SMEM) cq = pr.support;
-            else pipelined<Real>(n,
-                [&](uint32_t i0, Real* r) {
-#pragma unroll
-                    for (int b = 0; b < kB; ++b) {
-                        const uint32_t i = i0 + 32 * b + lane;
-                        r[b] = i < n ? Real(cb[i]) : Real(0);
-                    }
-                },
-                [&](uint32_t i0, const Real* r) {
-#pragma unroll
-                    for (int b = 0; b < kB; ++b) {
-                        const uint32_t i = i0 + 32 * b + lane;
-                        if (SMEM && i < n) pvec[i] = r[b];
-                        const bool nz = r[b] > Real(0);
-                        const unsigned bal = __ballot_sync(kFullMask, nz);
-                        if (nz) q[cq + __popc(bal & lt)] = i;
-                        cq += __popc(bal);
-                    }
-                });
-            __syncwarp();
-            qs = cq;
-            ell = pr.ell;
-            gmax = Real(pr.gmax);
-            gmin = qs < n ? Real(0) : Real(pr.gmin);
-            lap(1);
-        } else {
+        {
             // ---- round 1 in closed form (:457-503, first pass of the loop) ----
             // The frontier is {src} with residual 1 (pvec[src] = 1.0, then zeroed as it is drained):
             // every neighbour u is discovered in row order and receives 0 + 1/deg(u) = 1/deg(u), so
@@ -2020,7 +1839,7 @@ source_kernel(Pack pk) {
             // preds = 1/ds + (0 - 1/deg(u)) / ds follow from one pass over the row when the
             // neighbours are distinct.  Rows of a graph with repeated neighbours or self-loops
             // (p.multi, parity forms) take the general path below instead.
-            if (!JACOBI && p.multi) {
+            if (p.multi) {
                 // (1) each run of one neighbour u (rows are sorted, so repeats are adjacent) is
                 // handled by its first slot: k repeats add 1/deg(u) k times in order, as the
                 // reference's sequential += does; that slot discovers u (first-occurrence order)
@@ -2051,7 +1870,7 @@ source_kernel(Pack pk) {
                 // (2) preds[s -> t] = 1/ds + (pvec[s] - pvec[t]) / ds with the round's residuals
                 const Real ps = pvec[src];
                 for (uint32_t o = lane; o < dsi; o += 32)
-                    p.preds[rb + o] = row_update<Real, Acc>(pinit, ps, pvec[__ldg(adj + rb + o)], ds);
+                    p.preds[rb + o] = row_update<Real, Real>(pinit, ps, pvec[__ldg(adj + rb + o)], ds);
                 qs = found;
             } else {
             pipelined<uint2>(dsi,
@@ -2067,14 +1886,13 @@ source_kernel(Pack pk) {
                     for (int b = 0; b < kB; ++b) {
                         if (r[b].x == NONE) continue;
                         const uint32_t o = c + 32 * b + lane;
-                        const Real pu = JACOBI ? Real(from_fixed(kFixOne, r[b].y))
-                                               : rdiv(Real(1), from_u64<Real>(r[b].y));
+                        const Real pu = rdiv(Real(1), from_u64<Real>(r[b].y));
                         pvec[r[b].x] = pu;
                         qn[o] = r[b].x;
                         pcost += r[b].y;
                         mx = std_max(mx, pu);
                         mn = std_min(mn, pu);
-                        p.preds[rb + o] = row_update<Real, Acc>(pinit, Real(0), pu, ds);
+                        p.preds[rb + o] = row_update<Real, Real>(pinit, Real(0), pu, ds);
                     }
                 });
             qs = dsi;
@@ -2124,7 +1942,6 @@ source_kernel(Pack pk) {
                 uint32_t qns = 0;
                 pcost = 0;
                 st_pv += qs;
-                if constexpr (!JACOBI) {
                 if (p.gs_window) {
                 // ---- diffuse (:218-239), windowed ----
                 // The reference drains the frontier one vertex at a time: r = pvec[v], pvec[v] = 0,
@@ -2308,7 +2125,7 @@ source_kernel(Pack pk) {
                                 // before this one, as the reference's sequential loop does
                                 bool lead = act;
                                 uint32_t reps = 1;
-                                if (!JACOBI && p.multi) {
+                                if (p.multi) {
                                     const uint32_t pcu = __shfl_up_sync(kFullMask, cu, 1);
                                     const bool follow = act && lane > 0 && pcu == cu;
                                     const unsigned fb = __ballot_sync(kFullMask, follow);
@@ -2345,133 +2162,6 @@ source_kernel(Pack pk) {
                     }
                 }
                 }
-                } else {
-                    // ---- Jacobi push (mixed form) ----
-                    // The frontier's residuals are taken together, in 2^-62 fixed point
-                    // (r_i = to_fixed(pvec[q_i]), pvec[q_i] = 0, read as each group of 32 frontier
-                    // vertices starts: the round's pushes go to the accumulators, never to pvec, so
-                    // every r_i is the value the round started with), then pushed over the
-                    // concatenated adjacency of 32 frontier vertices at a time: each lane walks
-                    // entries lane, lane + 32, ... with a cursor over the vertices' start offsets,
-                    // and every entry (v -> u) adds r_v to u's 64-bit accumulator with an integer
-                    // atomic, so the sums do not depend on the order.  The touched vertices form the
-                    // new frontier in discovery order; once the round is over their residuals become
-                    // acc[u] / deg(u) (from_fixed), exactly as push_block_kernel computes them.
-                    unsigned long long* rvs = acc + 64;
-                    uint32_t* exs = reinterpret_cast<uint32_t*>(rvs + 32);
-                    uint32_t* vbs = exs + 33;
-                    for (uint32_t i0 = 0; i0 < qs; i0 += 32) {
-                        uint32_t vb = 0, vd = 0;
-                        unsigned long long rv = 0;
-                        if (i0 + lane < qs) {
-                            const uint32_t v = q[i0 + lane];
-                            vb = __ldg(idx + v);
-                            vd = __ldg(idx + v + 1) - vb;
-                            rv = to_fixed(float(pvec[v]));
-                            pvec[v] = Real(0);
-                        }
-                        uint32_t incl = vd;
-#pragma unroll
-                        for (int o = 1; o < 32; o <<= 1) {
-                            const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
-                            if (lane >= uint32_t(o)) incl += y;
-                        }
-                        const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-                        exs[lane] = incl - vd;
-                        vbs[lane] = vb;
-                        rvs[lane] = rv;
-                        if (lane == 31) exs[32] = total;
-                        __syncwarp();
-                        st_tr += total;
-                        uint32_t cm = 0;
-                        struct PEnt {
-                            uint32_t seg, u, du;
-                        };
-                        pipelined<PEnt>(total,
-                            [&](uint32_t e0, PEnt* r) {
-#pragma unroll
-                                for (int b = 0; b < kB; ++b) {
-                                    const uint32_t e = e0 + 32 * b + lane;
-                                    r[b].seg = 32u;
-                                    r[b].u = NONE;
-                                    r[b].du = 1u;
-                                    if (e < total) {
-                                        while (exs[cm + 1] <= e) ++cm;
-                                        const uint2 a = __ldg(p.adjd + vbs[cm] + (e - exs[cm]));
-                                        r[b].seg = cm;
-                                        r[b].u = a.x;
-                                        r[b].du = a.y;
-                                    }
-                                }
-                            },
-                            [&](uint32_t, const PEnt* r) {
-#pragma unroll
-                                for (int b = 0; b < kB; ++b) {
-                                    const bool valid = r[b].seg < 32u;
-                                    const uint32_t u = r[b].u;
-                                    // entries of one frontier vertex are distinct neighbours; only a
-                                    // step that spans several vertices can repeat one, and then the
-                                    // first lane of a repeated neighbour adds the group's residuals
-                                    // (integers: any order gives the same sum) and discovers it.
-                                    // The accumulators are this warp's own, so with one writer per
-                                    // neighbour a step needs no atomics.
-                                    unsigned long long add = valid ? rvs[r[b].seg] : 0ull;
-                                    const uint32_t seg0 = __shfl_sync(kFullMask, r[b].seg, 0);
-                                    const bool one_seg = __all_sync(kFullMask, !valid || r[b].seg == seg0);
-                                    const unsigned grp =
-                                        one_seg ? (1u << lane) : __match_any_sync(kFullMask, u);
-                                    const bool leader = valid && lane == uint32_t(__ffs(grp) - 1);
-                                    if (!one_seg) {
-                                        const unsigned others = __ballot_sync(kFullMask, valid && !leader);
-                                        for (unsigned mm = others; mm; mm &= mm - 1) {
-                                            const int t = __ffs(mm) - 1;
-                                            const unsigned long long ct = __shfl_sync(kFullMask, add, t);
-                                            if (leader && ((grp >> t) & 1u)) add += ct;
-                                        }
-                                    }
-                                    if (leader) fx[u] += add;
-                                    bool fresh = false;
-                                    if (leader && vis[u] == 0) {
-                                        vis[u] = 1;
-                                        fresh = true;
-                                    }
-                                    const unsigned bal = __ballot_sync(kFullMask, fresh);
-                                    if (fresh) {
-                                        qn[qns + __popc(bal & lt)] = u;
-                                        pcost += r[b].du;
-                                    }
-                                    qns += __popc(bal);
-                                    __syncwarp();
-                                }
-                            });
-                        __syncwarp();
-                    }
-                    // the touched vertices' new residuals; in the same pass their flags are
-                    // cleared and their residual max / min taken (:484-491), which the GS push
-                    // does after the row update below (neither touches what it reads)
-                    mx = Real(0);
-                    mn = Real(1);
-                    pipelined<uint32_t>(qns,
-                        [&](uint32_t i0, uint32_t* r) {
-#pragma unroll
-                            for (int b = 0; b < kB; ++b) {
-                                const uint32_t i = i0 + 32 * b + lane;
-                                r[b] = i < qns ? qn[i] : NONE;
-                            }
-                        },
-                        [&](uint32_t, const uint32_t* r) {
-#pragma unroll
-                            for (int b = 0; b < kB; ++b) {
-                                if (r[b] == NONE) continue;
-                                const Real val = Real(from_fixed(fx[r[b]], __ldg(p.deg + r[b])));
-                                pvec[r[b]] = val;
-                                fx[r[b]] = 0ull;
-                                vis[r[b]] = 0;
-                                mx = std_max(mx, val);
-                                mn = std_min(mn, val);
-                            }
-                        });
-                }
                 __syncwarp();
                 lap(1);
                 // preds[row] += (pvec[src] - pvec[adj]) / ds (:235-237); the first round adds to the
@@ -2480,7 +2170,7 @@ source_kernel(Pack pk) {
                     const Real ps = pvec[src];
                     struct SlotPred {
                         uint32_t w;
-                        Acc old;
+                        Real old;
                     };
                     pipelined<SlotPred>(dsi,
                         [&](uint32_t c, SlotPred* r) {
@@ -2500,12 +2190,11 @@ source_kernel(Pack pk) {
                             for (int b = 0; b < kB; ++b)
                                 if (r[b].w != NONE)
                                     p.preds[rb + c + 32 * b + lane] =
-                                        row_update<Real, Acc>(r[b].old, ps, pvec[r[b].w], ds);
+                                        row_update<Real, Real>(r[b].old, ps, pvec[r[b].w], ds);
                         });
                 }
                 // clear the new frontier's flags and take its residual max / min (:484-491; max and
-                // min do not depend on order); the Jacobi push did this with its new residuals
-                if constexpr (!JACOBI) {
+                // min do not depend on order)
                 mx = Real(0);
                 mn = Real(1);
                 pipelined<uint32_t>(qns,
@@ -2526,7 +2215,6 @@ source_kernel(Pack pk) {
                             mn = std_min(mn, val);
                         }
                     });
-                }
                 __syncwarp();
                 { uint32_t* tmp = q; q = qn; qn = tmp; }
                 qs = qns;
@@ -2539,7 +2227,7 @@ source_kernel(Pack pk) {
             dirty = true;
             break;
         }
-        if (!p.pre) st_rounds += ell;  // PrePush rounds are counted by push_block_kernel
+        st_rounds += ell;
         if (p.trace_ell && lane == 0) p.trace_ell[src] = uint32_t(ell);
 
         // slots that still need walks (rest = tau - ell > 0), compacted in slot order
@@ -2569,90 +2257,7 @@ source_kernel(Pack pk) {
             uint32_t* set = qn;  // free after the last swap
             int sc = 0;
             Real gamma_max;
-            const bool from_col = !SMEM && p.pre != nullptr;  // select from the column
-            if (p.gamma < nnz && from_col) {
-                Real t;
-                int need_eq;
-                // top-gamma threshold and, for gamma <= kTopK, the list of the only entries that
-                // can reach it (in index order, into q, free in this mode): the set is then taken
-                // from that list instead of a second pass over the column
-                const bool use_cand = rg <= kTopK;
-                uint32_t nc = 0;
-                kth_largest_col<Real>(pvec, n, rg, t, need_eq, use_cand ? q : nullptr, &nc);
-                int taken_eq = 0;
-                __syncwarp();
-                if (use_cand) {
-                    pipelined<uint32_t>(nc,
-                        [&](uint32_t i0, uint32_t* r) {
-#pragma unroll
-                            for (int b = 0; b < kB; ++b) {
-                                const uint32_t i = i0 + 32 * b + lane;
-                                r[b] = i < nc ? q[i] : NONE;
-                            }
-                        },
-                        [&](uint32_t, const uint32_t* r) {
-#pragma unroll
-                            for (int b = 0; b < kB; ++b) {
-                                const bool valid = r[b] != NONE;
-                                const Real v = valid ? pvec[r[b]] : Real(0);
-                                const Real x = v > Real(0) ? v : Real(-INFINITY);
-                                const bool gt = valid && x > t, eq = valid && x == t;
-                                const unsigned be = __ballot_sync(kFullMask, eq);
-                                const bool take_eq = eq && taken_eq + __popc(be & lt) < need_eq;
-                                const bool take = (gt || take_eq) && sc < rg;
-                                const unsigned bt = __ballot_sync(kFullMask, take);
-                                if (take) set[sc + __popc(bt & lt)] = r[b];
-                                sc += __popc(bt);
-                                taken_eq += __popc(__ballot_sync(kFullMask, take_eq));
-                            }
-                        });
-                } else
-                pipelined<Real>(n,
-                    [&](uint32_t i0, Real* r) {
-#pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const uint32_t i = i0 + 32 * b + lane;
-                            r[b] = i < n ? pvec[i] : Real(0);
-                        }
-                    },
-                    [&](uint32_t i0, const Real* r) {
-#pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const uint32_t i = i0 + 32 * b + lane;
-                            const Real x = r[b] > Real(0) ? r[b] : Real(-INFINITY);
-                            const bool gt = x > t, eq = x == t;
-                            const unsigned be = __ballot_sync(kFullMask, eq);
-                            const bool take_eq = eq && taken_eq + __popc(be & lt) < need_eq;
-                            const bool take = (gt || take_eq) && sc < rg;
-                            const unsigned bt = __ballot_sync(kFullMask, take);
-                            if (take) set[sc + __popc(bt & lt)] = i;
-                            sc += __popc(bt);
-                            taken_eq += __popc(__ballot_sync(kFullMask, take_eq));
-                        }
-                    });
-                gamma_max = std_min(Real(1), t);
-            } else if (from_col) {
-                // every frontier vertex is in the set: the column's positive entries in order
-                pipelined<Real>(n,
-                    [&](uint32_t i0, Real* r) {
-#pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const uint32_t i = i0 + 32 * b + lane;
-                            r[b] = i < n ? pvec[i] : Real(0);
-                        }
-                    },
-                    [&](uint32_t i0, const Real* r) {
-#pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const uint32_t i = i0 + 32 * b + lane;
-                            const bool nz = r[b] > Real(0);
-                            const unsigned bal = __ballot_sync(kFullMask, nz);
-                            if (nz) set[sc + __popc(bal & lt)] = i;
-                            sc += __popc(bal);
-                        }
-                    });
-                gamma_max = Real(0);
-            } else if (p.gamma < nnz) {
+            if (p.gamma < nnz) {
                 Real t;
                 int need_eq;
                 kth_largest<Real>(q, qs, pvec, rg, t, need_eq);
@@ -2855,34 +2460,7 @@ source_kernel(Pack pk) {
         lap(5);
 
         // ---- 2-way bouquet walks (:241-391): four bouquets per warp, one per 8-lane group ----
-        if (nitems && p.walk_queue) {
-            // handed to walk_queue_kernel / heavy_walk_kernel (the same walks, lanes and adds;
-            // more warps in flight)
-            for (uint32_t c = 0; c < nitems; c += 32) {
-                const uint32_t i = c + lane;
-                const bool has = i < nitems;
-                WalkItem w{};
-                bool heavy = false;
-                if (has) {
-                    w = items[i];
-                    w.pad = entry;
-                    heavy = w.nr >= kHeavyNr && w.len <= kHeavyLen;
-                }
-                const unsigned bh = __ballot_sync(kFullMask, has && heavy);
-                const unsigned bl = __ballot_sync(kFullMask, has && !heavy);
-                unsigned lb = 0, hb = 0;
-                if (lane == 0) {
-                    if (bl) lb = atomicAdd(p.walk_count, unsigned(__popc(bl)));
-                    if (bh) hb = atomicAdd(p.walk_count + 2, unsigned(__popc(bh)));
-                }
-                lb = __shfl_sync(kFullMask, lb, 0);
-                hb = __shfl_sync(kFullMask, hb, 0);
-                if (has) {
-                    if (heavy) p.walk_queue[p.walk_cap - 1u - (hb + __popc(bh & lt))] = w;
-                    else p.walk_queue[lb + __popc(bl & lt)] = w;
-                }
-            }
-        } else if (nitems) {
+        if (nitems) {
             const uint32_t j = lane & 7, grp = lane >> 3;
             uint32_t next = 0;
             bool has = false, start = false, primary = true;
@@ -2963,23 +2541,14 @@ source_kernel(Pack pk) {
                         x = radd(x, rsub(pa, pb));
                         pend = false;
                     }
-                    if constexpr (std::is_same<Real, Acc>::value) {
-                        // the eight lanes summed 0..7, then preds += xij / (ds * nr) (:386-390, :525)
-                        Real s = Real(0);
+                    // the eight lanes summed 0..7, then preds += xij / (ds * nr) (:386-390, :525)
+                    Real s = Real(0);
 #pragma unroll
-                        for (int b = 0; b < 8; ++b)
-                            s = radd(s, __shfl_sync(kFullMask, x, int(grp * 8 + b)));
-                        if (item_done && j == 0)
-                            p.preds[it.pos] =
-                                radd(p.preds[it.pos], rdiv(s, rmul(ds, from_u64<Real>(it.nr))));
-                    } else {
-                        double s = 0;
-#pragma unroll
-                        for (int b = 0; b < 8; ++b)
-                            s += double(__shfl_sync(kFullMask, x, int(grp * 8 + b)));
-                        if (item_done && j == 0)
-                            p.preds[it.pos] += s / (double(ds) * double(it.nr));
-                    }
+                    for (int b = 0; b < 8; ++b)
+                        s = radd(s, __shfl_sync(kFullMask, x, int(grp * 8 + b)));
+                    if (item_done && j == 0)
+                        p.preds[it.pos] =
+                            radd(p.preds[it.pos], rdiv(s, rmul(ds, from_u64<Real>(it.nr))));
                     if (item_done) has = false;
                 }
             }
@@ -2987,13 +2556,6 @@ source_kernel(Pack pk) {
         lap(6);
         // ---- next source starts from an all-zero residual vector ----
         __syncwarp();
-        if (!SMEM && p.pre) {
-            // the residual vector was the block push's column, read in place: the warp's own
-            // vector is untouched (and the flags used by the edge bound are back to zero)
-            pvec = p0.pvec_g + gw * size_t(sn);
-            lap(7);
-            continue;
-        }
         pipelined<uint32_t>(qs,
             [&](uint32_t i0, uint32_t* r) {
 #pragma unroll
@@ -3016,9 +2578,9 @@ source_kernel(Pack pk) {
 }
 
 // ---- walks of the block push's sources, as their own launch --------------------------------------
-// In PrePush mode the source kernel (a large kernel: 3 four-warp blocks per SM) leaves each
-// source's walking slots in a queue; this lean kernel walks them with many more warps in flight.
-// Everything a lane computes is what the source kernel's walk loop computes for the same item:
+// After a block push the per-source stage leaves each source's walking slots in a queue; this lean
+// kernel walks them with many more warps in flight.  Everything a lane computes is what the
+// per-source kernel's walk loop computes for the same item:
 // an 8-lane group takes one item, lane j walks the item's walks j, j + 8, ... in order over the
 // source's residual column, each hop's residual difference added to x in hop order, then the
 // group's eight x are summed in lane order into preds[slot] (src/aesc.h:241-391, 524-525).
@@ -3231,6 +2793,8 @@ __global__ void __launch_bounds__(kHeavyThreads) heavy_walk_kernel(const WalkQue
     if (lane == 0) stat_add(q.stats, kStFallback, st_fb);
 }
 
+#include "mixed_source.cuh"
+
 // ---- stage 3: symmetrise (src/aesc.h:532-550) -----------------------------------------------------
 // score[q] = p[q] + p[q'] with q' the slot that lands on q (sym_src; none in a row without its
 // reverse).  p comes from the source kernel for listed rows, and in closed form for the others:
@@ -3365,7 +2929,7 @@ __global__ void list_all_rows_kernel(RowMarks rm, uint32_t n) {
 RowMarks begin_row_marks(tgtp_graph* g) {
     grow(g, g->row_list, sizeof(uint32_t) * (g->n + 1));
     RowMarks rm;
-    rm.mark = run_work(g) + 4;
+    rm.mark = run_work(g) + kWorkWords;
     rm.list = g->row_list.as<uint32_t>();
     rm.len = run_work(g) + 2;
     rm.epoch = 1;
@@ -3425,11 +2989,10 @@ namespace {
 // Symmetrisation of one run (stage 3) on the graph's stream.
 template <class Real, class Acc>
 void launch_finish(tgtp_graph* g, float* out) {
-    const RowMarks rm{run_work(g) + 4, g->row_list.as<uint32_t>(), run_work(g) + 2, 1u};
     ScopedKernel k(g->prof, g->stream, "finish");
     launch(finish_kernel<Real, Acc>, grid_cap(g->m, 256, g->num_sms, 8), 256, 0, g->stream, true,
            g->preds.as<Acc>(), g->sym_src.as<uint32_t>(), g->row_of.as<uint32_t>(),
-           g->adjd.as<uint2>(), g->deg.as<uint32_t>(), rm.mark, rm.epoch, g->m, out,
+           g->adjd.as<uint2>(), g->deg.as<uint32_t>(), run_work(g) + kWorkWords, 1u, g->m, out,
            g->stats.as<unsigned long long>());
     TGTP_LAUNCH_CHECK("finish_kernel");
 }
@@ -3448,7 +3011,7 @@ struct BatchEntry {
     float* out;
     int key;    // form_key of the run
     bool smem;  // residual vectors in shared memory
-    std::vector<unsigned char> params;  // the run's SourceParams<Real, Acc>
+    std::vector<unsigned char> params;  // the run's SourceParams<Real> or MixedParams
 };
 struct BatchGroup {
     int key;
@@ -3463,9 +3026,8 @@ struct BatchPlan {
 namespace {
 thread_local BatchPlan* t_collect = nullptr;
 
-template <class Real, class Acc>
-bool defer_to_batch(tgtp_graph* g, const tgtp_config& cfg, float* out, bool smem,
-                    const SourceParams<Real, Acc>& p) {
+template <class Params>
+bool defer_to_batch(tgtp_graph* g, const tgtp_config& cfg, float* out, bool smem, const Params& p) {
     if (!t_collect) return false;
     BatchEntry e;
     e.g = g;
@@ -3478,18 +3040,489 @@ bool defer_to_batch(tgtp_graph* g, const tgtp_config& cfg, float* out, bool smem
     return true;
 }
 
-// One tgtp() run.  Real = residual / eigen projection type, Acc = score accumulator,
 // Whether a warp's FP32 residual vector and flags (the mixed form's) exceed the 112 KB of the
-// shared-memory tier, so that the per-warp push works on vectors in HBM.
+// shared-memory tier the mixed form's pushes had per warp; the learned push choice keeps to it.
 bool mixed_beyond_smem(uint64_t n) {
     return ((n * 4 + 15) & ~uint64_t(15)) + ((n + 15) & ~uint64_t(15)) + kAccBytes > uint64_t(112) * 1024;
 }
 void poll_push_hint(tgtp_graph* g);
 void post_push_hint(tgtp_graph* g, int key, double eps);
 
-// JACOBI = mixed form (lane-parallel tau over Vec storage, frontier-parallel push).
-template <class Real, class Acc, bool JACOBI, class Vec>
+// How a mixed run pushes.
+struct MixedPlan {
+    bool block_mode = false, shared_push = false;
+    uint32_t block_ctas = 0, wave_cap = 0, waves = 0;
+};
+MixedPlan plan_mixed(tgtp_graph* g, const tgtp_config& cfg) {
+    const uint64_t n = g->n;
+    const int key = form_key(cfg);
+    MixedPlan p;
+    poll_push_hint(g);
+    // mixed form, residual vectors too large for shared memory: multi-source push in waves of
+    // block_ctas x kBlockCols listed sources (each wave has its own claim counter)
+    // The block push gives the same bits as the per-warp push (fixed-point residual sums), so the
+    // choice is only about speed: the handle's tuned layout, else TGTP_MIXED_BLOCK, else what the
+    // last completed mixed run on this graph at this epsilon measured (push_hint), else the block
+    // push for
+    // vectors beyond shared memory at eps <= 0.01 (deep pushes: the block push was the faster one
+    // on every such graph measured) and the per-warp push otherwise.
+    if (g->src_layout[key]) p.block_mode = (g->src_layout[key] & kLayoutBlock) != 0;
+    else if (const char* e = std::getenv("TGTP_MIXED_BLOCK")) p.block_mode = std::atoi(e) != 0;
+    else if (g->push_hint[key] && g->push_hint_eps[key] == cfg.epsilon)
+        p.block_mode = g->push_hint[key] == 2;
+    else p.block_mode = mixed_beyond_smem(n) && cfg.epsilon <= 0.01;
+    // Graphs whose sums fit in shared memory push one source per block (push_shared_kernel), all
+    // listed sources in waves of at most 4 GiB of residual vectors; a knob of the 32-source block
+    // push asks for that one.  Sparse Chung-Lu graph (n = 25,860), eps = 0.005 / 0.05: push 208 / 109 ms
+    // with the 32-source block push (six waves), 79 / 19 ms with this one (its inner loop takes 55 ms of the 79:
+    // 21.6e9 additions of two shared atomics each).
+    const bool block_knob = std::getenv("TGTP_BLOCK_CTAS") || std::getenv("TGTP_BLOCK_ROUNDS") ||
+                            std::getenv("TGTP_BLOCK_MASKS") || std::getenv("TGTP_BLOCK_LIST_DIV");
+    p.shared_push = p.block_mode && push_shared_bytes(n) <= size_t(227) * 1024 && !block_knob;
+    const uint32_t shared_wave =
+        uint32_t(std::min<uint64_t>(n, std::max<uint64_t>(1, (uint64_t(4) << 30) / (sizeof(float) * n))));
+    // CTAs of the 32-source block push: one per SM, within a budget for their residual blocks of 24 GB or
+    // half the device memory free now (beside what the blocks already hold), whichever is larger
+    // (TGTP_BLOCK_CTAS lowers the count, e.g. to exercise many waves on small graphs)
+    p.block_ctas = uint32_t(g->num_sms);
+    if (p.block_mode && !p.shared_push) {
+        const size_t per_cta = 2 * size_t(n) * kBlockCols * sizeof(float);
+        size_t free_b = 0, total_b = 0;
+        TGTP_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        const size_t budget = std::max(size_t(24) << 30, (free_b + g->block_cols.bytes) / 2);
+        p.block_ctas = uint32_t(std::max<size_t>(1, std::min<size_t>(p.block_ctas, budget / per_cta)));
+        if (const char* e = std::getenv("TGTP_BLOCK_CTAS"))
+            p.block_ctas = std::max(1u, std::min(p.block_ctas, uint32_t(std::atoi(e))));
+    }
+    p.wave_cap = p.shared_push ? shared_wave : p.block_ctas * kBlockCols;
+    p.waves = p.block_mode ? uint32_t((n + uint64_t(p.wave_cap) - 1) / p.wave_cap) : 0u;
+    return p;
+}
+
+// Blocks of the mixed form's per-source kernel in one of its modes over up to n vertices.
+struct MixedLayout {
+    unsigned blocks, threads;
+    size_t smem, list_bytes, item_bytes, sum_bytes, touched_bytes, bit_bytes;
+    size_t scratch() const { return list_bytes + item_bytes + sum_bytes + touched_bytes + bit_bytes + 256; }
+};
+template <class Pack>
+const void* mixed_kernel(int mode) {
+    return mode == kShared   ? reinterpret_cast<const void*>(mixed_source_kernel<kShared, Pack>)
+           : mode == kGlobal ? reinterpret_cast<const void*>(mixed_source_kernel<kGlobal, Pack>)
+                             : reinterpret_cast<const void*>(mixed_source_kernel<kColumn, Pack>);
+}
+template <class Pack>
+MixedLayout mixed_layout(int mode, uint64_t n, uint64_t max_degree, uint64_t rows, int num_sms) {
+    MixedLayout l;
+    l.smem = mixed_shared_bytes(mode, n);
+    // about 1,024 resident threads per SM (64 registers each): as many sources at once as shared
+    // memory holds vectors of; in HBM two.  Threads per block in HBM, Chung-Lu n = 200,000 / 60,000,
+    // eps = 0.05, ms: 128 166 / 12.6, 256 143.9 / 11.6, 512 143.5 / 10.9, 1,024 158 / 15.2 (fewer
+    // sources at once wait for each other's barriers, more push each other's words out of L2)
+    if (mode == kShared)
+        l.threads = l.smem > size_t(113) * 1024 ? 1024u : (l.smem > size_t(56) * 1024 ? 512u : (l.smem > size_t(28) * 1024 ? 256u : 128u));
+    else
+        l.threads = mode == kGlobal ? 512u : 256u;
+    const int per_sm = blocks_per_sm(mixed_kernel<Pack>(mode), int(l.threads), l.smem);
+    if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "source kernel does not fit on an SM");
+    l.blocks = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(num_sms) * per_sm, rows)));
+    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
+    l.list_bytes = mode == kColumn ? 0 : align(sizeof(uint4) * size_t(n) * l.blocks);
+    l.item_bytes = align(sizeof(WalkItem) * std::max<uint64_t>(max_degree, 1) * l.blocks);
+    l.sum_bytes = mode == kGlobal ? align(sizeof(unsigned long long) * size_t(n) * l.blocks) : 0;
+    l.touched_bytes = mode == kGlobal ? align(sizeof(uint32_t) * size_t(n) * l.blocks) : 0;
+    l.bit_bytes = mode == kGlobal && 4 * mixed_words(n) > kBitsInSmem ? align(4 * mixed_words(n) * l.blocks) : 0;
+    return l;
+}
+void carve_mixed(MixedParams& p, const MixedLayout& l, unsigned char* base, uint64_t n, uint64_t max_degree) {
+    p.scratch_n = uint32_t(n);
+    p.max_degree = uint32_t(std::max<uint64_t>(max_degree, 1));
+    p.lists = l.list_bytes ? reinterpret_cast<uint4*>(base) : nullptr;
+    base += l.list_bytes;
+    p.items = reinterpret_cast<WalkItem*>(base);
+    base += l.item_bytes;
+    p.sums = l.sum_bytes ? reinterpret_cast<unsigned long long*>(base) : nullptr;
+    base += l.sum_bytes;
+    p.touched = l.touched_bytes ? reinterpret_cast<uint32_t*>(base) : nullptr;
+    base += l.touched_bytes;
+    p.gbits = l.bit_bytes ? reinterpret_cast<uint32_t*>(base) : nullptr;
+}
+template <class Pack>
+void launch_mixed(int mode, const MixedLayout& l, cudaStream_t s, bool pdl, const Pack& pk) {
+    if (mode == kShared) launch(mixed_source_kernel<kShared, Pack>, l.blocks, l.threads, l.smem, s, pdl, pk);
+    else if (mode == kGlobal) launch(mixed_source_kernel<kGlobal, Pack>, l.blocks, l.threads, l.smem, s, pdl, pk);
+    else launch(mixed_source_kernel<kColumn, Pack>, l.blocks, l.threads, l.smem, s, pdl, pk);
+    TGTP_LAUNCH_CHECK("mixed_source_kernel");
+}
+
+// Per-source stage of the mixed form; false when it is left to a batch.
+bool run_mixed(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMarks& rm, const MixedPlan& mp,
+               double logmd) {
+    cudaStream_t s = g->stream;
+    const uint64_t n = g->n, m = g->m;
+    const int key = form_key(cfg);
+    auto* stats = g->stats.as<unsigned long long>();
+    auto* work = run_work(g);
+    // sums in shared memory while they fit (the tuned layout's tier, else TGTP_PVEC_TIER)
+    int mode = kColumn;
+    if (!mp.block_mode) {
+        bool shared = mixed_fits_shared(n);
+        if (g->src_layout[key]) shared = shared && (g->src_layout[key] & kLayoutSmem) != 0;
+        else if (const char* t = std::getenv("TGTP_PVEC_TIER")) shared = shared && std::string(t) != "global";
+        mode = shared ? kShared : kGlobal;
+    }
+    const MixedLayout lay = mixed_layout<MixedPack<1>>(mode, n, g->max_degree, n, g->num_sms);
+    grow(g, g->scratch, lay.scratch());
+    MixedParams p{};
+    carve_mixed(p, lay, g->scratch.as<unsigned char>(), n, g->max_degree);
+    p.idx = g->idx.as<uint32_t>();
+    p.adj = g->adj.as<uint32_t>();
+    p.adjd = g->adjd.as<uint2>();
+    p.dinv = g->dinv.as<double>();
+    p.n = uint32_t(n);
+    p.taus = g->taus.as<int>();
+    p.preds = g->preds.as<double>();
+    p.work = work;
+    p.rows = rm.list;
+    p.eps = cfg.epsilon;
+    p.logmd = logmd;
+    p.gamma = cfg.gamma;
+    p.stats = stats;
+    p.budget_ns = deadline_from_env();
+    if (g->trace_on) {
+        grow(g, g->trace, sizeof(uint32_t) * (m + n));
+        TGTP_CUDA(cudaMemsetAsync(g->trace.ptr, 0, sizeof(uint32_t) * (m + n), s));
+        p.trace_nr = g->trace.as<uint32_t>();
+        p.trace_ell = p.trace_nr + m;
+        g->trace_valid = true;
+    }
+    // the per-block "sums are zero" marks hold only for the same carving of the same scratch
+    {
+        const uint64_t sig[5] = {uint64_t(key) | (uint64_t(mode) << 8) | (uint64_t(1) << 63), lay.blocks, uint64_t(n),
+                                 uint64_t(reinterpret_cast<uintptr_t>(g->scratch.ptr)),
+                                 uint64_t(g->scratch.bytes)};
+        grow(g, g->wclean, lay.blocks + 16);
+        if (std::memcmp(sig, g->wclean_sig, sizeof(sig)) != 0) {
+            TGTP_CUDA(cudaMemsetAsync(g->wclean.ptr, 0, lay.blocks + 16, s));
+            std::memcpy(g->wclean_sig, sig, sizeof(sig));
+        }
+        p.clean = g->wclean.as<unsigned char>();
+    }
+    MixedPack<1> pk;
+    pk.count = 1;
+    if (!mp.block_mode) {
+        p.claim = work;
+        if (defer_to_batch(g, cfg, out, mode == kShared, p)) return false;
+        pk.g[0] = p;
+        ScopedKernel k(g->prof, s, "source");
+        launch_mixed(mode, lay, s, true, pk);
+        return true;
+    }
+    grow(g, g->block_pre, sizeof(PrePush) * (n + 1));
+    PushBlockParams bp;
+    PushSharedParams sp;
+    size_t bsm = 0;
+    unsigned push_blocks = mp.block_ctas;
+    unsigned push_threads = 1024u;
+    if (mp.shared_push) {
+        // the block's threads by its shared memory: 1,024 resident threads per SM
+        bsm = push_shared_bytes(n);
+        push_threads = bsm > size_t(113) * 1024 ? 1024u : (bsm > size_t(56) * 1024 ? 512u : 256u);
+        const int per_sm =
+            blocks_per_sm(reinterpret_cast<const void*>(push_shared_kernel), int(push_threads), bsm);
+        if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "block push does not fit on an SM");
+        push_blocks = unsigned(std::min<uint64_t>(uint64_t(g->num_sms) * per_sm, mp.wave_cap));
+        grow(g, g->block_cols, sizeof(float) * size_t(n) * mp.wave_cap);
+        grow(g, g->block_lists, sizeof(uint4) * size_t(n) * push_blocks + 16);
+        sp.idx = p.idx;
+        sp.adj = p.adj;
+        sp.adjd = p.adjd;
+        sp.dinv = g->dinv.as<double>();
+        sp.n = uint32_t(n);
+        sp.taus = p.taus;
+        sp.preds = p.preds;
+        sp.work = work;
+        sp.eps = cfg.epsilon;
+        sp.logmd = logmd;
+        sp.lists = g->block_lists.as<uint4>();
+        sp.cols = g->block_cols.as<float>();
+        sp.pre = g->block_pre.as<PrePush>();
+        sp.stats = stats;
+        sp.budget_ns = p.budget_ns;
+        sp.cap = mp.wave_cap;
+    } else {
+        grow(g, g->block_cols, 2 * size_t(n) * kBlockCols * sizeof(float) * mp.block_ctas);
+        grow(g, g->block_final, sizeof(uint32_t) * (mp.block_ctas + 1));
+        bp.idx = p.idx;
+        bp.adj = p.adj;
+        bp.deg = g->deg.as<uint32_t>();
+        bp.adjd = p.adjd;
+        bp.n = uint32_t(n);
+        bp.taus = p.taus;
+        bp.preds = p.preds;
+        bp.work = work;
+        bp.rows = rm.list;
+        bp.eps = cfg.epsilon;
+        bp.logmd = logmd;
+        bp.cols = g->block_cols.as<float>();
+        bp.final_buf = g->block_final.as<uint32_t>();
+        bp.pre = g->block_pre.as<PrePush>();
+        bp.stats = stats;
+        bp.budget_ns = p.budget_ns;
+        // three row masks in shared memory while they fit beside the kernel's static 1.5 KB, else
+        // the current round's mask alone (n up to about 1.6 million), else none; the others in
+        // global memory; four row lists of n entries per CTA.  TGTP_BLOCK_MASKS=global|cur picks
+        // the placement of larger graphs on small ones.
+        const size_t mask_bytes = sizeof(uint32_t) * ((size_t(n) + 31) / 32);
+        const size_t bits_bytes = 3 * mask_bytes;
+        bp.bits = bits_bytes <= size_t(200) * 1024;
+        bp.cur_smem = !bp.bits && mask_bytes <= size_t(200) * 1024;
+        if (const char* e = std::getenv("TGTP_BLOCK_MASKS")) {
+            if (std::string(e) == "global") bp.bits = bp.cur_smem = false;
+            else if (std::string(e) == "cur") {
+                bp.bits = false;
+                bp.cur_smem = true;
+            }
+        }
+        bsm = bp.bits ? bits_bytes : (bp.cur_smem ? mask_bytes : 0);
+        if (!bp.bits) grow(g, g->block_bits, bits_bytes * mp.block_ctas + 16);
+        bp.gbits = bp.bits ? nullptr : g->block_bits.as<uint32_t>();
+        grow(g, g->block_lists, sizeof(uint32_t) * 4 * size_t(n) * mp.block_ctas + 16);
+        bp.lists = g->block_lists.as<uint32_t>();
+        bp.m = m;
+        // a round is compacted when its live rows' degree sum is below m / list_div (the tuned
+        // layout's threshold, else TGTP_BLOCK_LIST_DIV, else 4); TGTP_BLOCK_ROUNDS=compact|full
+        // fixes the choice (the values do not depend on it)
+        bp.list_div = layout_list_div(g->src_layout[key]);
+        if (const char* e = std::getenv("TGTP_BLOCK_LIST_DIV"))
+            if (!g->src_layout[key]) bp.list_div = uint32_t(std::atoi(e));
+        bp.rounds_mode = bp.list_div == 0 ? 2 : 0;
+        if (const char* e = std::getenv("TGTP_BLOCK_ROUNDS")) {
+            if (std::string(e) == "compact") bp.rounds_mode = 1;
+            else if (std::string(e) == "full") bp.rounds_mode = 2;
+        }
+        if (bsm) (void)blocks_per_sm(reinterpret_cast<const void*>(push_block_kernel), 1024, bsm);
+    }
+    p.pre = g->block_pre.as<PrePush>();
+    p.pre_cols = g->block_cols.as<float>();
+    p.pre_final = mp.shared_push ? nullptr : g->block_final.as<uint32_t>();
+    // the listed rows ordered by their largest tau (unlisted rows sort last, key 0)
+    grow(g, g->block_keys, sizeof(uint32_t) * 4 * (n + 1));
+    uint32_t* rkey = g->block_keys.as<uint32_t>();
+    uint32_t* ids = rkey + (n + 1);
+    uint32_t* skey = ids + (n + 1);
+    uint32_t* sorted = skey + (n + 1);
+    size_t tbytes = 0;
+    TGTP_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tbytes, rkey, skey, ids, sorted,
+                                                        int(n), 0, 32, s));
+    grow(g, g->block_tmp, tbytes + 16);
+    {
+        ScopedKernel k(g->prof, s, "row_key");
+        launch(row_key_kernel, grid_cap(uint64_t(n) * 32, 256, g->num_sms, 8), 256u, size_t(0), s,
+               true, g->idx.as<uint32_t>(), g->taus.as<int>(), rm.mark, uint32_t(n), rkey, ids);
+        TGTP_LAUNCH_CHECK("row_key_kernel");
+    }
+    TGTP_CUDA(cub::DeviceRadixSort::SortPairsDescending(g->block_tmp.ptr, tbytes, rkey, skey, ids,
+                                                        sorted, int(n), 0, 32, s));
+    bp.rows = sp.rows = sorted;
+    p.rows = sorted;
+    unsigned* claims = work + kWorkWords + n + 1;
+    // the walks of each wave's sources: a queue of (slot, its source's list entry) items that
+    // walk_queue_kernel works through (a wave's sources hold at most m slots), and per wave a
+    // queue length and a claim counter
+    grow(g, g->walk_queue, sizeof(WalkItem) * (m + 1));
+    grow(g, g->walk_ctl, sizeof(unsigned) * 4 * (mp.waves + 1));
+    unsigned* ctl = g->walk_ctl.as<unsigned>();
+    TGTP_CUDA(cudaMemsetAsync(ctl, 0, sizeof(unsigned) * 4 * (mp.waves + 1), s));
+    p.walk_queue = g->walk_queue.as<WalkItem>();
+    p.walk_cap = uint32_t(m + 1);
+    WalkQueueParams wq;
+    wq.idx = p.idx;
+    wq.adj = p.adj;
+    wq.rows = sorted;
+    wq.pre_cols = p.pre_cols;
+    wq.pre_final = p.pre_final;
+    wq.n = uint32_t(n);
+    wq.preds = p.preds;
+    wq.items = p.walk_queue;
+    wq.stats = stats;
+    const int walk_per_sm =
+        blocks_per_sm(reinterpret_cast<const void*>(walk_queue_kernel), kWalkThreads, 0);
+    const unsigned walk_blocks = unsigned(g->num_sms) * unsigned(std::max(walk_per_sm, 1));
+    const int heavy_per_sm = blocks_per_sm(reinterpret_cast<const void*>(heavy_walk_kernel),
+                                           kHeavyThreads, kHeavySmem);
+    const unsigned heavy_blocks = unsigned(g->num_sms) * unsigned(std::max(heavy_per_sm, 1));
+    // These kernels run for milliseconds each, and the next one's blocks started early take slots
+    // from them: without programmatic dependent launch the whole run on the sparse Chung-Lu graph
+    // (n = 25,860, eps = 0.005) takes 95 ms, with it 109 ms.
+    for (uint32_t w = 0; w < mp.waves; ++w) {
+        bp.base = sp.base = w * mp.wave_cap;
+        {
+            ScopedKernel k(g->prof, s, "push_block");
+            if (mp.shared_push) {
+                sp.claim = claims + mp.waves + w;
+                launch(push_shared_kernel, push_blocks, push_threads, bsm, s, false, sp);
+            } else {
+                launch(push_block_kernel, mp.block_ctas, 1024u, bsm, s, false, bp);
+            }
+            TGTP_LAUNCH_CHECK("push_block_kernel");
+        }
+        p.claim = claims + w;
+        p.list_base = bp.base;
+        p.list_cap = mp.wave_cap;
+        p.walk_count = ctl + 4 * w;
+        pk.g[0] = p;
+        {
+            ScopedKernel k(g->prof, s, "source");
+            launch(mixed_source_kernel<kColumn, MixedPack<1>>, lay.blocks, lay.threads, lay.smem, s, false, pk);
+            TGTP_LAUNCH_CHECK("mixed_source_kernel");
+        }
+        wq.list_base = p.list_base;
+        wq.count = ctl + 4 * w;
+        wq.claim = ctl + 4 * w + 1;
+        {
+            ScopedKernel k(g->prof, s, "walk_queue");
+            launch(walk_queue_kernel, walk_blocks, unsigned(kWalkThreads), size_t(0), s, false, wq);
+            TGTP_LAUNCH_CHECK("walk_queue_kernel");
+        }
+        WalkQueueParams wh = wq;
+        wh.count = ctl + 4 * w + 2;
+        wh.claim = ctl + 4 * w + 3;
+        ScopedKernel k(g->prof, s, "heavy_walk");
+        launch(heavy_walk_kernel, heavy_blocks, unsigned(kHeavyThreads), kHeavySmem, s, false, wh,
+               uint32_t(m + 1));
+        TGTP_LAUNCH_CHECK("heavy_walk_kernel");
+    }
+    return true;
+}
+
+// Per-source stage of the parity forms; false when it is left to a batch.
+template <class Real>
+bool run_sources(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMarks& rm, bool multi, double logmd) {
+    cudaStream_t s = g->stream;
+    const uint64_t n = g->n, m = g->m;
+    const int key = form_key(cfg);
+    auto* stats = g->stats.as<unsigned long long>();
+    auto* work = run_work(g);
+    // source kernel.  Shared-memory tier: each warp's residual vector and flags in shared memory.
+    // Global tier (large n): vectors in HBM.  The layout (tier, warps per block) comes from the
+    // handle's tuned choice for this form, else from the default rule (shared memory with one-warp
+    // blocks while a warp's copy fits in 112 KB, else HBM with four warps per block);
+    // TGTP_PVEC_TIER=smem|global overrides the tier of the default rule.
+    const size_t pv_bytes = (size_t(n) * sizeof(Real) + 15) & ~size_t(15);
+    const size_t vis_bytes = (size_t(n) + 15) & ~size_t(15);
+    const size_t per_warp = pv_bytes + vis_bytes + kAccBytes;
+    bool use_smem;
+    int wpb;
+    if (g->src_layout[key]) {
+        use_smem = (g->src_layout[key] & kLayoutSmem) != 0;
+        wpb = std::max(1, g->src_layout[key] & 0xff);
+    } else {
+        use_smem = per_warp <= size_t(112) * 1024;
+        if (const char* t = std::getenv("TGTP_PVEC_TIER")) {
+            if (std::string(t) == "global") use_smem = false;
+            else if (std::string(t) == "smem" && per_warp <= size_t(227) * 1024) use_smem = true;
+        }
+        wpb = use_smem ? 1 : 4;
+    }
+    if (use_smem && per_warp * wpb > size_t(227) * 1024)
+        fail(TGTP_ERR_UNSUPPORTED, "source layout does not fit in shared memory");
+    const int threads = wpb * 32;
+    const size_t smem = use_smem ? per_warp * wpb : size_t(wpb) * kAccBytes;
+    using Pack1 = SourcePack<Real, 1>;
+    auto kern = use_smem ? source_kernel<Real, true, Pack1>
+                         : source_kernel<Real, false, Pack1>;
+    const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(kern), threads, smem);
+    if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "source kernel does not fit on an SM");
+    uint64_t blocks = uint64_t(g->num_sms) * per_sm;
+    blocks = std::min<uint64_t>(blocks, (n + wpb - 1) / wpb);
+    const uint64_t warps = blocks * wpb;
+    const size_t maxd = std::max<uint32_t>(g->max_degree, 1);
+    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t q_bytes = align(warps * 2 * size_t(n) * 4);
+    const size_t it_bytes = align(warps * maxd * sizeof(WalkItem));
+    const size_t pvg_bytes = use_smem ? 0 : align(warps * size_t(n) * sizeof(Real));
+    const size_t visg_bytes = use_smem ? 0 : align(warps * vis_bytes);
+    grow(g, g->scratch, q_bytes + it_bytes + pvg_bytes + visg_bytes + 256);
+    unsigned char* base = g->scratch.as<unsigned char>();
+    SourceParams<Real> p;
+    p.idx = g->idx.as<uint32_t>();
+    p.adj = g->adj.as<uint32_t>();
+    p.deg = g->deg.as<uint32_t>();
+    p.n = uint32_t(n);
+    p.taus = g->taus.as<int>();
+    p.preds = g->preds.as<Real>();
+    p.work = work;
+    p.rows = rm.list;
+    p.qbuf = reinterpret_cast<uint32_t*>(base);
+    base += q_bytes;
+    p.items = reinterpret_cast<WalkItem*>(base);
+    base += it_bytes;
+    p.pvec_g = use_smem ? nullptr : reinterpret_cast<Real*>(base);
+    base += pvg_bytes;
+    p.vis_g = use_smem ? nullptr : base;
+    // the per-warp "vectors are zero" marks hold only for the same carving of the same scratch
+    {
+        const uint64_t sig[5] = {uint64_t(key) | (uint64_t(use_smem) << 8) | (uint64_t(wpb) << 16),
+                                 blocks, uint64_t(n),
+                                 uint64_t(reinterpret_cast<uintptr_t>(g->scratch.ptr)),
+                                 uint64_t(g->scratch.bytes)};
+        grow(g, g->wclean, warps + 16);
+        if (std::memcmp(sig, g->wclean_sig, sizeof(sig)) != 0) {
+            TGTP_CUDA(cudaMemsetAsync(g->wclean.ptr, 0, warps + 16, s));
+            std::memcpy(g->wclean_sig, sig, sizeof(sig));
+        }
+        p.wclean = g->wclean.as<unsigned char>();
+    }
+    p.vis_stride = vis_bytes;
+    p.smem_per_warp = per_warp;
+    p.max_degree = uint32_t(maxd);
+    p.eps = cfg.epsilon;
+    p.logmd = logmd;
+    p.gamma = cfg.gamma;
+    p.stats = stats;
+    p.adjd = g->adjd.as<uint2>();
+    p.budget_ns = deadline_from_env();
+    p.trace_nr = p.trace_ell = nullptr;
+    if (g->trace_on) {
+        grow(g, g->trace, sizeof(uint32_t) * (m + n));
+        TGTP_CUDA(cudaMemsetAsync(g->trace.ptr, 0, sizeof(uint32_t) * (m + n), s));
+        p.trace_nr = g->trace.as<uint32_t>();
+        p.trace_ell = p.trace_nr + m;
+        g->trace_valid = true;
+    }
+    p.multi = multi;
+    p.scratch_n = uint32_t(n);
+    {
+        // The windowed push pays off when rows are short: several frontier vertices share a
+        // 32-entry step.  When rows average 32 entries or more, each vertex fills its steps anyway
+        // and adjacent frontier vertices cut windows often, so one vertex at a time is used
+        // (4,039-vertex Chung-Lu graph, 44 entries per row: 0.73 against 0.86 ms at eps = 0.01;
+        // sparse Chung-Lu, 9.3 per row: 4.1 against 1.4 s at eps = 0.005).  The tuned layout,
+        // then TGTP_GS_WINDOW=0/1, override the rule.
+        const uint16_t lay = g->src_layout[key];
+        const char* e = std::getenv("TGTP_GS_WINDOW");
+        if (lay & kLayoutWindow) p.gs_window = true;
+        else if (lay & kLayoutNoWindow) p.gs_window = false;
+        else if (e) p.gs_window = std::string(e) != "0";
+        else p.gs_window = m < 32 * n;
+    }
+    Pack1 pk;
+    pk.count = 1;
+    p.claim = work;
+    if (defer_to_batch(g, cfg, out, use_smem, p)) return false;
+    pk.g[0] = p;
+    ScopedKernel k(g->prof, s, "source");
+    launch(kern, unsigned(blocks), unsigned(threads), smem, s, true, pk);
+    TGTP_LAUNCH_CHECK("source_kernel");
+    return true;
+}
+
+// One tgtp() run.  Real = residual type, MIXED = the mixed form (scores accumulated in FP64), Vec =
+// eigenvector storage of the split tau kernels.
+template <class Real, bool MIXED, class Vec>
 void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
+    using Acc = typename std::conditional<MIXED, double, Real>::type;
     cudaStream_t s = g->stream;
     const uint64_t n = g->n, m = g->m;
     const uint32_t omega = uint32_t(cfg.omega);
@@ -3506,57 +3539,19 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
     grow(g, g->preds, sizeof(Acc) * (m + 1));
     // one zeroing for the striped counters, the work words and the row marks behind them
     const size_t stat_bytes = sizeof(unsigned long long) * kStCount * kStStripes;
-    // mixed form, residual vectors too large for shared memory: multi-source push in waves of
-    // block_ctas x kBlockCols listed sources (each wave has its own claim counter)
-    // The block push gives the same bits as the per-warp push (fixed-point residual sums), so the
-    // choice is only about speed: the handle's tuned layout, else TGTP_MIXED_BLOCK, else what the
-    // last completed mixed run on this graph at this epsilon measured (push_hint), else the block
-    // push for
-    // vectors beyond shared memory at eps <= 0.01 (deep pushes: the block push was the faster one
-    // on every such graph measured) and the per-warp push otherwise.
     const int key = form_key(cfg);
-    if (JACOBI) poll_push_hint(g);
-    bool block_mode = false;
-    if (g->src_layout[key]) block_mode = JACOBI && (g->src_layout[key] & kLayoutBlock) != 0;
-    else if (const char* e = std::getenv("TGTP_MIXED_BLOCK")) block_mode = JACOBI && std::atoi(e) != 0;
-    else if (g->push_hint[key] && g->push_hint_eps[key] == cfg.epsilon)
-        block_mode = JACOBI && g->push_hint[key] == 2;
-    else block_mode = JACOBI && mixed_beyond_smem(n) && cfg.epsilon <= 0.01;
+    MixedPlan mp;
+    if (MIXED) mp = plan_mixed(g, cfg);
     g->last_key = key;
     g->last_eps = cfg.epsilon;
-    // Graphs whose sums fit in shared memory push one source per block (push_shared_kernel), all
-    // listed sources in waves of at most 4 GiB of residual vectors; a knob of the 32-source block
-    // push asks for that one.  Sparse Chung-Lu graph (n = 25,860), eps = 0.005 / 0.05: push 208 / 109 ms
-    // with the 32-source block push (six waves), 79 / 19 ms with this one (its inner loop takes 55 ms of the 79:
-    // 21.6e9 additions of two shared atomics each).
-    const bool block_knob = std::getenv("TGTP_BLOCK_CTAS") || std::getenv("TGTP_BLOCK_ROUNDS") ||
-                            std::getenv("TGTP_BLOCK_MASKS") || std::getenv("TGTP_BLOCK_LIST_DIV");
-    const bool shared_push = block_mode && push_shared_bytes(n) <= size_t(227) * 1024 && !block_knob;
-    const uint32_t shared_wave =
-        uint32_t(std::min<uint64_t>(n, std::max<uint64_t>(1, (uint64_t(4) << 30) / (sizeof(float) * n))));
-    // CTAs of the 32-source block push: one per SM, within a budget for their residual blocks of 24 GB or
-    // half the device memory free now (beside what the blocks already hold), whichever is larger
-    // (TGTP_BLOCK_CTAS lowers the count, e.g. to exercise many waves on small graphs)
-    uint32_t block_ctas = uint32_t(g->num_sms);
-    if (block_mode && !shared_push) {
-        const size_t per_cta = 2 * size_t(n) * kBlockCols * sizeof(float);
-        size_t free_b = 0, total_b = 0;
-        TGTP_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        const size_t budget = std::max(size_t(24) << 30, (free_b + g->block_cols.bytes) / 2);
-        block_ctas = uint32_t(std::max<size_t>(1, std::min<size_t>(block_ctas, budget / per_cta)));
-        if (const char* e = std::getenv("TGTP_BLOCK_CTAS"))
-            block_ctas = std::max(1u, std::min(block_ctas, uint32_t(std::atoi(e))));
-    }
-    const uint32_t wave_cap = shared_push ? shared_wave : block_ctas * kBlockCols;
-    const uint32_t waves = block_mode ? uint32_t((n + uint64_t(wave_cap) - 1) / wave_cap) : 0u;
-    const size_t zero_bytes = stat_bytes + sizeof(unsigned) * (4 + n + 1 + 2 * size_t(waves));
+    const size_t zero_bytes = stat_bytes + sizeof(unsigned) * (kWorkWords + n + 1 + 2 * size_t(mp.waves));
     grow(g, g->stats, zero_bytes);
     auto* stats = g->stats.as<unsigned long long>();
     auto* work = run_work(g);
     TGTP_CUDA(cudaMemsetAsync(stats, 0, zero_bytes, s));
 
     const RowMarks rm = begin_row_marks(g);
-    const bool multi = !JACOBI && g->has_multi_edges;
+    const bool multi = !MIXED && g->has_multi_edges;
     if (multi) {
         // the reference leaves tau = 0 in the slots no forward edge writes (the later repeats of
         // a neighbour u < v in row v, src/aesc.h:179-209), and every row goes to the source kernel
@@ -3564,7 +3559,7 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
         list_all_rows_kernel<<<grid_cap(n, 256, g->num_sms, 8), 256, 0, s>>>(rm, uint32_t(n));
         TGTP_LAUNCH_CHECK("list_all_rows_kernel");
     }
-    if constexpr (JACOBI || std::is_same<Real, double>::value) {
+    if constexpr (MIXED || std::is_same<Real, double>::value) {
         // FP64 and mixed forms: eight lanes per edge over F64 / F32 / BF16 rows
         prepare_split_tables(g, omega);
         using Part = typename Split<Vec>::Part;
@@ -3658,320 +3653,19 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
             g->taus.as<int>(), rm, stats);
         TGTP_LAUNCH_CHECK("tau_kernel");
     }
-
-    // source kernel.  Shared-memory tier: each warp's residual vector and flags in shared memory.
-    // Global tier (large n): vectors in HBM.  The layout (tier, warps per block) comes from the
-    // handle's tuned choice for this form, else from the default rule (shared memory with one-warp
-    // blocks while a warp's copy fits in 112 KB, else HBM with four warps per block);
-    // TGTP_PVEC_TIER=smem|global overrides the tier of the default rule.
-    const size_t pv_bytes = (size_t(n) * sizeof(Real) + 15) & ~size_t(15);
-    const size_t vis_bytes = (size_t(n) + 15) & ~size_t(15);
-    const size_t fx_bytes = JACOBI ? sizeof(unsigned long long) * size_t(n) : 0;
-    // the mixed form's fixed-point accumulators join the shared-memory copy only while the three
-    // arrays fit in 112 KB; beyond that they move to HBM and the residual vector stays in shared
-    // memory up to the same size as in the other forms
-    const bool fx_in_smem = JACOBI && pv_bytes + vis_bytes + fx_bytes + kAccBytes <= size_t(112) * 1024;
-    const size_t per_warp = pv_bytes + vis_bytes + (fx_in_smem ? fx_bytes : 0) + kAccBytes;
-    bool use_smem;
-    int wpb;
-    if (g->src_layout[key]) {
-        use_smem = (g->src_layout[key] & kLayoutSmem) != 0;
-        wpb = std::max(1, g->src_layout[key] & 0xff);
+    if constexpr (MIXED) {
+        if (!run_mixed(g, cfg, out, rm, mp, logmd)) return;
     } else {
-        use_smem = per_warp <= size_t(112) * 1024;
-        if (const char* t = std::getenv("TGTP_PVEC_TIER")) {
-            if (std::string(t) == "global") use_smem = false;
-            else if (std::string(t) == "smem" && per_warp <= size_t(227) * 1024) use_smem = true;
-        }
-        wpb = use_smem ? 1 : 4;
-    }
-    if (use_smem && per_warp * wpb > size_t(227) * 1024)
-        fail(TGTP_ERR_UNSUPPORTED, "source layout does not fit in shared memory");
-    const int threads = wpb * 32;
-    const size_t smem = use_smem ? per_warp * wpb : size_t(wpb) * kAccBytes;
-    using Pack1 = SourcePack<Real, Acc, 1>;
-    auto kern = use_smem ? source_kernel<Real, Acc, true, JACOBI, Pack1>
-                         : source_kernel<Real, Acc, false, JACOBI, Pack1>;
-    const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(kern), threads, smem);
-    if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "source kernel does not fit on an SM");
-    uint64_t blocks = uint64_t(g->num_sms) * per_sm;
-    blocks = std::min<uint64_t>(blocks, (n + wpb - 1) / wpb);
-    const uint64_t warps = blocks * wpb;
-    const size_t maxd = std::max<uint32_t>(g->max_degree, 1);
-    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t q_bytes = align(warps * 2 * size_t(n) * 4);
-    const size_t it_bytes = align(warps * maxd * sizeof(WalkItem));
-    const size_t pvg_bytes = use_smem ? 0 : align(warps * size_t(n) * sizeof(Real));
-    const size_t visg_bytes = use_smem ? 0 : align(warps * vis_bytes);
-    const size_t fxg_bytes = (JACOBI && !(use_smem && fx_in_smem)) ? align(warps * fx_bytes) : 0;
-    grow(g, g->scratch, q_bytes + it_bytes + pvg_bytes + visg_bytes + fxg_bytes + 256);
-    unsigned char* base = g->scratch.as<unsigned char>();
-    SourceParams<Real, Acc> p;
-    p.idx = g->idx.as<uint32_t>();
-    p.adj = g->adj.as<uint32_t>();
-    p.deg = g->deg.as<uint32_t>();
-    p.n = uint32_t(n);
-    p.taus = g->taus.as<int>();
-    p.preds = g->preds.as<Acc>();
-    p.work = work;
-    p.rows = rm.list;
-    p.qbuf = reinterpret_cast<uint32_t*>(base);
-    base += q_bytes;
-    p.items = reinterpret_cast<WalkItem*>(base);
-    base += it_bytes;
-    p.pvec_g = use_smem ? nullptr : reinterpret_cast<Real*>(base);
-    base += pvg_bytes;
-    p.vis_g = use_smem ? nullptr : base;
-    base += visg_bytes;
-    p.fx_g = fxg_bytes ? reinterpret_cast<unsigned long long*>(base) : nullptr;
-    // the per-warp "vectors are zero" marks hold only for the same carving of the same scratch
-    {
-        const uint64_t sig[5] = {uint64_t(key) | (uint64_t(use_smem) << 8) | (uint64_t(wpb) << 16),
-                                 blocks, uint64_t(n),
-                                 uint64_t(reinterpret_cast<uintptr_t>(g->scratch.ptr)),
-                                 uint64_t(g->scratch.bytes)};
-        grow(g, g->wclean, warps + 16);
-        if (std::memcmp(sig, g->wclean_sig, sizeof(sig)) != 0) {
-            TGTP_CUDA(cudaMemsetAsync(g->wclean.ptr, 0, warps + 16, s));
-            std::memcpy(g->wclean_sig, sig, sizeof(sig));
-        }
-        p.wclean = g->wclean.as<unsigned char>();
-    }
-    p.vis_stride = vis_bytes;
-    p.smem_per_warp = per_warp;
-    p.max_degree = uint32_t(maxd);
-    p.eps = cfg.epsilon;
-    p.logmd = logmd;
-    p.gamma = cfg.gamma;
-    p.stats = stats;
-    p.adjd = g->adjd.as<uint2>();
-    p.budget_ns = deadline_from_env();
-    p.trace_nr = p.trace_ell = nullptr;
-    p.walk_queue = nullptr;
-    p.walk_count = nullptr;
-    p.walk_cap = 0;
-    if (g->trace_on) {
-        grow(g, g->trace, sizeof(uint32_t) * (m + n));
-        TGTP_CUDA(cudaMemsetAsync(g->trace.ptr, 0, sizeof(uint32_t) * (m + n), s));
-        p.trace_nr = g->trace.as<uint32_t>();
-        p.trace_ell = p.trace_nr + m;
-        g->trace_valid = true;
-    }
-    p.pre = nullptr;
-    p.pre_cols = nullptr;
-    p.pre_final = nullptr;
-    p.multi = multi;
-    p.scratch_n = uint32_t(n);
-    {
-        // The windowed push pays off when rows are short: several frontier vertices share a
-        // 32-entry step.  When rows average 32 entries or more, each vertex fills its steps anyway
-        // and adjacent frontier vertices cut windows often, so one vertex at a time is used
-        // (4,039-vertex Chung-Lu graph, 44 entries per row: 0.73 against 0.86 ms at eps = 0.01;
-        // sparse Chung-Lu, 9.3 per row: 4.1 against 1.4 s at eps = 0.005).  The tuned layout,
-        // then TGTP_GS_WINDOW=0/1, override the rule.
-        const uint16_t lay = g->src_layout[key];
-        const char* e = std::getenv("TGTP_GS_WINDOW");
-        if (lay & kLayoutWindow) p.gs_window = true;
-        else if (lay & kLayoutNoWindow) p.gs_window = false;
-        else if (e) p.gs_window = std::string(e) != "0";
-        else p.gs_window = m < 32 * n;
-    }
-    Pack1 pk;
-    pk.count = 1;
-    if (!block_mode) {
-        p.claim = work;
-        p.list_base = 0;
-        p.list_cap = uint32_t(n);
-        if (defer_to_batch<Real, Acc>(g, cfg, out, use_smem, p)) return;
-        pk.g[0] = p;
-        ScopedKernel k(g->prof, s, "source");
-        launch(kern, unsigned(blocks), unsigned(threads), smem, s, true, pk);
-        TGTP_LAUNCH_CHECK("source_kernel");
-    } else if constexpr (JACOBI) {  // the block push exists for the mixed form only
-        grow(g, g->block_pre, sizeof(PrePush) * (n + 1));
-        PushBlockParams bp;
-        PushSharedParams sp;
-        size_t bsm = 0;
-        unsigned push_blocks = block_ctas;
-        unsigned push_threads = 1024u;
-        if (shared_push) {
-            // the block's threads by its shared memory: 1,024 resident threads per SM
-            bsm = push_shared_bytes(n);
-            push_threads = bsm > size_t(113) * 1024 ? 1024u : (bsm > size_t(56) * 1024 ? 512u : 256u);
-            const int per_sm =
-                blocks_per_sm(reinterpret_cast<const void*>(push_shared_kernel), int(push_threads), bsm);
-            if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "block push does not fit on an SM");
-            push_blocks = unsigned(std::min<uint64_t>(uint64_t(g->num_sms) * per_sm, wave_cap));
-            grow(g, g->block_cols, sizeof(float) * size_t(n) * wave_cap);
-            grow(g, g->block_lists, sizeof(uint4) * size_t(n) * push_blocks + 16);
-            sp.idx = p.idx;
-            sp.adj = p.adj;
-            sp.adjd = p.adjd;
-            sp.dinv = g->dinv.as<double>();
-            sp.n = uint32_t(n);
-            sp.taus = p.taus;
-            sp.preds = reinterpret_cast<double*>(p.preds);
-            sp.work = work;
-            sp.eps = cfg.epsilon;
-            sp.logmd = logmd;
-            sp.lists = g->block_lists.as<uint4>();
-            sp.cols = g->block_cols.as<float>();
-            sp.pre = g->block_pre.as<PrePush>();
-            sp.stats = stats;
-            sp.budget_ns = p.budget_ns;
-            sp.cap = wave_cap;
-        } else {
-            grow(g, g->block_cols, 2 * size_t(n) * kBlockCols * sizeof(float) * block_ctas);
-            grow(g, g->block_final, sizeof(uint32_t) * (block_ctas + 1));
-            bp.idx = p.idx;
-            bp.adj = p.adj;
-            bp.deg = p.deg;
-            bp.adjd = p.adjd;
-            bp.n = uint32_t(n);
-            bp.taus = p.taus;
-            bp.preds = p.preds;
-            bp.work = work;
-            bp.rows = rm.list;
-            bp.eps = cfg.epsilon;
-            bp.logmd = logmd;
-            bp.cols = g->block_cols.as<float>();
-            bp.final_buf = g->block_final.as<uint32_t>();
-            bp.pre = g->block_pre.as<PrePush>();
-            bp.stats = stats;
-            bp.budget_ns = p.budget_ns;
-            // three row masks in shared memory while they fit beside the kernel's static 1.5 KB, else
-            // the current round's mask alone (n up to about 1.6 million), else none; the others in
-            // global memory; four row lists of n entries per CTA.  TGTP_BLOCK_MASKS=global|cur picks
-            // the placement of larger graphs on small ones.
-            const size_t mask_bytes = sizeof(uint32_t) * ((size_t(n) + 31) / 32);
-            const size_t bits_bytes = 3 * mask_bytes;
-            bp.bits = bits_bytes <= size_t(200) * 1024;
-            bp.cur_smem = !bp.bits && mask_bytes <= size_t(200) * 1024;
-            if (const char* e = std::getenv("TGTP_BLOCK_MASKS")) {
-                if (std::string(e) == "global") bp.bits = bp.cur_smem = false;
-                else if (std::string(e) == "cur") {
-                    bp.bits = false;
-                    bp.cur_smem = true;
-                }
-            }
-            bsm = bp.bits ? bits_bytes : (bp.cur_smem ? mask_bytes : 0);
-            if (!bp.bits) grow(g, g->block_bits, bits_bytes * block_ctas + 16);
-            bp.gbits = bp.bits ? nullptr : g->block_bits.as<uint32_t>();
-            grow(g, g->block_lists, sizeof(uint32_t) * 4 * size_t(n) * block_ctas + 16);
-            bp.lists = g->block_lists.as<uint32_t>();
-            bp.m = m;
-            // a round is compacted when its live rows' degree sum is below m / list_div (the tuned
-            // layout's threshold, else TGTP_BLOCK_LIST_DIV, else 4); TGTP_BLOCK_ROUNDS=compact|full
-            // fixes the choice (the values do not depend on it)
-            bp.list_div = layout_list_div(g->src_layout[key]);
-            if (const char* e = std::getenv("TGTP_BLOCK_LIST_DIV"))
-                if (!g->src_layout[key]) bp.list_div = uint32_t(std::atoi(e));
-            bp.rounds_mode = bp.list_div == 0 ? 2 : 0;
-            if (const char* e = std::getenv("TGTP_BLOCK_ROUNDS")) {
-                if (std::string(e) == "compact") bp.rounds_mode = 1;
-                else if (std::string(e) == "full") bp.rounds_mode = 2;
-            }
-            if (bsm) (void)blocks_per_sm(reinterpret_cast<const void*>(push_block_kernel), 1024, bsm);
-        }
-        p.pre = g->block_pre.as<PrePush>();
-        p.pre_cols = g->block_cols.as<float>();
-        p.pre_final = shared_push ? nullptr : g->block_final.as<uint32_t>();
-        // the listed rows ordered by their largest tau (unlisted rows sort last, key 0)
-        grow(g, g->block_keys, sizeof(uint32_t) * 4 * (n + 1));
-        uint32_t* key = g->block_keys.as<uint32_t>();
-        uint32_t* ids = key + (n + 1);
-        uint32_t* skey = ids + (n + 1);
-        uint32_t* sorted = skey + (n + 1);
-        size_t tbytes = 0;
-        TGTP_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tbytes, key, skey, ids, sorted,
-                                                            int(n), 0, 32, s));
-        grow(g, g->block_tmp, tbytes + 16);
-        {
-            ScopedKernel k(g->prof, s, "row_key");
-            launch(row_key_kernel, grid_cap(uint64_t(n) * 32, 256, g->num_sms, 8), 256u, size_t(0), s,
-                   true, g->idx.as<uint32_t>(), g->taus.as<int>(), rm.mark, uint32_t(n), key, ids);
-            TGTP_LAUNCH_CHECK("row_key_kernel");
-        }
-        TGTP_CUDA(cub::DeviceRadixSort::SortPairsDescending(g->block_tmp.ptr, tbytes, key, skey, ids,
-                                                            sorted, int(n), 0, 32, s));
-        bp.rows = sp.rows = sorted;
-        p.rows = sorted;
-        unsigned* claims = work + 4 + n + 1;
-        // the walks of each wave's sources: a queue of (slot, its source's list entry) items that
-        // walk_queue_kernel works through (a wave's sources hold at most m slots), and per wave a
-        // queue length and a claim counter
-        grow(g, g->walk_queue, sizeof(WalkItem) * (m + 1));
-        grow(g, g->walk_ctl, sizeof(unsigned) * 4 * (waves + 1));
-        unsigned* ctl = g->walk_ctl.as<unsigned>();
-        TGTP_CUDA(cudaMemsetAsync(ctl, 0, sizeof(unsigned) * 4 * (waves + 1), s));
-        p.walk_queue = g->walk_queue.as<WalkItem>();
-        p.walk_cap = uint32_t(m + 1);
-        WalkQueueParams wq;
-        wq.idx = p.idx;
-        wq.adj = p.adj;
-        wq.rows = sorted;
-        wq.pre_cols = p.pre_cols;
-        wq.pre_final = p.pre_final;
-        wq.n = uint32_t(n);
-        wq.preds = reinterpret_cast<double*>(p.preds);
-        wq.items = p.walk_queue;
-        wq.stats = stats;
-        const int walk_per_sm =
-            blocks_per_sm(reinterpret_cast<const void*>(walk_queue_kernel), kWalkThreads, 0);
-        const unsigned walk_blocks = unsigned(g->num_sms) * unsigned(std::max(walk_per_sm, 1));
-        const int heavy_per_sm = blocks_per_sm(reinterpret_cast<const void*>(heavy_walk_kernel),
-                                               kHeavyThreads, kHeavySmem);
-        const unsigned heavy_blocks = unsigned(g->num_sms) * unsigned(std::max(heavy_per_sm, 1));
-        // These kernels run for milliseconds each, and the next one's blocks started early take slots
-        // from them: without programmatic dependent launch the whole run on the sparse Chung-Lu graph
-        // (n = 25,860, eps = 0.005) takes 95 ms, with it 109 ms.
-        for (uint32_t w = 0; w < waves; ++w) {
-            bp.base = sp.base = w * wave_cap;
-            {
-                ScopedKernel k(g->prof, s, "push_block");
-                if (shared_push) {
-                    sp.claim = claims + waves + w;
-                    launch(push_shared_kernel, push_blocks, push_threads, bsm, s, false, sp);
-                } else {
-                    launch(push_block_kernel, block_ctas, 1024u, bsm, s, false, bp);
-                }
-                TGTP_LAUNCH_CHECK("push_block_kernel");
-            }
-            p.claim = claims + w;
-            p.list_base = bp.base;
-            p.list_cap = wave_cap;
-            p.walk_count = ctl + 4 * w;
-            pk.g[0] = p;
-            {
-                ScopedKernel k(g->prof, s, "source");
-                launch(kern, unsigned(blocks), unsigned(threads), smem, s, false, pk);
-                TGTP_LAUNCH_CHECK("source_kernel");
-            }
-            wq.list_base = p.list_base;
-            wq.count = ctl + 4 * w;
-            wq.claim = ctl + 4 * w + 1;
-            {
-                ScopedKernel k(g->prof, s, "walk_queue");
-                launch(walk_queue_kernel, walk_blocks, unsigned(kWalkThreads), size_t(0), s, false, wq);
-                TGTP_LAUNCH_CHECK("walk_queue_kernel");
-            }
-            WalkQueueParams wh = wq;
-            wh.count = ctl + 4 * w + 2;
-            wh.claim = ctl + 4 * w + 3;
-            ScopedKernel k(g->prof, s, "heavy_walk");
-            launch(heavy_walk_kernel, heavy_blocks, unsigned(kHeavyThreads), kHeavySmem, s, false, wh,
-                   uint32_t(m + 1));
-            TGTP_LAUNCH_CHECK("heavy_walk_kernel");
-        }
+        if (!run_sources<Real>(g, cfg, out, rm, multi, logmd)) return;
     }
     launch_finish<Real, Acc>(g, out);
 }
 
 // The persistent source kernel of one batch group: per-warp scratch for the group's largest
 // graph, packs of up to kBatchPack graphs, each pack one launch on `s` with its own claim counter.
-template <class Real, class Acc, bool SMEM, bool JACOBI>
+template <class Real, bool SMEM>
 void launch_group(BatchPlan& plan, BatchGroup& grp, cudaStream_t s, int num_sms) {
-    using Pack = SourcePack<Real, Acc, kBatchPack>;
+    using Pack = SourcePack<Real, kBatchPack>;
     static_assert(sizeof(Pack) < 32000, "pack must fit in the kernel parameter space");
     uint32_t sn = 1, maxd = 1;
     uint64_t rows = 0;
@@ -3983,14 +3677,11 @@ void launch_group(BatchPlan& plan, BatchGroup& grp, cudaStream_t s, int num_sms)
     }
     const size_t pv_bytes = (size_t(sn) * sizeof(Real) + 15) & ~size_t(15);
     const size_t vis_bytes = (size_t(sn) + 15) & ~size_t(15);
-    const size_t fx_bytes = JACOBI ? sizeof(unsigned long long) * size_t(sn) : 0;
-    const bool fx_in_smem = SMEM && JACOBI &&
-                            pv_bytes + vis_bytes + fx_bytes + kAccBytes <= size_t(112) * 1024;
-    const size_t per_warp = pv_bytes + vis_bytes + (fx_in_smem ? fx_bytes : 0) + kAccBytes;
+    const size_t per_warp = pv_bytes + vis_bytes + kAccBytes;
     const int wpb = SMEM ? 1 : 4;
     const int threads = 32 * wpb;
     const size_t smem = SMEM ? per_warp * wpb : size_t(wpb) * kAccBytes;
-    auto kern = source_kernel<Real, Acc, SMEM, JACOBI, Pack>;
+    auto kern = source_kernel<Real, SMEM, Pack>;
     const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(kern), threads, smem);
     if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "batch source kernel does not fit on an SM");
     uint64_t blocks = std::min<uint64_t>(uint64_t(num_sms) * per_sm, (rows + wpb - 1) / wpb);
@@ -4001,8 +3692,7 @@ void launch_group(BatchPlan& plan, BatchGroup& grp, cudaStream_t s, int num_sms)
     const size_t it_bytes = align(warps * maxd * sizeof(WalkItem));
     const size_t pvg_bytes = SMEM ? 0 : align(warps * size_t(sn) * sizeof(Real));
     const size_t visg_bytes = SMEM ? 0 : align(warps * vis_bytes);
-    const size_t fxg_bytes = (JACOBI && !fx_in_smem) ? align(warps * fx_bytes) : 0;
-    grp.scratch.reserve(q_bytes + it_bytes + pvg_bytes + visg_bytes + fxg_bytes + 256);
+    grp.scratch.reserve(q_bytes + it_bytes + pvg_bytes + visg_bytes + 256);
     grp.wclean.reserve(warps + 16);
     const size_t packs = (grp.members.size() + kBatchPack - 1) / kBatchPack;
     grp.claims.reserve(sizeof(unsigned) * (packs + 1));
@@ -4014,7 +3704,7 @@ void launch_group(BatchPlan& plan, BatchGroup& grp, cudaStream_t s, int num_sms)
         Pack pk;
         pk.count = uint32_t(std::min<size_t>(kBatchPack, grp.members.size() - pk0));
         for (uint32_t j = 0; j < pk.count; ++j) {
-            SourceParams<Real, Acc> p;
+            SourceParams<Real> p;
             std::memcpy(&p, plan.entries[grp.members[pk0 + j]].params.data(), sizeof(p));
             unsigned char* b = base;
             p.qbuf = reinterpret_cast<uint32_t*>(b);
@@ -4024,8 +3714,6 @@ void launch_group(BatchPlan& plan, BatchGroup& grp, cudaStream_t s, int num_sms)
             p.pvec_g = SMEM ? nullptr : reinterpret_cast<Real*>(b);
             b += pvg_bytes;
             p.vis_g = SMEM ? nullptr : b;
-            b += visg_bytes;
-            p.fx_g = fxg_bytes ? reinterpret_cast<unsigned long long*>(b) : nullptr;
             p.wclean = grp.wclean.as<unsigned char>();
             p.vis_stride = vis_bytes;
             p.smem_per_warp = per_warp;
@@ -4036,6 +3724,41 @@ void launch_group(BatchPlan& plan, BatchGroup& grp, cudaStream_t s, int num_sms)
         }
         launch(kern, unsigned(blocks), unsigned(threads), smem, s, false, pk);
         TGTP_LAUNCH_CHECK("source_kernel (batch)");
+    }
+}
+
+// The same for the mixed form: one block per source, per-block scratch for the group's largest graph.
+void launch_mixed_group(BatchPlan& plan, BatchGroup& grp, cudaStream_t s, int num_sms) {
+    using Pack = MixedPack<kBatchPack>;
+    static_assert(sizeof(Pack) < 32000, "pack must fit in the kernel parameter space");
+    uint64_t sn = 1, maxd = 1, rows = 0;
+    for (size_t i : grp.members) {
+        const tgtp_graph* g = plan.entries[i].g;
+        sn = std::max<uint64_t>(sn, g->n);
+        maxd = std::max<uint64_t>(maxd, g->max_degree);
+        rows += g->n;
+    }
+    const int mode = grp.smem ? kShared : kGlobal;
+    const MixedLayout lay = mixed_layout<Pack>(mode, sn, maxd, rows, num_sms);
+    grp.scratch.reserve(lay.scratch());
+    grp.wclean.reserve(lay.blocks + 16);
+    const size_t packs = (grp.members.size() + kBatchPack - 1) / kBatchPack;
+    grp.claims.reserve(sizeof(unsigned) * (packs + 1));
+    // each replay starts from "sums not known to be zero" and fresh claim counters
+    TGTP_CUDA(cudaMemsetAsync(grp.wclean.ptr, 0, lay.blocks + 16, s));
+    TGTP_CUDA(cudaMemsetAsync(grp.claims.ptr, 0, sizeof(unsigned) * (packs + 1), s));
+    for (size_t pk0 = 0; pk0 < grp.members.size(); pk0 += kBatchPack) {
+        auto pk = std::make_unique<Pack>();
+        pk->count = uint32_t(std::min<size_t>(kBatchPack, grp.members.size() - pk0));
+        for (uint32_t j = 0; j < pk->count; ++j) {
+            MixedParams p;
+            std::memcpy(&p, plan.entries[grp.members[pk0 + j]].params.data(), sizeof(p));
+            carve_mixed(p, lay, grp.scratch.as<unsigned char>(), sn, maxd);
+            p.clean = grp.wclean.as<unsigned char>();
+            p.claim = grp.claims.as<unsigned>() + pk0 / kBatchPack;
+            pk->g[j] = p;
+        }
+        launch_mixed(mode, lay, s, false, *pk);
     }
 }
 
@@ -4068,17 +3791,14 @@ void batch_plan_launch(BatchPlan* plan, cudaStream_t s, int num_sms) {
     for (auto& grp : plan->groups) {
         switch (grp->key) {
             case 0:
-                if (grp->smem) launch_group<float, float, true, false>(*plan, *grp, s, num_sms);
-                else launch_group<float, float, false, false>(*plan, *grp, s, num_sms);
+                if (grp->smem) launch_group<float, true>(*plan, *grp, s, num_sms);
+                else launch_group<float, false>(*plan, *grp, s, num_sms);
                 break;
             case 1:
-                if (grp->smem) launch_group<double, double, true, false>(*plan, *grp, s, num_sms);
-                else launch_group<double, double, false, false>(*plan, *grp, s, num_sms);
+                if (grp->smem) launch_group<double, true>(*plan, *grp, s, num_sms);
+                else launch_group<double, false>(*plan, *grp, s, num_sms);
                 break;
-            default:
-                if (grp->smem) launch_group<float, double, true, true>(*plan, *grp, s, num_sms);
-                else launch_group<float, double, false, true>(*plan, *grp, s, num_sms);
-                break;
+            default: launch_mixed_group(*plan, *grp, s, num_sms); break;
         }
     }
 }
@@ -4118,19 +3838,19 @@ void aesc_run(tgtp_graph* g, const tgtp_config& cfg, float* device_scores) {
     switch (cfg.precision) {
         case TGTP_PRECISION_FP32:
             if (!g->has_f32) fail(TGTP_ERR_INVALID_ARGUMENT, "FP32 form needs F32 eigenvectors");
-            run_form<float, float, false, float>(g, cfg, device_scores);
+            run_form<float, false, float>(g, cfg, device_scores);
             break;
         case TGTP_PRECISION_FP64:
             if (!g->has_f64) fail(TGTP_ERR_INVALID_ARGUMENT, "FP64 form needs F64 eigenvectors");
-            run_form<double, double, false, double>(g, cfg, device_scores);
+            run_form<double, false, double>(g, cfg, device_scores);
             break;
         case TGTP_PRECISION_MIXED:
             if (cfg.vec_dtype == TGTP_VEC_BF16) {
                 if (!g->has_bf16) fail(TGTP_ERR_INVALID_ARGUMENT, "MIXED/BF16 needs BF16 eigenvectors");
-                run_form<float, double, true, __nv_bfloat16>(g, cfg, device_scores);
+                run_form<float, true, __nv_bfloat16>(g, cfg, device_scores);
             } else if (cfg.vec_dtype == TGTP_VEC_F32) {
                 if (!g->has_f32) fail(TGTP_ERR_INVALID_ARGUMENT, "MIXED/F32 needs F32 eigenvectors");
-                run_form<float, double, true, float>(g, cfg, device_scores);
+                run_form<float, true, float>(g, cfg, device_scores);
             } else {
                 fail(TGTP_ERR_INVALID_ARGUMENT, "MIXED form stores eigenvectors as F32 or BF16");
             }
@@ -4234,22 +3954,23 @@ int aesc_tune(tgtp_graph* g, const tgtp_config& cfg, float* device_scores, int t
     const int key = form_key(cfg);
     const size_t rs = cfg.precision == TGTP_PRECISION_FP64 ? 8 : 4;
     const bool mixed = cfg.precision == TGTP_PRECISION_MIXED;
-    size_t per_warp = ((g->n * rs + 15) & ~size_t(15)) + ((g->n + 15) & ~size_t(15)) + kAccBytes;
-    if (mixed && per_warp + 8 * g->n <= size_t(112) * 1024) per_warp += 8 * g->n;
     std::vector<uint16_t> cand;
-    // the parity forms also try the windowed and the one-vertex-at-a-time push in each layout
-    const std::vector<uint16_t> push_kinds =
-        mixed ? std::vector<uint16_t>{0} : std::vector<uint16_t>{kLayoutWindow, kLayoutNoWindow};
-    for (uint16_t pk : push_kinds) {
-        for (int w : {1, 2})
-            if (per_warp * w <= size_t(227) * 1024) cand.push_back(uint16_t(pk | kLayoutSmem | w));
-        for (int w : {1, 2, 4}) cand.push_back(uint16_t(pk | w));
-    }
-    if (mixed) {  // the block push, with the per-source stage in the best layout that fits,
-                  // at each compaction threshold
-        const uint16_t post = per_warp <= size_t(112) * 1024 ? uint16_t(kLayoutSmem | 1) : uint16_t(4);
-        for (int ld = 0; ld < 4; ++ld)
-            cand.push_back(uint16_t(kLayoutBlock | post | (ld << kLayoutListShift)));
+    if (mixed) {
+        // one source per block with its sums in shared memory or in HBM, and the block push at each
+        // compaction threshold of its 32-source form (one while the sums fit in shared memory)
+        const bool shared = mixed_fits_shared(g->n);
+        if (shared) cand.push_back(uint16_t(kLayoutSmem | 1));
+        cand.push_back(4);
+        for (int ld = 0; ld < (push_shared_bytes(g->n) <= size_t(227) * 1024 ? 1 : 4); ++ld)
+            cand.push_back(uint16_t(kLayoutBlock | 4 | (ld << kLayoutListShift)));
+    } else {
+        // residual vectors in shared memory or in HBM, warps per block, windowed or one-vertex push
+        const size_t per_warp = ((g->n * rs + 15) & ~size_t(15)) + ((g->n + 15) & ~size_t(15)) + kAccBytes;
+        for (uint16_t pk : {kLayoutWindow, kLayoutNoWindow}) {
+            for (int w : {1, 2})
+                if (per_warp * w <= size_t(227) * 1024) cand.push_back(uint16_t(pk | kLayoutSmem | w));
+            for (int w : {1, 2, 4}) cand.push_back(uint16_t(pk | w));
+        }
     }
     cudaEvent_t e0, e1;
     TGTP_CUDA(cudaEventCreate(&e0));

@@ -43,9 +43,9 @@ __device__ __forceinline__ uint32_t find_segment(const uint32_t* offs, uint32_t 
 }
 
 // Concatenates the rows of up to kChunk vertices: thread i < cnt passes vertex i's row start, its
-// degree (at least 1) and a value; f(entry's slot, value of its vertex, the vertex's index in the
-// chunk) is called once for every entry, with the warp's lanes on consecutive entries (converged
-// except for the last step).  All threads of the block call it; the scratch is free again after
+// degree (at least 1) and a value.  Every entry is loaded, load(slot, whether there is an entry), and
+// then used, use(loaded, value of its vertex, the vertex's index in the chunk, the lanes with an
+// entry in this step), with the warp's lanes on consecutive entries.  All threads of the block call it; the scratch is free again after
 // the caller's next __syncthreads.
 template <class Load, class Use>
 __device__ __forceinline__ uint32_t for_entries(ChunkScratch& s, uint32_t cnt, uint32_t beg, uint32_t deg,
@@ -91,7 +91,8 @@ __device__ __forceinline__ uint32_t for_entries(ChunkScratch& s, uint32_t cnt, u
                 slotn = inn ? s.base[kn] + en + lane : 0u;
                 xn = load(slotn, inn);
             }
-            if (in) use(x, s.val[k], k);
+            const unsigned lanes = __ballot_sync(kFullMask, in);
+            if (in) use(x, s.val[k], k, lanes);
             if (!more) break;
             e = en;
             k = kn;
@@ -228,7 +229,7 @@ __device__ __forceinline__ void push_frontier(PushScratch& s, const Frontier& f,
         for_entries(
             s.chunk, cnt, q.x, q.y, to_fixed(__uint_as_float(q.z)),
             [&](uint32_t slot, bool in) { return in ? __ldg(adj + slot) : 0u; },
-            [&](uint32_t u, unsigned long long v, uint32_t) { add(u, v); });
+            [&](uint32_t u, unsigned long long v, uint32_t, unsigned) { add(u, v); });
     }
     // light vertices: batches of 32 claimed by the warps, the next one loaded while one is pushed
     auto claim = [&]() {
