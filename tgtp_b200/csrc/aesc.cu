@@ -52,10 +52,6 @@ namespace tgtp {
 namespace {
 
 constexpr int kTauThreads = 32;
-constexpr int kSrcMaxThreads = 128;
-constexpr int kPushAhead = 4;         // adjacency chunks loaded ahead in the push
-constexpr int kB = 4;                 // 32-wide chunks per pipelined load step
-constexpr int kTopK = 16;            // register top-k used for gamma <= 16
 // per-warp shared scratch of the chi step: 64 u64 max/min images + 33 + 32 u32 slot offsets
 constexpr size_t kAccBytes = 1280;
 constexpr int kTauTableRows = 64;    // rows of the eigen_t_1 power table (api.cu)
@@ -967,57 +963,6 @@ struct PrePush {
     uint32_t support;  // size of the final frontier
 };
 
-template <class Real>
-struct SourceParams {
-    const uint32_t* idx;
-    const uint32_t* adj;
-    const uint32_t* deg;
-    uint32_t n;
-    const int* taus;
-    Real* preds;          // pre-symmetric row scores
-    unsigned* work;       // [0] next list entry, [1] error flags, [2] list length
-    const uint32_t* rows; // the sources to run (rows with a slot of tau > 1), in any order
-    uint32_t* qbuf;       // 2 * n per warp
-    WalkItem* items;      // max_degree per warp
-    Real* pvec_g;         // n per warp (global tier)
-    unsigned char* wclean;     // per warp: 1 = its HBM vectors are all zero (left so by its last run)
-    unsigned char* vis_g; // vis_stride per warp (global tier)
-    size_t vis_stride;
-    size_t smem_per_warp;
-    uint32_t max_degree;
-    double eps;
-    double logmd;         // log(m / delta), formed on the host
-    int gamma;
-    unsigned long long* stats;
-    const uint2* adjd;    // (neighbour, neighbour degree) per slot
-    uint64_t budget_ns;   // device time budget; past it every warp stops and flags a timeout
-    unsigned* claim;      // the claim counter of this launch
-    // The graph has rows that repeat a neighbour or hold their own vertex (the reference's loader
-    // keeps duplicate edges and self-loops, src/graph.h:63-66, 75-78): the first round takes the
-    // general path and the push serialises each run of a repeated neighbour.
-    bool multi;
-    // Vertex count the per-warp scratch is laid out for (the graph's n, or the largest n of a
-    // batch whose graphs share the scratch of one persistent launch).
-    uint32_t scratch_n;
-    bool gs_window;  // the windowed sequential push (else one vertex at a time)
-    // Optional run trace (null when off): the walk count nr of every walking slot, and the rounds
-    // pushed (ell) of every listed row.
-    uint32_t* trace_nr;
-    uint32_t* trace_ell;
-};
-
-// The source kernel's parameters: one graph (N = 1), or up to N graphs whose listed rows one
-// persistent launch works through as a single queue of (graph, row) items.  Every entry shares the
-// first entry's per-warp scratch (qbuf, items, residual vectors, flags, claim counter).  The pack
-// travels in the kernel's parameter space, so a warp reads its graph's fields from the constant
-// bank with a warp-uniform index.
-template <class Real, int N>
-struct SourcePack {
-    static constexpr int kMax = N;
-    uint32_t count;
-    SourceParams<Real> g[N];
-};
-constexpr int kBatchPack = 64;  // graphs per persistent batch launch
 
 template <class Real>
 __device__ __forceinline__ Real warp_max(Real x) {
@@ -1035,22 +980,6 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long x)
 #pragma unroll
     for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(kFullMask, x, o);
     return x;
-}
-
-// Runs over [0, count) in steps of 32 * kB: load(i0, regs) issues the loads of one step into
-// registers, proc(i0, regs) consumes them.  The next step's loads are issued before the current
-// step is processed, so a pass over a frontier or a row waits for memory once, not once per step.
-template <class T, class Load, class Proc>
-__device__ __forceinline__ void pipelined(uint32_t count, Load load, Proc proc) {
-    if (count == 0) return;
-    T a[kB], b[kB];
-    load(0u, a);
-    for (uint32_t i0 = 0; i0 < count; i0 += 32 * kB) {
-        if (i0 + 32 * kB < count) load(i0 + 32 * kB, b);
-        proc(i0, a);
-#pragma unroll
-        for (int k = 0; k < kB; ++k) a[k] = b[k];
-    }
 }
 
 // preds[pos] += (pvec[src] - pvec[w]) / ds (:236): in the row's own real type in the parity forms,
@@ -1076,90 +1005,6 @@ template <> __device__ __forceinline__ float from_ord<float>(unsigned long long 
 }
 template <> __device__ __forceinline__ double from_ord<double>(unsigned long long b) {
     return __longlong_as_double((long long)b);
-}
-
-// The real_gamma-th largest residual of the frontier (counting multiplicity) and how many of the
-// chosen values equal it.  gamma <= kTopK: one pass keeping a sorted top-k per lane, then a
-// warp merge.  Larger gamma: one pass per distinct value from the top.
-template <class Real>
-__device__ void kth_largest(const uint32_t* q, uint32_t qs, const Real* pvec, int rg, Real& t,
-                            int& n_eq_taken) {
-    const uint32_t lane = threadIdx.x & 31;
-    auto load_q = [&](uint32_t i0, uint32_t* r) {
-#pragma unroll
-        for (int b = 0; b < kB; ++b) {
-            const uint32_t i = i0 + 32 * b + lane;
-            r[b] = i < qs ? q[i] : 0xffffffffu;
-        }
-    };
-    if (rg <= kTopK) {
-        Real L[kTopK];
-#pragma unroll
-        for (int j = 0; j < kTopK; ++j) L[j] = Real(-INFINITY);
-        pipelined<uint32_t>(qs, load_q, [&](uint32_t, const uint32_t* r) {
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                if (r[b] == 0xffffffffu) continue;
-                const Real x = pvec[r[b]];
-                if (x > L[kTopK - 1]) {
-#pragma unroll
-                    for (int j = kTopK - 1; j > 0; --j) {
-                        const Real prev = L[j - 1];
-                        L[j] = x > prev ? prev : (x > L[j] ? x : L[j]);
-                    }
-                    L[0] = x > L[0] ? x : L[0];
-                }
-            }
-        });
-        Real last = Real(-INFINITY);
-        int run = 0;
-        for (int r = 0; r < rg; ++r) {
-            const Real mx = warp_max(L[0]);
-            const unsigned who = __ballot_sync(kFullMask, L[0] == mx);
-            if (lane == uint32_t(__ffs(who) - 1)) {
-#pragma unroll
-                for (int j = 0; j < kTopK - 1; ++j) L[j] = L[j + 1];
-                L[kTopK - 1] = Real(-INFINITY);
-            }
-            run = (r > 0 && mx == last) ? run + 1 : 1;
-            last = mx;
-        }
-        t = last;
-        n_eq_taken = run;
-        return;
-    }
-    Real thr = Real(INFINITY);
-    int remaining = rg;
-    while (true) {
-        Real best = Real(-INFINITY);
-        unsigned cnt = 0;
-        pipelined<uint32_t>(qs, load_q, [&](uint32_t, const uint32_t* r) {
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                if (r[b] == 0xffffffffu) continue;
-                const Real x = pvec[r[b]];
-                if (x < thr) {
-                    if (x > best) {
-                        best = x;
-                        cnt = 1;
-                    } else if (x == best) {
-                        ++cnt;
-                    }
-                }
-            }
-        });
-        const Real mx = warp_max(best);
-        unsigned c = best == mx ? cnt : 0;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(kFullMask, c, o);
-        if (int(c) >= remaining) {
-            t = mx;
-            n_eq_taken = remaining;
-            return;
-        }
-        remaining -= int(c);
-        thr = mx;
-    }
 }
 
 // ---- stage 2a (mixed form, large graphs): multi-source Jacobi push as a pull product -----------
@@ -1667,916 +1512,6 @@ __global__ void row_key_kernel(const uint32_t* __restrict__ idx, const int* __re
     }
 }
 
-// The HBM-tier variants with FP32 residuals keep at least three 128-thread blocks per SM (at most
-// 168 registers): their phases are latency-bound on HBM and need the warps.  The FP64 variant
-// compiled to about 240 registers (two blocks per SM) without spills before and is left so.
-template <class Real, bool SMEM, class Pack>
-__global__ void __launch_bounds__(kSrcMaxThreads, (!SMEM && sizeof(Real) == 4) ? 3 : 1)
-source_kernel(Pack pk) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ uint32_t s_pre[Pack::kMax + 1];  // item prefix over the pack's row lists
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t wib = threadIdx.x >> 5;
-    const uint32_t wpb = blockDim.x >> 5;
-    const uint64_t gw = uint64_t(blockIdx.x) * wpb + wib;
-    // the per-warp scratch (shared by every graph of the pack) comes from the first entry
-    const SourceParams<Real>& p0 = pk.g[0];
-    const uint32_t sn = p0.scratch_n;
-    const unsigned lt = (1u << lane) - 1u;
-    constexpr uint32_t NONE = 0xffffffffu;
-    Real* pvec;
-    unsigned char* vis;       // per vertex: 1 = discovered this round, 2 = in the top-gamma set
-    unsigned long long* acc;  // 64 per warp: per-slot neighbourhood max (0..31) / min (32..63)
-    if (SMEM) {
-        unsigned char* base = smem + size_t(wib) * p0.smem_per_warp;
-        pvec = reinterpret_cast<Real*>(base);
-        const size_t pv = (size_t(sn) * sizeof(Real) + 15) & ~size_t(15);
-        vis = base + pv;
-        const size_t vb = (size_t(sn) + 15) & ~size_t(15);
-        acc = reinterpret_cast<unsigned long long*>(base + pv + vb);
-    } else {
-        pvec = p0.pvec_g + gw * size_t(sn);
-        vis = p0.vis_g + gw * p0.vis_stride;
-        acc = reinterpret_cast<unsigned long long*>(smem + size_t(wib) * kAccBytes);
-    }
-    // pvec and flags are zeroed once, before the warp's first source, unless the warp's last run
-    // (same layout, HBM tier) left them zero: every source resets what it touched
-    bool cleared = !SMEM && p0.wclean[gw] != 0;
-    bool dirty = false;  // a source stopped midway (time-out): its vectors are not zero
-    uint32_t* qa = p0.qbuf + gw * 2 * size_t(sn);
-    uint32_t* qb = qa + sn;
-    WalkItem* items = p0.items + gw * size_t(p0.max_degree);
-    unsigned long long st_rounds = 0, st_pv = 0, st_tr = 0, st_we = 0, st_wc = 0, st_wh = 0,
-                       st_fb = 0;
-    const uint64_t deadline = globaltimer_ns() + p0.budget_ns;
-    // SM cycles spent per phase of a source (claim/init, push, post-push, cost test, edge bound,
-    // chi/nr, walks, reset), summed over the warp's sources
-    long long ph[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    long long tmark = clock64();
-    auto lap = [&](int i) {
-        const long long now = clock64();
-        ph[i] += now - tmark;
-        tmark = now;
-    };
-
-    // Run counters go to the stats of the graph a source belongs to: flushed when a warp moves
-    // to another graph of the pack, and at the end.
-    auto flush_stats = [&](unsigned long long* stats) {
-        if (lane == 0) {
-            stat_add(stats, kStPushRounds, st_rounds);
-            stat_add(stats, kStPushVertices, st_pv);
-            stat_add(stats, kStPushTraversals, st_tr);
-        }
-        st_we = warp_sum_u64(st_we);
-        st_wc = warp_sum_u64(st_wc);
-        st_wh = warp_sum_u64(st_wh);
-        st_fb = warp_sum_u64(st_fb);
-        if (lane == 0) {
-            stat_add(stats, kStWalkEdges, st_we);
-            stat_add(stats, kStWalkCount, st_wc);
-            stat_add(stats, kStWalkHops, st_wh);
-            stat_add(stats, kStFallback, st_fb);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) stat_add(stats, kStPhase0 + i, (unsigned long long)ph[i]);
-        }
-        st_rounds = st_pv = st_tr = st_we = st_wc = st_wh = st_fb = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) ph[i] = 0;
-    };
-    __syncwarp();
-
-    pdl_launch_dependents();
-    pdl_wait();  // taus, row lists and their lengths from the tau kernels
-    // items: the listed rows of the pack's graphs one after another (a list's length is final:
-    // the tau kernel that appends to it has ended)
-    if (threadIdx.x == 0) {
-        uint32_t acc_items = 0;
-        s_pre[0] = 0;
-        for (uint32_t i = 0; i < pk.count; ++i) {
-            acc_items += pk.g[i].work[2];
-            s_pre[i + 1] = acc_items;
-        }
-    }
-    __syncthreads();
-    const unsigned nrows = s_pre[pk.count];
-    // item gw first, then items past the grid's warps claimed one at a time (warps past the
-    // end leave without touching the counter)
-    const uint64_t nwarps = uint64_t(gridDim.x) * wpb;
-    bool first_claim = true;
-    uint32_t last_gi = 0xffffffffu;
-    while (true) {
-        uint64_t k = gw;
-        if (!first_claim) {
-            unsigned c = 0;
-            if (lane == 0) c = atomicAdd(p0.claim, 1u);
-            k = nwarps + __shfl_sync(kFullMask, c, 0);
-        }
-        first_claim = false;
-        if (k >= nrows) break;
-        // the item's graph: the last list whose prefix is at most k (warp-uniform)
-        uint32_t gi = 0;
-        for (uint32_t hi = pk.count; hi - gi > 1;) {
-            const uint32_t mid = (gi + hi) >> 1;
-            if (s_pre[mid] <= k) gi = mid;
-            else hi = mid;
-        }
-        const SourceParams<Real>& p = pk.g[gi];
-        if (gi != last_gi) {
-            if (last_gi != 0xffffffffu) flush_stats(pk.g[last_gi].stats);
-            last_gi = gi;
-        }
-        if (globaltimer_ns() > deadline) {
-            if (lane == 0) atomicOr(p.work + 1, kErrDeadline);
-            break;
-        }
-        const uint32_t n = p.n;
-        const uint32_t* __restrict__ idx = p.idx;
-        const uint32_t* __restrict__ adj = p.adj;
-        const int* __restrict__ taus = p.taus;
-        const uint32_t src = __ldg(p.rows + uint32_t(k - s_pre[gi]));
-        if (!cleared) {
-            for (uint32_t i = lane; i < sn; i += 32) {
-                pvec[i] = Real(0);
-                vis[i] = 0;
-            }
-            cleared = true;
-            __syncwarp();
-        }
-        uint32_t* q = qa;
-        uint32_t* qn = qb;
-        const uint32_t rb = __ldg(idx + src), re = __ldg(idx + src + 1);
-        const uint32_t dsi = re - rb;
-        const Real ds = from_u64<Real>(dsi);
-        // preds = 1.0 / ds (:468-470); stored together with the first round's update below
-        const Real pinit = from_f64<Real>(__ddiv_rn(1.0, double(ds)));
-        uint32_t qs = 0;
-        int ell = 0;
-        Real gmin, gmax;
-        bool timed_out = false;
-        unsigned long long pcost = 0;
-        Real mx = Real(0), mn = Real(1);
-        // row loaders (neighbour, tau) for the pipelined passes over the source's row
-        auto load_adj = [&](uint32_t c, uint32_t* r) {
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                const uint32_t o = c + 32 * b + lane;
-                r[b] = o < dsi ? __ldg(adj + rb + o) : NONE;
-            }
-        };
-        auto load_tau = [&](uint32_t c, int* r) {
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                const uint32_t o = c + 32 * b + lane;
-                r[b] = o < dsi ? __ldg(taus + rb + o) : 0;
-            }
-        };
-        lap(0);
-        {
-            // ---- round 1 in closed form (:457-503, first pass of the loop) ----
-            // The frontier is {src} with residual 1 (pvec[src] = 1.0, then zeroed as it is drained):
-            // every neighbour u is discovered in row order and receives 0 + 1/deg(u) = 1/deg(u), so
-            // the round's new frontier, residuals, degree sum, max / min and row update
-            // preds = 1/ds + (0 - 1/deg(u)) / ds follow from one pass over the row when the
-            // neighbours are distinct.  Rows of a graph with repeated neighbours or self-loops
-            // (p.multi, parity forms) take the general path below instead.
-            if (p.multi) {
-                // (1) each run of one neighbour u (rows are sorted, so repeats are adjacent) is
-                // handled by its first slot: k repeats add 1/deg(u) k times in order, as the
-                // reference's sequential += does; that slot discovers u (first-occurrence order)
-                // and adds deg(u) to picost.  pvec[src] starts at 0 (it was drained), so a
-                // self-loop run adds to it like to any neighbour.
-                uint32_t found = 0;
-                for (uint32_t c = 0; c < dsi; c += 32) {
-                    const uint32_t o = c + lane;
-                    const bool in = o < dsi;
-                    const uint2 a = in ? __ldg(p.adjd + rb + o) : make_uint2(NONE, 1u);
-                    const bool lead = in && (o == 0 || __ldg(adj + rb + o - 1) != a.x);
-                    Real pu = Real(0);
-                    if (lead) {
-                        const Real x = rdiv(Real(1), from_u64<Real>(a.y));
-                        pu = x;
-                        for (uint32_t k = o + 1; k < dsi && __ldg(adj + rb + k) == a.x; ++k)
-                            pu = radd(pu, x);
-                        pvec[a.x] = pu;
-                        pcost += a.y;
-                        mx = std_max(mx, pu);
-                        mn = std_min(mn, pu);
-                    }
-                    const unsigned bl = __ballot_sync(kFullMask, lead);
-                    if (lead) qn[found + __popc(bl & lt)] = a.x;
-                    found += __popc(bl);
-                }
-                __syncwarp();
-                // (2) preds[s -> t] = 1/ds + (pvec[s] - pvec[t]) / ds with the round's residuals
-                const Real ps = pvec[src];
-                for (uint32_t o = lane; o < dsi; o += 32)
-                    p.preds[rb + o] = row_update<Real, Real>(pinit, ps, pvec[__ldg(adj + rb + o)], ds);
-                qs = found;
-            } else {
-            pipelined<uint2>(dsi,
-                [&](uint32_t c, uint2* r) {
-    #pragma unroll
-                    for (int b = 0; b < kB; ++b) {
-                        const uint32_t o = c + 32 * b + lane;
-                        r[b] = o < dsi ? __ldg(p.adjd + rb + o) : make_uint2(NONE, 1u);
-                    }
-                },
-                [&](uint32_t c, const uint2* r) {
-    #pragma unroll
-                    for (int b = 0; b < kB; ++b) {
-                        if (r[b].x == NONE) continue;
-                        const uint32_t o = c + 32 * b + lane;
-                        const Real pu = rdiv(Real(1), from_u64<Real>(r[b].y));
-                        pvec[r[b].x] = pu;
-                        qn[o] = r[b].x;
-                        pcost += r[b].y;
-                        mx = std_max(mx, pu);
-                        mn = std_min(mn, pu);
-                        p.preds[rb + o] = row_update<Real, Real>(pinit, Real(0), pu, ds);
-                    }
-                });
-            qs = dsi;
-            }
-            st_pv += 1;
-            st_tr += dsi;
-            ell = 1;
-            { uint32_t* tmp = q; q = qn; qn = tmp; }
-            __syncwarp();
-            lap(1);
-            while (true) {
-                // ---- the push/walk cost test (:483-502) ----
-                const double picost = double(warp_sum_u64(pcost));
-                gmax = warp_max(mx);
-                gmin = warp_min(mn);
-                gmin = qs < n ? Real(0) : gmin;
-                const double dse0 = __dmul_rn(double(ds), p.eps);
-                const double dse2 = __dmul_rn(dse0, dse0);
-                double rw = 0;
-                pipelined<int>(dsi, load_tau, [&](uint32_t c, const int* tv) {
-    #pragma unroll
-                    for (int b = 0; b < kB; ++b) {
-                        const uint32_t o = c + 32 * b + lane;
-                        const int rest = tv[b] - ell;
-                        double nrd = 0;
-                        const bool has = o < dsi && rest > 0;
-                        if (has) {
-                            const double chi = __dmul_rn(__dmul_rn(2.0, double(rest)),
-                                                         __dsub_rn(double(gmax), double(gmin)));
-                            const double num = __dmul_rn(__dmul_rn(8.0, __dmul_rn(chi, chi)), p.logmd);
-                            nrd = std_max(ceil(__ddiv_rn(num, dse2)), 1.0);
-                        }
-                        unsigned hb = __ballot_sync(kFullMask, has);
-                        while (hb) {  // rwcost += nr in slot order
-                            const int l = __ffs(hb) - 1;
-                            hb &= hb - 1;
-                            rw = __dadd_rn(rw, __shfl_sync(kFullMask, nrd, l));
-                        }
-                    }
-                });
-                lap(3);
-                if (picost >= __dmul_rn(25.0, rw)) break;
-                if (globaltimer_ns() > deadline) {
-                    timed_out = true;
-                    break;
-                }
-                uint32_t qns = 0;
-                pcost = 0;
-                st_pv += qs;
-                if (p.gs_window) {
-                // ---- diffuse (:218-239), windowed ----
-                // The reference drains the frontier one vertex at a time: r = pvec[v], pvec[v] = 0,
-                // then pvec[u] += r / deg(u) for u in N(v) in row order, discovering each u on its
-                // first visit.  Here up to 32 consecutive frontier vertices form a window whose
-                // residuals are taken at once and whose rows are concatenated and processed 32
-                // entries per step, in order.  That gives the reference's values as long as no
-                // entry of a window vertex j targets a later window vertex k (it would have changed
-                // r_k before k was drained): such an entry cuts the window before k -- found before
-                // anything of its step is applied, the cut vertices get their residuals back and
-                // are drained by a later window.  Entries targeting the vertex itself or an earlier
-                // window vertex are ordinary adds (those were drained first in the reference too).
-                // Lanes of one step that hit the same neighbour form a group whose lowest lane adds
-                // the group's contributions one by one in lane (= the reference's) order; the
-                // lowest lane is also the first visit, so discovery order is the reference's.  vis
-                // holds 1 + the window index in its upper six bits while a vertex is in a window.
-                uint32_t* exs = reinterpret_cast<uint32_t*>(acc + 64 + 32);  // 33 entry offsets
-                uint32_t* vbs = exs + 33;                                     // 32 row starts
-                for (uint32_t i0 = 0; i0 < qs;) {
-                    const uint32_t cnt = min(32u, qs - i0);
-                    uint32_t myv = 0, vb = 0, vd = 0;
-                    Real rv = Real(0);
-                    if (lane < cnt) {
-                        myv = q[i0 + lane];
-                        vb = __ldg(idx + myv);
-                        vd = __ldg(idx + myv + 1) - vb;
-                        rv = pvec[myv];
-                    }
-                    __syncwarp();
-                    if (lane < cnt) {
-                        pvec[myv] = Real(0);
-                        vis[myv] = (unsigned char)((vis[myv] & 3u) | ((lane + 1u) << 2));
-                    }
-                    uint32_t incl = vd;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
-                        if (lane >= uint32_t(o)) incl += y;
-                    }
-                    const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-                    exs[lane] = incl - vd;
-                    vbs[lane] = vb;
-                    if (lane == 31) exs[32] = total;
-                    __syncwarp();
-                    uint32_t wend = cnt;  // the window: frontier vertices i0 .. i0 + wend - 1
-                    uint32_t pm = 0;      // entry cursor of the loader (one step ahead)
-                    auto load_step = [&](uint32_t e0, uint32_t& cur_m, uint32_t& sg, uint2& a) {
-                        const uint32_t e = e0 + lane;
-                        sg = 32u;
-                        a = make_uint2(NONE, 1u);
-                        if (e < total) {
-                            while (exs[cur_m + 1] <= e) ++cur_m;
-                            sg = cur_m;
-                            a = __ldg(p.adjd + vbs[cur_m] + (e - exs[cur_m]));
-                        }
-                    };
-                    uint32_t sg = 32u, nsg = 32u;
-                    uint2 ea, nea;
-                    load_step(0u, pm, sg, ea);
-                    for (uint32_t e0 = 0; e0 < total; e0 += 32) {
-                        if (e0 + 32 < total) load_step(e0 + 32, pm, nsg, nea);
-                        if (__all_sync(kFullMask, sg >= wend)) break;  // past the (cut) window
-                        const bool valid = sg < wend;
-                        const uint32_t u = ea.x, du = ea.y;
-                        const uint32_t vv = valid ? uint32_t(vis[u]) : 0u;
-                        const uint32_t wk = vv >> 2;  // 1 + window index of u, 0 if none
-                        const bool conflict = valid && wk > sg + 1u;
-                        if (__any_sync(kFullMask, conflict)) {
-                            uint32_t kmin = conflict ? wk - 1u : 32u;
-#pragma unroll
-                            for (int o = 16; o; o >>= 1) kmin = min(kmin, __shfl_xor_sync(kFullMask, kmin, o));
-                            // window vertices kmin .. wend - 1 leave the window undrained
-                            if (lane >= kmin && lane < wend) {
-                                pvec[myv] = rv;
-                                vis[myv] = (unsigned char)(vis[myv] & 3u);
-                            }
-                            wend = kmin;
-                            __syncwarp();
-                        }
-                        const bool apply = sg < wend;
-                        const uint32_t vis_u = apply ? uint32_t(vis[u]) : 0u;
-                        const unsigned grp = __match_any_sync(kFullMask, apply ? u : (0xffffffe0u | lane));
-                        const bool lead = apply && lane == uint32_t(__ffs(grp) - 1);
-                        const Real r = __shfl_sync(kFullMask, rv, int(sg & 31u));
-                        const Real c = apply ? rdiv(r, from_u64<Real>(du)) : Real(0);
-                        bool fresh = false;
-                        if (lead && (vis_u & 1u) == 0u) {
-                            vis[u] = (unsigned char)(vis_u | 1u);
-                            fresh = true;
-                        }
-                        const unsigned bal = __ballot_sync(kFullMask, fresh);
-                        if (fresh) {
-                            qn[qns + __popc(bal & lt)] = u;
-                            pcost += du;
-                        }
-                        qns += __popc(bal);
-                        const unsigned others = __ballot_sync(kFullMask, apply && !lead);
-                        Real pv = Real(0);
-                        if (lead) pv = radd(pvec[u], c);
-                        for (unsigned mm = others; mm; mm &= mm - 1) {
-                            const int t = __ffs(mm) - 1;
-                            const Real ct = __shfl_sync(kFullMask, c, t);
-                            if (lead && ((grp >> t) & 1u)) pv = radd(pv, ct);
-                        }
-                        if (lead) pvec[u] = pv;
-                        __syncwarp();
-                        sg = nsg;
-                        ea = nea;
-                        nsg = 32u;
-                    }
-                    if (lane < wend) vis[myv] = (unsigned char)(vis[myv] & 3u);
-                    st_tr += __shfl_sync(kFullMask, incl, int(wend - 1));
-                    __syncwarp();
-                    i0 += wend;
-                }
-                } else {
-                // ---- diffuse (:218-239) ----
-                // The frontier is drained in order, one vertex at a time; the lanes share the
-                // vertex's adjacency (distinct neighbours, so the lanes' flag and residual updates
-                // touch distinct bytes and words).  Per batch of 32 frontier vertices the adjacency is
-                // cut into 32-slot chunks walked by a cursor; a chunk's (neighbour, degree) pairs are
-                // one coalesced 8-byte load per lane, issued kPushAhead chunks before use.  picost (the
-                // new frontier's degree sum) is summed on discovery.  Every vertex has at least one
-                // chunk: tgtp_run rejects isolated vertices.
-
-                for (uint32_t i0 = 0; i0 < qs; i0 += 32) {
-                    uint32_t myv = 0, myb = 0, myd = 0;
-                    if (i0 + lane < qs) {
-                        myv = q[i0 + lane];
-                        myb = __ldg(idx + myv);
-                        myd = __ldg(idx + myv + 1) - myb;
-                    }
-                    const uint32_t cnt = min(32u, qs - i0);
-                    uint32_t pt = 0, pc = 0;  // prefetch cursor: batch vertex, chunk offset
-                    uint2 cur[kPushAhead];
-                    uint32_t ct[kPushAhead], cco[kPushAhead];
-                    auto load_group = [&](uint2* dst, uint32_t* dt, uint32_t* dc) {
-    #pragma unroll
-                        for (int jj = 0; jj < kPushAhead; ++jj) {
-                            dst[jj] = make_uint2(0u, 1u);
-                            dt[jj] = cnt;
-                            dc[jj] = 0;
-                            if (pt < cnt) {
-                                const uint32_t vb = __shfl_sync(kFullMask, myb, pt);
-                                const uint32_t vd = __shfl_sync(kFullMask, myd, pt);
-                                if (pc + lane < vd) dst[jj] = __ldg(p.adjd + vb + pc + lane);
-                                dt[jj] = pt;
-                                dc[jj] = pc;
-                                pc += 32;
-                                if (pc >= vd) {
-                                    ++pt;
-                                    pc = 0;
-                                }
-                            }
-                        }
-                    };
-                    load_group(cur, ct, cco);
-                    Real r = Real(0);
-                    while (ct[0] < cnt) {
-                        uint2 nxt[kPushAhead];
-                        uint32_t nt[kPushAhead], nc[kPushAhead];
-                        load_group(nxt, nt, nc);
-    #pragma unroll
-                        for (int jj = 0; jj < kPushAhead; ++jj) {
-                            if (ct[jj] < cnt) {
-                                const uint32_t t = ct[jj], c0 = cco[jj];
-                                const uint32_t vd = __shfl_sync(kFullMask, myd, t);
-                                if (c0 == 0) {
-                                    const uint32_t v = __shfl_sync(kFullMask, myv, t);
-                                    r = pvec[v];
-                                    __syncwarp();
-                                    if (lane == 0) pvec[v] = Real(0);
-                                    __syncwarp();
-                                    st_tr += vd;
-                                }
-                                const bool act = c0 + lane < vd;
-                                const uint32_t cu = cur[jj].x, cd = cur[jj].y;
-                                // a run of one repeated neighbour (adjacent lanes: rows are
-                                // sorted) is applied by its first lane, one add per repeat in
-                                // order; runs continued from the previous chunk were applied
-                                // before this one, as the reference's sequential loop does
-                                bool lead = act;
-                                uint32_t reps = 1;
-                                if (p.multi) {
-                                    const uint32_t pcu = __shfl_up_sync(kFullMask, cu, 1);
-                                    const bool follow = act && lane > 0 && pcu == cu;
-                                    const unsigned fb = __ballot_sync(kFullMask, follow);
-                                    lead = act && !follow;
-                                    const unsigned rest = lane == 31 ? 0u : (fb >> (lane + 1));
-                                    reps = uint32_t(__ffs(int(~rest)));
-                                }
-                                bool fresh = false;
-                                if (lead && vis[cu] == 0) {
-                                    vis[cu] = 1;
-                                    fresh = true;
-                                }
-                                const unsigned bal = __ballot_sync(kFullMask, fresh);
-                                if (fresh) {
-                                    qn[qns + __popc(bal & lt)] = cu;
-                                    pcost += cd;
-                                }
-                                qns += __popc(bal);
-                                if (lead) {
-                                    const Real add = rdiv(r, from_u64<Real>(cd));
-                                    Real pv = pvec[cu];
-                                    for (uint32_t k = 0; k < reps; ++k) pv = radd(pv, add);
-                                    pvec[cu] = pv;
-                                }
-                                __syncwarp();
-                            }
-                        }
-    #pragma unroll
-                        for (int jj = 0; jj < kPushAhead; ++jj) {
-                            cur[jj] = nxt[jj];
-                            ct[jj] = nt[jj];
-                            cco[jj] = nc[jj];
-                        }
-                    }
-                }
-                }
-                __syncwarp();
-                lap(1);
-                // preds[row] += (pvec[src] - pvec[adj]) / ds (:235-237); the first round adds to the
-                // initial 1 / ds directly
-                {
-                    const Real ps = pvec[src];
-                    struct SlotPred {
-                        uint32_t w;
-                        Real old;
-                    };
-                    pipelined<SlotPred>(dsi,
-                        [&](uint32_t c, SlotPred* r) {
-    #pragma unroll
-                            for (int b = 0; b < kB; ++b) {
-                                const uint32_t o = c + 32 * b + lane;
-                                r[b].w = NONE;
-                                r[b].old = pinit;
-                                if (o < dsi) {
-                                    r[b].w = __ldg(adj + rb + o);
-                                    if (ell > 0) r[b].old = p.preds[rb + o];
-                                }
-                            }
-                        },
-                        [&](uint32_t c, const SlotPred* r) {
-    #pragma unroll
-                            for (int b = 0; b < kB; ++b)
-                                if (r[b].w != NONE)
-                                    p.preds[rb + c + 32 * b + lane] =
-                                        row_update<Real, Real>(r[b].old, ps, pvec[r[b].w], ds);
-                        });
-                }
-                // clear the new frontier's flags and take its residual max / min (:484-491; max and
-                // min do not depend on order)
-                mx = Real(0);
-                mn = Real(1);
-                pipelined<uint32_t>(qns,
-                    [&](uint32_t i0, uint32_t* r) {
-    #pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const uint32_t i = i0 + 32 * b + lane;
-                            r[b] = i < qns ? qn[i] : NONE;
-                        }
-                    },
-                    [&](uint32_t, const uint32_t* r) {
-    #pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            if (r[b] == NONE) continue;
-                            vis[r[b]] = 0;
-                            const Real val = pvec[r[b]];
-                            mx = std_max(mx, val);
-                            mn = std_min(mn, val);
-                        }
-                    });
-                __syncwarp();
-                { uint32_t* tmp = q; q = qn; qn = tmp; }
-                qs = qns;
-                ++ell;
-                lap(2);
-            }
-        }
-        if (timed_out) {
-            if (lane == 0) atomicOr(p.work + 1, kErrDeadline);
-            dirty = true;
-            break;
-        }
-        st_rounds += ell;
-        if (p.trace_ell && lane == 0) p.trace_ell[src] = uint32_t(ell);
-
-        // slots that still need walks (rest = tau - ell > 0), compacted in slot order
-        uint32_t nitems = 0;
-        pipelined<int>(dsi, load_tau, [&](uint32_t c, const int* tv) {
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                const uint32_t o = c + 32 * b + lane;
-                const bool has = o < dsi && tv[b] - ell > 0;
-                const unsigned hb = __ballot_sync(kFullMask, has);
-                if (has)
-                    items[nitems + __popc(hb & lt)] =
-                        WalkItem{rb + o, __ldg(adj + rb + o), uint32_t(tv[b] - ell), 0u, 0ull};
-                nitems += __popc(hb);
-            }
-        });
-        __syncwarp();
-
-        // ---- edge bound (:414-442, :504-506); it only feeds chi of walking slots ----
-        Real edge_max = Real(0);
-        if (nitems == 0) {
-        } else if (p.gamma == 1) {
-            edge_max = rmul(Real(2), gmax);
-        } else {
-            const int nnz = int(qs);
-            const int rg = p.gamma < nnz ? p.gamma : nnz;
-            uint32_t* set = qn;  // free after the last swap
-            int sc = 0;
-            Real gamma_max;
-            if (p.gamma < nnz) {
-                Real t;
-                int need_eq;
-                kth_largest<Real>(q, qs, pvec, rg, t, need_eq);
-                int taken_eq = 0;
-                pipelined<uint32_t>(qs,
-                    [&](uint32_t i0, uint32_t* r) {
-#pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const uint32_t i = i0 + 32 * b + lane;
-                            r[b] = i < qs ? q[i] : NONE;
-                        }
-                    },
-                    [&](uint32_t, const uint32_t* r) {
-#pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const Real x = r[b] != NONE ? pvec[r[b]] : Real(-INFINITY);
-                            const bool gt = x > t, eq = x == t;
-                            const unsigned be = __ballot_sync(kFullMask, eq);
-                            const bool take_eq = eq && taken_eq + __popc(be & lt) < need_eq;
-                            const bool take = (gt || take_eq) && sc < rg;
-                            const unsigned bt = __ballot_sync(kFullMask, take);
-                            if (take) set[sc + __popc(bt & lt)] = r[b];
-                            sc += __popc(bt);
-                            taken_eq += __popc(__ballot_sync(kFullMask, take_eq));
-                        }
-                    });
-                gamma_max = std_min(Real(1), t);
-            } else {
-                for (uint32_t i = lane; i < qs; i += 32) set[i] = q[i];
-                sc = int(qs);
-                gamma_max = Real(0);
-            }
-            __syncwarp();
-            edge_max = radd(gmax, gamma_max);
-            for (int i = lane; i < sc; i += 32) vis[set[i]] = 2;
-            __syncwarp();
-            // pairs (u, w) with both in the set and w adjacent to u: the members' adjacency lists
-            // are flattened 32 members at a time so a warp scans them in parallel
-            Real best = edge_max;
-            for (int s0 = 0; s0 < sc; s0 += 32) {
-                uint32_t ub = 0, ud = 0;
-                Real pu = Real(0);
-                if (s0 + int(lane) < sc) {
-                    const uint32_t u = set[s0 + lane];
-                    pu = pvec[u];
-                    ub = __ldg(idx + u);
-                    ud = __ldg(idx + u + 1) - ub;
-                }
-                uint32_t incl = ud;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
-                    if (lane >= uint32_t(o)) incl += y;
-                }
-                const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-                const uint32_t excl = incl - ud;
-                for (uint32_t e0 = 0; e0 < total; e0 += 32) {
-                    const uint32_t e = e0 + lane;
-                    uint32_t mm = 0;
-#pragma unroll
-                    for (uint32_t step = 16; step; step >>= 1) {
-                        const uint32_t cand = mm + step;
-                        const uint32_t ex = __shfl_sync(kFullMask, excl, cand & 31u);
-                        if (cand < 32u && ex <= e) mm = cand;
-                    }
-                    const uint32_t mb = __shfl_sync(kFullMask, ub, mm);
-                    const uint32_t mex = __shfl_sync(kFullMask, excl, mm);
-                    const Real mpu = __shfl_sync(kFullMask, pu, mm);
-                    if (e < total) {
-                        const uint32_t w = __ldg(adj + mb + (e - mex));
-                        if (vis[w] == 2) best = std_max(best, radd(mpu, pvec[w]));
-                    }
-                }
-            }
-            edge_max = warp_max(best);
-            __syncwarp();
-            for (int i = lane; i < sc; i += 32) vis[set[i]] = 0;
-            __syncwarp();
-        }
-        lap(4);
-
-        // ---- chi and walk counts per edge (:392-412, :508-521) ----
-        // Neighbourhood max / min of the walking slots' targets, 32 slots at a time: their
-        // adjacency lists are concatenated and each lane walks entries lane, lane + 32, ... with a
-        // cursor over the slots' start offsets (in shared memory; entries of a slot are
-        // consecutive, so the cursor rarely moves), keeps its running max / min in registers and
-        // flushes them with one shared atomic when it leaves a slot.  Then each lane forms its
-        // slot's chi and nr with the reference's roundings.
-        if (nitems) {
-            Real smax = Real(0), smin = Real(FLT_MAX);
-            pipelined<uint32_t>(dsi, load_adj, [&](uint32_t, const uint32_t* w) {
-#pragma unroll
-                for (int b = 0; b < kB; ++b) {
-                    if (w[b] == NONE) continue;
-                    const Real x = pvec[w[b]];
-                    smax = std_max(smax, x);
-                    smin = std_min(smin, x);
-                }
-            });
-            smax = warp_max(smax);
-            smin = warp_min(smin);
-            const Real dse = from_f64<Real>(__dmul_rn(double(ds), p.eps));
-            const double den = double(rmul(dse, dse));
-            uint32_t* exs = reinterpret_cast<uint32_t*>(acc + 64);  // 33 slot offsets
-            uint32_t* vbs = exs + 33;                               // 32 row starts
-            for (uint32_t s0 = 0; s0 < nitems; s0 += 32) {
-                const uint32_t my = s0 + lane;
-                uint32_t vb = 0, vd = 0, L = 0;
-                if (my < nitems) {
-                    const WalkItem it = items[my];
-                    vb = __ldg(idx + it.v);
-                    vd = __ldg(idx + it.v + 1) - vb;
-                    L = it.len;
-                }
-                acc[lane] = ord_bits(Real(0));
-                acc[32 + lane] = ord_bits(Real(FLT_MAX));
-                uint32_t incl = vd;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(kFullMask, incl, o);
-                    if (lane >= uint32_t(o)) incl += y;
-                }
-                const uint32_t total = __shfl_sync(kFullMask, incl, 31);
-                exs[lane] = incl - vd;
-                vbs[lane] = vb;
-                if (lane == 31) exs[32] = total;
-                __syncwarp();
-                uint32_t cm = 0;                  // address cursor
-                uint32_t cseg = 32;               // accumulation cursor (32: none yet)
-                Real amx = Real(0), amn = Real(FLT_MAX);
-                auto flush = [&]() {
-                    if (cseg < 32u) {
-                        atomicMax(acc + cseg, ord_bits(amx));
-                        atomicMin(acc + 32 + cseg, ord_bits(amn));
-                    }
-                };
-                struct Ent {
-                    uint32_t seg, w;
-                };
-                pipelined<Ent>(total,
-                    [&](uint32_t e0, Ent* r) {
-#pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            const uint32_t e = e0 + 32 * b + lane;
-                            r[b].seg = 32u;
-                            r[b].w = 0u;
-                            if (e < total) {
-                                while (exs[cm + 1] <= e) ++cm;
-                                r[b].seg = cm;
-                                r[b].w = __ldg(adj + vbs[cm] + (e - exs[cm]));
-                            }
-                        }
-                    },
-                    [&](uint32_t, const Ent* r) {
-#pragma unroll
-                        for (int b = 0; b < kB; ++b) {
-                            if (r[b].seg == 32u) continue;
-                            if (r[b].seg != cseg) {
-                                flush();
-                                cseg = r[b].seg;
-                                amx = Real(0);
-                                amn = Real(FLT_MAX);
-                            }
-                            const Real x = pvec[r[b].w];
-                            amx = std_max(amx, x);
-                            amn = std_min(amn, x);
-                        }
-                    });
-                flush();
-                if (my < nitems) {
-                    const Real tmax = from_ord<Real>(acc[lane]);
-                    const Real tmin = from_ord<Real>(acc[32 + lane]);
-                    // get_chi (:410): float terms rounded as in the reference, summed in double
-                    const int Li = int(L);
-                    const double A = __dadd_rn(double(gmax), __ddiv_rn(double(radd(smax, tmax)), 2.0));
-                    const double B = __dadd_rn(A, double(rmul(Real(Li - 1), edge_max)));
-                    const double C = __dsub_rn(__dsub_rn(B, double(smin)), double(tmin));
-                    const double E = __dsub_rn(C, double(rmul(Real(2 * (Li - 1)), gmin)));
-                    const Real chi = from_f64<Real>(E);
-                    // nr (:519-521)
-                    const Real c8 = rmul(Real(8), rmul(chi, chi));
-                    const double num = __dmul_rn(double(c8), p.logmd);
-                    const double nrd = std_max(ceil(__ddiv_rn(num, den)), 1.0);
-                    unsigned long long nr = (unsigned long long)nrd;
-                    nr += 8ull - (nr % 8ull);
-                    if (nr > kMaxWalks) {
-                        atomicOr(p.work + 1, kErrWalkCount);
-                        nr = 0;  // skipped by the walk loop
-                    } else {
-                        st_we += 1;
-                        st_wc += nr;
-                        st_wh += nr * (unsigned long long)L;
-                    }
-                    items[my].nr = nr;
-                    if (p.trace_nr) p.trace_nr[items[my].pos] = uint32_t(nr);
-                }
-                __syncwarp();
-            }
-        }
-        lap(5);
-
-        // ---- 2-way bouquet walks (:241-391): four bouquets per warp, one per 8-lane group ----
-        if (nitems) {
-            const uint32_t j = lane & 7, grp = lane >> 3;
-            uint32_t next = 0;
-            bool has = false, start = false, primary = true;
-            WalkItem it{};
-            unsigned long long bi = 0;
-            uint32_t len = 0, step = 0, cur = 0, cur2 = 0, sec = 0, sec2 = 0, state = 0;
-            Real x = Real(0);
-            // Each hop's residual difference is added to x one hop later (after the next hop's
-            // row offsets are requested), so the residual loads overlap the next hop instead of
-            // stalling it; the adds stay in hop order, and the last one is made before the
-            // item's lanes are summed.
-            Real pa = Real(0), pb = Real(0);
-            bool pend = false;
-            while (true) {
-                const unsigned need = __ballot_sync(kFullMask, !has && j == 0);
-                if (!has) {
-                    const uint32_t rank = __popc(need & ((1u << (grp * 8)) - 1u));
-                    const uint32_t my = next + rank;
-                    if (my < nitems) {
-                        it = items[my];
-                        if (it.nr) {
-                            has = true;
-                            start = true;
-                            bi = 0;
-                            x = Real(0);
-                            step = uint32_t(0xffffffffull / it.nr);
-                        }
-                    }
-                }
-                next += __popc(need);
-                if (!__any_sync(kFullMask, has) && next >= nitems) break;
-                if (has && start) {
-                    cur = src;
-                    cur2 = it.v;
-                    sec = (uint32_t(bi) + j + 1u) * step;
-                    sec2 = sec;
-                    state = sec;
-                    primary = true;
-                    len = 0;
-                    start = false;
-                }
-                const unsigned z =
-                    __ballot_sync(kFullMask, has && primary && (sec == 0u || sec2 == 0u));
-                if (has && primary && ((z >> (grp * 8)) & 0xffu)) {
-                    primary = false;
-                    if (j == 0) ++st_fb;
-                }
-                bool item_done = false;
-                if (has) {
-                    const uint32_t b1 = __ldg(idx + cur), d1 = __ldg(idx + cur + 1) - b1;
-                    const uint32_t b2 = __ldg(idx + cur2), d2 = __ldg(idx + cur2 + 1) - b2;
-                    if (pend) x = radd(x, rsub(pa, pb));
-                    uint32_t k1, k2;
-                    if (primary) {
-                        k1 = __umulhi(sec ^ fmix32(cur), d1);
-                        k2 = __umulhi(sec2 ^ fmix32(cur2), d2);
-                        sec *= d1;
-                        sec2 *= d2;
-                    } else {
-                        const uint32_t r1 = splitmix32(state);
-                        const uint32_t r2 = splitmix32(state);
-                        k1 = r1 % d1;
-                        k2 = r2 % d2;
-                    }
-                    cur = __ldg(adj + b1 + k1);
-                    cur2 = __ldg(adj + b2 + k2);
-                    pa = pvec[cur];
-                    pb = pvec[cur2];
-                    pend = true;
-                    if (++len == it.len) {
-                        bi += 8;
-                        start = true;
-                        item_done = bi >= it.nr;
-                    }
-                }
-                if (__any_sync(kFullMask, item_done)) {
-                    if (item_done && pend) {
-                        x = radd(x, rsub(pa, pb));
-                        pend = false;
-                    }
-                    // the eight lanes summed 0..7, then preds += xij / (ds * nr) (:386-390, :525)
-                    Real s = Real(0);
-#pragma unroll
-                    for (int b = 0; b < 8; ++b)
-                        s = radd(s, __shfl_sync(kFullMask, x, int(grp * 8 + b)));
-                    if (item_done && j == 0)
-                        p.preds[it.pos] =
-                            radd(p.preds[it.pos], rdiv(s, rmul(ds, from_u64<Real>(it.nr))));
-                    if (item_done) has = false;
-                }
-            }
-        }
-        lap(6);
-        // ---- next source starts from an all-zero residual vector ----
-        __syncwarp();
-        pipelined<uint32_t>(qs,
-            [&](uint32_t i0, uint32_t* r) {
-#pragma unroll
-                for (int b = 0; b < kB; ++b) {
-                    const uint32_t i = i0 + 32 * b + lane;
-                    r[b] = i < qs ? q[i] : NONE;
-                }
-            },
-            [&](uint32_t, const uint32_t* r) {
-#pragma unroll
-                for (int b = 0; b < kB; ++b)
-                    if (r[b] != NONE) pvec[r[b]] = Real(0);
-            });
-        if (lane == 0) pvec[src] = Real(0);
-        __syncwarp();
-        lap(7);
-    }
-    if (!SMEM && lane == 0) p0.wclean[gw] = (cleared && !dirty) ? 1 : 0;
-    flush_stats(pk.g[last_gi == 0xffffffffu ? 0u : last_gi].stats);
-}
-
 // ---- walks of the block push's sources, as their own launch --------------------------------------
 // After a block push the per-source stage leaves each source's walking slots in a queue; this lean
 // kernel walks them with many more warps in flight.  Everything a lane computes is what the
@@ -2794,6 +1729,7 @@ __global__ void __launch_bounds__(kHeavyThreads) heavy_walk_kernel(const WalkQue
 }
 
 #include "mixed_source.cuh"
+#include "gs_source.cuh"
 
 // ---- stage 3: symmetrise (src/aesc.h:532-550) -----------------------------------------------------
 // score[q] = p[q] + p[q'] with q' the slot that lands on q (sym_src; none in a row without its
@@ -3396,94 +2332,110 @@ bool run_mixed(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMarks
     return true;
 }
 
-// Per-source stage of the parity forms; false when it is left to a batch.
+// Blocks of the FP32 / FP64 forms' per-source kernel over up to n vertices.
+struct GsLayout {
+    unsigned blocks, threads;
+    size_t smem, q_bytes, item_bytes, vec_bytes;
+    size_t scratch() const { return q_bytes + item_bytes + vec_bytes + 256; }
+};
+template <class Real, class Pack>
+GsLayout gs_layout(bool use_smem, uint64_t n, uint64_t max_degree, uint64_t rows, int num_sms) {
+    GsLayout l;
+    l.threads = unsigned(use_smem ? GsShape<Real, true>::kThreads : GsShape<Real, false>::kThreads);
+    l.smem = gs_shared_bytes<Real>(use_smem, n);
+    const void* kern = use_smem ? reinterpret_cast<const void*>(source_kernel<Real, true, Pack>)
+                                : reinterpret_cast<const void*>(source_kernel<Real, false, Pack>);
+    int per_sm = blocks_per_sm(kern, int(l.threads), l.smem);
+    if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "source kernel does not fit on an SM");
+    // Small vectors: where registers and not shared memory limit the 128-thread blocks and there are
+    // sources for more than one round of them, blocks of half the threads, so that more sources push
+    // at a time (FP64, n = 2,000, 20 neighbours, eps = 0.005: 2.81 ms against 3.13; at n = 600, one
+    // round, 0.626 against 0.610; at n = 5,500, shared memory the limit, 17.3 against 16.7).
+    if (use_smem && rows * 4 > uint64_t(num_sms) * per_sm * 5) {
+        const int half = blocks_per_sm(kern, int(l.threads) / 2, l.smem);
+        if (half > per_sm) {
+            l.threads /= 2;
+            per_sm = half;
+        }
+    }
+    // vectors and lists in HBM: eight blocks per SM where more would take over 16 GB
+    if (!use_smem && uint64_t(num_sms) * per_sm * n * (8 + sizeof(Real)) > (uint64_t(16) << 30))
+        per_sm = std::min(per_sm, 8);
+    l.blocks = unsigned(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(num_sms) * per_sm, rows)));
+    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
+    l.q_bytes = align(size_t(l.blocks) * 2 * size_t(n) * 4);
+    l.item_bytes = align(size_t(l.blocks) * std::max<uint64_t>(max_degree, 1) * sizeof(WalkItem));
+    l.vec_bytes = use_smem ? 0 : align(size_t(l.blocks) * size_t(n) * sizeof(Real));
+    return l;
+}
+template <class Real>
+void carve_gs(SourceParams<Real>& p, const GsLayout& l, unsigned char* base, uint64_t n, uint64_t max_degree) {
+    p.scratch_n = uint32_t(n);
+    p.max_degree = uint32_t(std::max<uint64_t>(max_degree, 1));
+    p.qbuf = reinterpret_cast<uint32_t*>(base);
+    base += l.q_bytes;
+    p.items = reinterpret_cast<WalkItem*>(base);
+    base += l.item_bytes;
+    p.pvec_g = l.vec_bytes ? reinterpret_cast<Real*>(base) : nullptr;
+}
+template <class Real, class Pack>
+void launch_gs(bool use_smem, const GsLayout& l, cudaStream_t s, bool pdl, const Pack& pk) {
+    if (use_smem) launch(source_kernel<Real, true, Pack>, l.blocks, l.threads, l.smem, s, pdl, pk);
+    else launch(source_kernel<Real, false, Pack>, l.blocks, l.threads, l.smem, s, pdl, pk);
+    TGTP_LAUNCH_CHECK("source_kernel");
+}
+
+// Largest shared memory of a block that keeps its residual vector there by default.  Shared memory
+// shortens a step of the push and limits the sources in flight; the HBM tier's windowed push gains
+// on it as rows get shorter.  Measured, shared memory against HBM, in ms:
+//   44 neighbours  FP64  51 KB 1.55 / 1.73,  63 KB 2.53 / 2.31;  FP32  55 KB 3.12 / 3.77
+//   30             FP64  31 KB 1.73 / 2.62,  51 KB 4.35 / 4.94
+//   20             FP64  23 KB 2.81 / 3.12,  39 KB 8.31 / 8.30,  51 KB 16.7 / 12.8
+//                  FP32  31 KB 5.43 / 6.89,  39 KB 7.56 / 8.83,  51 KB 12.7 / 12.8
+//   15, 14         FP64  23 KB 2.78 / 2.95,  35 KB 7.91 / 7.18;  FP32  21 KB 4.34 / 4.94,  35 KB 12.7 / 12.1
+//   9.5            FP64  19 KB 2.03 / 2.24,  39 KB 8.55 / 7.19
+inline size_t gs_smem_most(uint64_t n, uint64_t m) {
+    return size_t(m >= 24 * n ? 56 : m >= 18 * n ? 40 : 24) * 1024;
+}
+
+// Per-source stage of the FP32 and FP64 forms; false when it is left to a batch.
 template <class Real>
 bool run_sources(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMarks& rm, bool multi, double logmd) {
     cudaStream_t s = g->stream;
     const uint64_t n = g->n, m = g->m;
     const int key = form_key(cfg);
-    auto* stats = g->stats.as<unsigned long long>();
-    auto* work = run_work(g);
-    // source kernel.  Shared-memory tier: each warp's residual vector and flags in shared memory.
-    // Global tier (large n): vectors in HBM.  The layout (tier, warps per block) comes from the
-    // handle's tuned choice for this form, else from the default rule (shared memory with one-warp
-    // blocks while a warp's copy fits in 112 KB, else HBM with four warps per block);
-    // TGTP_PVEC_TIER=smem|global overrides the tier of the default rule.
-    const size_t pv_bytes = (size_t(n) * sizeof(Real) + 15) & ~size_t(15);
-    const size_t vis_bytes = (size_t(n) + 15) & ~size_t(15);
-    const size_t per_warp = pv_bytes + vis_bytes + kAccBytes;
-    bool use_smem;
-    int wpb;
-    if (g->src_layout[key]) {
-        use_smem = (g->src_layout[key] & kLayoutSmem) != 0;
-        wpb = std::max(1, g->src_layout[key] & 0xff);
-    } else {
-        use_smem = per_warp <= size_t(112) * 1024;
-        if (const char* t = std::getenv("TGTP_PVEC_TIER")) {
-            if (std::string(t) == "global") use_smem = false;
-            else if (std::string(t) == "smem" && per_warp <= size_t(227) * 1024) use_smem = true;
-        }
-        wpb = use_smem ? 1 : 4;
+    const uint16_t lay = g->src_layout[key];
+    // Shared-memory tier: the residual vector in shared memory; HBM tier: in HBM.  The tuned
+    // layout's, else shared memory while a block takes at most gs_smem_most; TGTP_PVEC_TIER=smem|global
+    // overrides the rule.
+    const size_t smem = gs_shared_bytes<Real>(true, n);
+    const bool fits = smem + 512 <= size_t(227) * 1024;
+    bool use_smem = smem <= gs_smem_most(n, m);
+    if (lay) use_smem = fits && (lay & kLayoutSmem) != 0;
+    else if (const char* t = std::getenv("TGTP_PVEC_TIER")) {
+        if (std::string(t) == "global") use_smem = false;
+        else if (std::string(t) == "smem" && fits) use_smem = true;
     }
-    if (use_smem && per_warp * wpb > size_t(227) * 1024)
-        fail(TGTP_ERR_UNSUPPORTED, "source layout does not fit in shared memory");
-    const int threads = wpb * 32;
-    const size_t smem = use_smem ? per_warp * wpb : size_t(wpb) * kAccBytes;
     using Pack1 = SourcePack<Real, 1>;
-    auto kern = use_smem ? source_kernel<Real, true, Pack1>
-                         : source_kernel<Real, false, Pack1>;
-    const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(kern), threads, smem);
-    if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "source kernel does not fit on an SM");
-    uint64_t blocks = uint64_t(g->num_sms) * per_sm;
-    blocks = std::min<uint64_t>(blocks, (n + wpb - 1) / wpb);
-    const uint64_t warps = blocks * wpb;
-    const size_t maxd = std::max<uint32_t>(g->max_degree, 1);
-    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t q_bytes = align(warps * 2 * size_t(n) * 4);
-    const size_t it_bytes = align(warps * maxd * sizeof(WalkItem));
-    const size_t pvg_bytes = use_smem ? 0 : align(warps * size_t(n) * sizeof(Real));
-    const size_t visg_bytes = use_smem ? 0 : align(warps * vis_bytes);
-    grow(g, g->scratch, q_bytes + it_bytes + pvg_bytes + visg_bytes + 256);
-    unsigned char* base = g->scratch.as<unsigned char>();
-    SourceParams<Real> p;
+    const GsLayout l = gs_layout<Real, Pack1>(use_smem, n, g->max_degree, n, g->num_sms);
+    grow(g, g->scratch, l.scratch());
+    SourceParams<Real> p{};
+    carve_gs(p, l, g->scratch.as<unsigned char>(), n, g->max_degree);
     p.idx = g->idx.as<uint32_t>();
     p.adj = g->adj.as<uint32_t>();
-    p.deg = g->deg.as<uint32_t>();
+    p.adjd = g->adjd.as<uint2>();
+    p.dinv = g->dinv.as<double>();
     p.n = uint32_t(n);
     p.taus = g->taus.as<int>();
     p.preds = g->preds.as<Real>();
-    p.work = work;
+    p.work = run_work(g);
     p.rows = rm.list;
-    p.qbuf = reinterpret_cast<uint32_t*>(base);
-    base += q_bytes;
-    p.items = reinterpret_cast<WalkItem*>(base);
-    base += it_bytes;
-    p.pvec_g = use_smem ? nullptr : reinterpret_cast<Real*>(base);
-    base += pvg_bytes;
-    p.vis_g = use_smem ? nullptr : base;
-    // the per-warp "vectors are zero" marks hold only for the same carving of the same scratch
-    {
-        const uint64_t sig[5] = {uint64_t(key) | (uint64_t(use_smem) << 8) | (uint64_t(wpb) << 16),
-                                 blocks, uint64_t(n),
-                                 uint64_t(reinterpret_cast<uintptr_t>(g->scratch.ptr)),
-                                 uint64_t(g->scratch.bytes)};
-        grow(g, g->wclean, warps + 16);
-        if (std::memcmp(sig, g->wclean_sig, sizeof(sig)) != 0) {
-            TGTP_CUDA(cudaMemsetAsync(g->wclean.ptr, 0, warps + 16, s));
-            std::memcpy(g->wclean_sig, sig, sizeof(sig));
-        }
-        p.wclean = g->wclean.as<unsigned char>();
-    }
-    p.vis_stride = vis_bytes;
-    p.smem_per_warp = per_warp;
-    p.max_degree = uint32_t(maxd);
     p.eps = cfg.epsilon;
     p.logmd = logmd;
     p.gamma = cfg.gamma;
-    p.stats = stats;
-    p.adjd = g->adjd.as<uint2>();
+    p.stats = g->stats.as<unsigned long long>();
     p.budget_ns = deadline_from_env();
-    p.trace_nr = p.trace_ell = nullptr;
+    p.multi = multi;
     if (g->trace_on) {
         grow(g, g->trace, sizeof(uint32_t) * (m + n));
         TGTP_CUDA(cudaMemsetAsync(g->trace.ptr, 0, sizeof(uint32_t) * (m + n), s));
@@ -3491,30 +2443,38 @@ bool run_sources(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMar
         p.trace_ell = p.trace_nr + m;
         g->trace_valid = true;
     }
-    p.multi = multi;
-    p.scratch_n = uint32_t(n);
+    // the per-block "vector is zero" marks hold only for the same carving of the same scratch
     {
-        // The windowed push pays off when rows are short: several frontier vertices share a
-        // 32-entry step.  When rows average 32 entries or more, each vertex fills its steps anyway
-        // and adjacent frontier vertices cut windows often, so one vertex at a time is used
-        // (4,039-vertex Chung-Lu graph, 44 entries per row: 0.73 against 0.86 ms at eps = 0.01;
-        // sparse Chung-Lu, 9.3 per row: 4.1 against 1.4 s at eps = 0.005).  The tuned layout,
-        // then TGTP_GS_WINDOW=0/1, override the rule.
-        const uint16_t lay = g->src_layout[key];
+        const uint64_t sig[5] = {uint64_t(key) | (uint64_t(use_smem) << 8) | (uint64_t(1) << 62), l.blocks, uint64_t(n),
+                                 uint64_t(reinterpret_cast<uintptr_t>(g->scratch.ptr)),
+                                 uint64_t(g->scratch.bytes)};
+        grow(g, g->wclean, l.blocks + 16);
+        if (std::memcmp(sig, g->wclean_sig, sizeof(sig)) != 0) {
+            TGTP_CUDA(cudaMemsetAsync(g->wclean.ptr, 0, l.blocks + 16, s));
+            std::memcpy(g->wclean_sig, sig, sizeof(sig));
+        }
+        p.clean = g->wclean.as<unsigned char>();
+    }
+    {
+        // The windowed push pays off when rows are short: several frontier vertices share a 32-entry
+        // step.  With long rows each vertex fills its steps anyway and adjacent frontier vertices cut
+        // windows often.  In shared memory the line is at 15 neighbours (one vertex at a time /
+        // windowed, ms: 9.5 neighbours 2.96 / 2.02; 14: 3.04 / 2.78; 16: 2.37 / 2.39; 20: 2.81 / 3.17;
+        // 44: 0.73 / 1.42), in HBM, where a step waits for its words, at 32 (20: 18.7 / 12.8; 30:
+        // 5.18 / 4.94; 44: 1.73 / 2.44).  The tuned layout, then TGTP_GS_WINDOW=0/1, override the rule.
         const char* e = std::getenv("TGTP_GS_WINDOW");
         if (lay & kLayoutWindow) p.gs_window = true;
         else if (lay & kLayoutNoWindow) p.gs_window = false;
         else if (e) p.gs_window = std::string(e) != "0";
-        else p.gs_window = m < 32 * n;
+        else p.gs_window = m < (use_smem ? 15 : 32) * n;
     }
+    p.claim = run_work(g);
+    if (defer_to_batch(g, cfg, out, use_smem, p)) return false;
     Pack1 pk;
     pk.count = 1;
-    p.claim = work;
-    if (defer_to_batch(g, cfg, out, use_smem, p)) return false;
     pk.g[0] = p;
     ScopedKernel k(g->prof, s, "source");
-    launch(kern, unsigned(blocks), unsigned(threads), smem, s, true, pk);
-    TGTP_LAUNCH_CHECK("source_kernel");
+    launch_gs<Real>(use_smem, l, s, true, pk);
     return true;
 }
 
@@ -3661,69 +2621,39 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
     launch_finish<Real, Acc>(g, out);
 }
 
-// The persistent source kernel of one batch group: per-warp scratch for the group's largest
+// The persistent source kernel of one batch group: per-block scratch for the group's largest
 // graph, packs of up to kBatchPack graphs, each pack one launch on `s` with its own claim counter.
-template <class Real, bool SMEM>
+template <class Real>
 void launch_group(BatchPlan& plan, BatchGroup& grp, cudaStream_t s, int num_sms) {
     using Pack = SourcePack<Real, kBatchPack>;
     static_assert(sizeof(Pack) < 32000, "pack must fit in the kernel parameter space");
-    uint32_t sn = 1, maxd = 1;
-    uint64_t rows = 0;
+    uint64_t sn = 1, maxd = 1, rows = 0;
     for (size_t i : grp.members) {
         const tgtp_graph* g = plan.entries[i].g;
-        sn = std::max<uint32_t>(sn, uint32_t(g->n));
-        maxd = std::max<uint32_t>(maxd, g->max_degree);
+        sn = std::max<uint64_t>(sn, g->n);
+        maxd = std::max<uint64_t>(maxd, g->max_degree);
         rows += g->n;
     }
-    const size_t pv_bytes = (size_t(sn) * sizeof(Real) + 15) & ~size_t(15);
-    const size_t vis_bytes = (size_t(sn) + 15) & ~size_t(15);
-    const size_t per_warp = pv_bytes + vis_bytes + kAccBytes;
-    const int wpb = SMEM ? 1 : 4;
-    const int threads = 32 * wpb;
-    const size_t smem = SMEM ? per_warp * wpb : size_t(wpb) * kAccBytes;
-    auto kern = source_kernel<Real, SMEM, Pack>;
-    const int per_sm = blocks_per_sm(reinterpret_cast<const void*>(kern), threads, smem);
-    if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "batch source kernel does not fit on an SM");
-    uint64_t blocks = std::min<uint64_t>(uint64_t(num_sms) * per_sm, (rows + wpb - 1) / wpb);
-    blocks = std::max<uint64_t>(blocks, 1);
-    const uint64_t warps = blocks * wpb;
-    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t q_bytes = align(warps * 2 * size_t(sn) * 4);
-    const size_t it_bytes = align(warps * maxd * sizeof(WalkItem));
-    const size_t pvg_bytes = SMEM ? 0 : align(warps * size_t(sn) * sizeof(Real));
-    const size_t visg_bytes = SMEM ? 0 : align(warps * vis_bytes);
-    grp.scratch.reserve(q_bytes + it_bytes + pvg_bytes + visg_bytes + 256);
-    grp.wclean.reserve(warps + 16);
+    const GsLayout lay = gs_layout<Real, Pack>(grp.smem, sn, maxd, rows, num_sms);
+    grp.scratch.reserve(lay.scratch());
+    grp.wclean.reserve(lay.blocks + 16);
     const size_t packs = (grp.members.size() + kBatchPack - 1) / kBatchPack;
     grp.claims.reserve(sizeof(unsigned) * (packs + 1));
-    unsigned char* base = grp.scratch.as<unsigned char>();
     // each replay starts from "vectors not known to be zero" and fresh claim counters
-    TGTP_CUDA(cudaMemsetAsync(grp.wclean.ptr, 0, warps + 16, s));
+    TGTP_CUDA(cudaMemsetAsync(grp.wclean.ptr, 0, lay.blocks + 16, s));
     TGTP_CUDA(cudaMemsetAsync(grp.claims.ptr, 0, sizeof(unsigned) * (packs + 1), s));
     for (size_t pk0 = 0; pk0 < grp.members.size(); pk0 += kBatchPack) {
-        Pack pk;
-        pk.count = uint32_t(std::min<size_t>(kBatchPack, grp.members.size() - pk0));
-        for (uint32_t j = 0; j < pk.count; ++j) {
+        auto pk = std::make_unique<Pack>();
+        pk->count = uint32_t(std::min<size_t>(kBatchPack, grp.members.size() - pk0));
+        for (uint32_t j = 0; j < pk->count; ++j) {
             SourceParams<Real> p;
             std::memcpy(&p, plan.entries[grp.members[pk0 + j]].params.data(), sizeof(p));
-            unsigned char* b = base;
-            p.qbuf = reinterpret_cast<uint32_t*>(b);
-            b += q_bytes;
-            p.items = reinterpret_cast<WalkItem*>(b);
-            b += it_bytes;
-            p.pvec_g = SMEM ? nullptr : reinterpret_cast<Real*>(b);
-            b += pvg_bytes;
-            p.vis_g = SMEM ? nullptr : b;
-            p.wclean = grp.wclean.as<unsigned char>();
-            p.vis_stride = vis_bytes;
-            p.smem_per_warp = per_warp;
-            p.max_degree = maxd;
-            p.scratch_n = sn;
+            carve_gs(p, lay, grp.scratch.as<unsigned char>(), sn, maxd);
+            p.clean = grp.wclean.as<unsigned char>();
             p.claim = grp.claims.as<unsigned>() + pk0 / kBatchPack;
-            pk.g[j] = p;
+            pk->g[j] = p;
         }
-        launch(kern, unsigned(blocks), unsigned(threads), smem, s, false, pk);
-        TGTP_LAUNCH_CHECK("source_kernel (batch)");
+        launch_gs<Real>(grp.smem, lay, s, false, *pk);
     }
 }
 
@@ -3790,14 +2720,8 @@ void batch_plan_launch(BatchPlan* plan, cudaStream_t s, int num_sms) {
     }
     for (auto& grp : plan->groups) {
         switch (grp->key) {
-            case 0:
-                if (grp->smem) launch_group<float, true>(*plan, *grp, s, num_sms);
-                else launch_group<float, false>(*plan, *grp, s, num_sms);
-                break;
-            case 1:
-                if (grp->smem) launch_group<double, true>(*plan, *grp, s, num_sms);
-                else launch_group<double, false>(*plan, *grp, s, num_sms);
-                break;
+            case 0: launch_group<float>(*plan, *grp, s, num_sms); break;
+            case 1: launch_group<double>(*plan, *grp, s, num_sms); break;
             default: launch_mixed_group(*plan, *grp, s, num_sms); break;
         }
     }
@@ -3952,7 +2876,6 @@ void aesc_read_stats(tgtp_graph* g, unsigned long long* st) {
 
 int aesc_tune(tgtp_graph* g, const tgtp_config& cfg, float* device_scores, int trials) {
     const int key = form_key(cfg);
-    const size_t rs = cfg.precision == TGTP_PRECISION_FP64 ? 8 : 4;
     const bool mixed = cfg.precision == TGTP_PRECISION_MIXED;
     std::vector<uint16_t> cand;
     if (mixed) {
@@ -3964,12 +2887,13 @@ int aesc_tune(tgtp_graph* g, const tgtp_config& cfg, float* device_scores, int t
         for (int ld = 0; ld < (push_shared_bytes(g->n) <= size_t(227) * 1024 ? 1 : 4); ++ld)
             cand.push_back(uint16_t(kLayoutBlock | 4 | (ld << kLayoutListShift)));
     } else {
-        // residual vectors in shared memory or in HBM, warps per block, windowed or one-vertex push
-        const size_t per_warp = ((g->n * rs + 15) & ~size_t(15)) + ((g->n + 15) & ~size_t(15)) + kAccBytes;
+        // residual vectors in shared memory (four warps a block) or in HBM (two), windowed or
+        // one-vertex push
+        const bool f64 = cfg.precision == TGTP_PRECISION_FP64;
+        const size_t smem = f64 ? gs_shared_bytes<double>(true, g->n) : gs_shared_bytes<float>(true, g->n);
         for (uint16_t pk : {kLayoutWindow, kLayoutNoWindow}) {
-            for (int w : {1, 2})
-                if (per_warp * w <= size_t(227) * 1024) cand.push_back(uint16_t(pk | kLayoutSmem | w));
-            for (int w : {1, 2, 4}) cand.push_back(uint16_t(pk | w));
+            if (smem + 512 <= size_t(227) * 1024) cand.push_back(uint16_t(pk | kLayoutSmem | 4));
+            cand.push_back(uint16_t(pk | 2));
         }
     }
     cudaEvent_t e0, e1;

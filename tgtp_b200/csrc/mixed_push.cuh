@@ -19,39 +19,43 @@
 constexpr uint32_t kHeavyRow = 256;
 constexpr uint32_t kChunk = 512;  // frontier vertices whose adjacency is concatenated at a time
 
-// Shared scratch of the concatenation: entry offsets (kChunk + 1, and 33 words read but not used
-// past them), row start minus offset, the vertex's value.
-struct ChunkScratch {
-    uint32_t offs[kChunk + 34];
-    uint32_t base[kChunk];
-    unsigned long long val[kChunk];
+// Shared scratch of the concatenation of up to C rows: entry offsets (C + 1, and 33 words read but
+// not used past them), row start minus offset, the vertex's value.
+template <int C>
+struct ChunkScratchOf {
+    static constexpr uint32_t kRows = C;
+    uint32_t offs[C + 34];
+    uint32_t base[C];
+    unsigned long long val[C];
     uint32_t tmp[32];
     uint32_t total;
 };
+using ChunkScratch = ChunkScratchOf<kChunk>;
 
 // The segment of entry e among cnt segments starting at offs[0 .. cnt) (offs[cnt] = total > e):
 // the last one that starts at or before e.  All lanes of a warp call it with the same e.
+template <int C>
 __device__ __forceinline__ uint32_t find_segment(const uint32_t* offs, uint32_t cnt, uint32_t e) {
     const uint32_t lane = threadIdx.x & 31;
-    static_assert(kChunk == 512, "two steps of 32 and 16");
-    const uint32_t c0 = lane * 16u;
+    constexpr uint32_t R = C / 32;
+    static_assert(R >= 1 && R <= 32 && R * 32 == C, "a step over 32 runs of R, a step inside one");
+    const uint32_t c0 = lane * R;
     const unsigned b0 = __ballot_sync(kFullMask, c0 < cnt && offs[c0] <= e);
-    const uint32_t coarse = (uint32_t(__popc(b0)) - 1u) * 16u;
-    const uint32_t c1 = coarse + (lane & 15u);
-    const unsigned b1 = __ballot_sync(kFullMask, lane < 16u && c1 < cnt && offs[c1] <= e);
+    const uint32_t coarse = (uint32_t(__popc(b0)) - 1u) * R;
+    const uint32_t c1 = coarse + (lane & (R - 1u));
+    const unsigned b1 = __ballot_sync(kFullMask, lane < R && c1 < cnt && offs[c1] <= e);
     return coarse + uint32_t(__popc(b1)) - 1u;
 }
 
-// Concatenates the rows of up to kChunk vertices: thread i < cnt passes vertex i's row start, its
+// Concatenates the rows of up to C vertices: thread i < cnt passes vertex i's row start, its
 // degree (at least 1) and a value.  Every entry is loaded, load(slot, whether there is an entry), and
-// then used, use(loaded, value of its vertex, the vertex's index in the chunk, the lanes with an
-// entry in this step), with the warp's lanes on consecutive entries.  All threads of the block call it; the scratch is free again after
+// then used, use(loaded, value of its vertex, the vertex's index in the chunk, whether there is an
+// entry), by all lanes of a warp together, on consecutive entries.  All threads of the block call it; the scratch is free again after
 // the caller's next __syncthreads.
-template <class Load, class Use>
-__device__ __forceinline__ uint32_t for_entries(ChunkScratch& s, uint32_t cnt, uint32_t beg, uint32_t deg,
+template <int C, class Load, class Use>
+__device__ __forceinline__ uint32_t for_entries(ChunkScratchOf<C>& s, uint32_t cnt, uint32_t beg, uint32_t deg,
                                                 unsigned long long val, Load load, Use use) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // up to kChunk vertices are passed by the first threads; smaller blocks pass fewer
     const uint32_t off = block_exclusive_scan(deg, s.tmp, &s.total);
     if (threadIdx.x < cnt) {
         s.offs[threadIdx.x] = off;
@@ -64,7 +68,7 @@ __device__ __forceinline__ uint32_t for_entries(ChunkScratch& s, uint32_t cnt, u
     const uint32_t per = ((total + nw - 1) / nw + 31u) & ~31u;
     const uint32_t e0 = warp * per, end = min(total, e0 + per);
     if (e0 < end) {
-        uint32_t seg = find_segment(s.offs, cnt, e0);
+        uint32_t seg = find_segment<C>(s.offs, cnt, e0);
         uint32_t e = e0;
         // lane's segment in the step of entries e .. e + 31, and the step's next first segment
         auto step = [&](uint32_t at, uint32_t& first) {
@@ -91,8 +95,7 @@ __device__ __forceinline__ uint32_t for_entries(ChunkScratch& s, uint32_t cnt, u
                 slotn = inn ? s.base[kn] + en + lane : 0u;
                 xn = load(slotn, inn);
             }
-            const unsigned lanes = __ballot_sync(kFullMask, in);
-            if (in) use(x, s.val[k], k, lanes);
+            use(x, in ? s.val[k] : 0ull, k, in);
             if (!more) break;
             e = en;
             k = kn;
@@ -102,6 +105,20 @@ __device__ __forceinline__ uint32_t for_entries(ChunkScratch& s, uint32_t cnt, u
         }
     }
     return total;
+}
+
+// Whether w is in u's row or u in w's (a hand-built CSR may hold an edge in one direction only); the
+// shorter row is searched first.
+__device__ __forceinline__ bool adjacent(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ adj,
+                                         uint32_t u, uint32_t w) {
+    const uint32_t ub = __ldg(idx + u), ue = __ldg(idx + u + 1), wb = __ldg(idx + w), we = __ldg(idx + w + 1);
+    for (int k = 0; k < 2; ++k) {
+        const bool in_u = (ue - ub <= we - wb) == (k == 0);
+        const uint32_t e = in_u ? ue : we, v = in_u ? w : u;
+        const uint32_t at = lower_bound_u32(adj, in_u ? ub : wb, e, v);
+        if (at < e && __ldg(adj + at) == v) return true;
+    }
+    return false;
 }
 
 // Adds a 64-bit value to the sum kept as lo[u], hi[u].
@@ -229,7 +246,9 @@ __device__ __forceinline__ void push_frontier(PushScratch& s, const Frontier& f,
         for_entries(
             s.chunk, cnt, q.x, q.y, to_fixed(__uint_as_float(q.z)),
             [&](uint32_t slot, bool in) { return in ? __ldg(adj + slot) : 0u; },
-            [&](uint32_t u, unsigned long long v, uint32_t, unsigned) { add(u, v); });
+            [&](uint32_t u, unsigned long long v, uint32_t, bool in) {
+                if (in) add(u, v);
+            });
     }
     // light vertices: batches of 32 claimed by the warps, the next one loaded while one is pushed
     auto claim = [&]() {

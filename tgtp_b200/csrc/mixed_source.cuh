@@ -63,6 +63,7 @@ struct MixedPack {
 
 struct SourceScratch {
     PushScratch push;
+    unsigned long long st[3], ph[8];
     uint32_t hist[kCandMax];  // digit histogram, or the candidates' residuals
     uint32_t cand_v[kCandMax];
     uint32_t set_v[kSetMax], set_r[kSetMax];  // set_r: first the groups' maxima
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
     SourceScratch& S = *reinterpret_cast<SourceScratch*>(mixed_smem);
     PushScratch& s = S.push;
     const MixedParams& p0 = pk.g[0];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, nw = blockDim.x >> 5;
     const uint32_t sn = p0.scratch_n, pad = (sn + 3u) & ~3u;
     uint32_t* const smem_words = reinterpret_cast<uint32_t*>(mixed_smem + sizeof(SourceScratch));
     uint32_t* const lo = smem_words;        // kShared
@@ -286,14 +287,17 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
         if (lane == 0) s_pre[0] = 0;
     }
     const uint64_t deadline = globaltimer_ns() + p0.budget_ns;
-    unsigned long long st_rounds = 0, st_pv = 0, st_tr = 0, st_we = 0, st_wc = 0, st_wh = 0, st_fb = 0;
+    // run counters: the push's (rounds, vertices, traversals) and the phases' by thread 0 in shared
+    // memory, the walks' per thread
+    if (tid < 3) S.st[tid] = 0;
+    if (tid < 8) S.ph[tid] = 0;
+    unsigned long long st_we = 0, st_wc = 0, st_wh = 0, st_fb = 0;
     // SM cycles per phase as thread 0 sees them, counted once per warp of the block
-    long long ph[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     long long tmark = clock64();
     auto lap = [&](int i) {
         if (tid == 0) {
             const long long now = clock64();
-            ph[i] += (now - tmark) * nw;
+            S.ph[i] += (unsigned long long)(now - tmark) * nw;
             tmark = now;
         }
     };
@@ -309,15 +313,14 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
             stat_add(stats, kStFallback, st_fb);
         }
         if (tid == 0) {
-            stat_add(stats, kStPushRounds, st_rounds);
-            stat_add(stats, kStPushVertices, st_pv);
-            stat_add(stats, kStPushTraversals, st_tr);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) stat_add(stats, kStPhase0 + i, (unsigned long long)ph[i]);
+            stat_add(stats, kStPushRounds, S.st[0]);
+            stat_add(stats, kStPushVertices, S.st[1]);
+            stat_add(stats, kStPushTraversals, S.st[2]);
+            for (int i = 0; i < 8; ++i) stat_add(stats, kStPhase0 + i, S.ph[i]);
+            for (int i = 0; i < 3; ++i) S.st[i] = 0;
+            for (int i = 0; i < 8; ++i) S.ph[i] = 0;
         }
-        st_rounds = st_pv = st_tr = st_we = st_wc = st_wh = st_fb = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) ph[i] = 0;
+        st_we = st_wc = st_wh = st_fb = 0;
     };
     uint32_t last_gi = 0xffffffffu;
     bool dirty = false;
@@ -384,8 +387,8 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
                 else sums[u] = __float_as_uint(r);
             });
             if (tid == 0) {
-                st_pv += 1;
-                st_tr += dsi;
+                S.st[1] += 1;
+                S.st[2] += dsi;
             }
             lap(1);
             while (true) {
@@ -401,8 +404,8 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
                 timed_out = s.late != 0 && !stop;
                 if (stop || timed_out) break;
                 if (tid == 0) {
-                    st_pv += qs;
-                    st_tr += s.picost;
+                    S.st[1] += qs;
+                    S.st[2] += s.picost;
                 }
                 // the old residuals leave the vector before the round's sums start
                 if (MODE == kShared && qs * 4u > n) {
@@ -486,7 +489,7 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
                 dirty = true;
                 break;
             }
-            if (tid == 0) st_rounds += uint64_t(ell);
+            if (tid == 0) S.st[0] += uint64_t(ell);
         }
         if (p.trace_ell && tid == 0) p.trace_ell[src] = uint32_t(ell);
 
@@ -563,16 +566,7 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
                     for (uint32_t q = tid; q < c * c; q += blockDim.x) {
                         const uint32_t i = q / c, j = q % c;
                         if (i >= j) continue;
-                        uint32_t u = S.set_v[i], w = S.set_v[j];
-                        uint32_t ub = __ldg(idx + u), ue = __ldg(idx + u + 1);
-                        const uint32_t wb = __ldg(idx + w), we = __ldg(idx + w + 1);
-                        if (we - wb < ue - ub) {  // look in the shorter row
-                            ub = wb;
-                            ue = we;
-                            w = u;
-                        }
-                        const uint32_t at = lower_bound_u32(adj, ub, ue, w);
-                        if (at < ue && __ldg(adj + at) == w)
+                        if (adjacent(idx, adj, S.set_v[i], S.set_v[j]))
                             best = max(best, __float_as_uint(__fadd_rn(__uint_as_float(S.set_r[i]),
                                                                        __uint_as_float(S.set_r[j]))));
                     }
@@ -608,8 +602,8 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
                             for_entries(
                                 s.chunk, cnt, beg, deg, r,
                                 [&](uint32_t slot, bool in) { return in ? __ldg(adj + slot) : 0u; },
-                                [&](uint32_t w, unsigned long long m, uint32_t, unsigned) {
-                                    const float y = pv(w);
+                                [&](uint32_t w, unsigned long long m, uint32_t, bool in) {
+                                    const float y = in ? pv(w) : 0.f;
                                     if (__float_as_uint(y) > t)
                                         best = max(best, __float_as_uint(__fadd_rn(
                                                              __uint_as_float(uint32_t(m)), y)));
@@ -645,15 +639,16 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
                 for_entries(
                     s.chunk, cnt, beg, deg, static_cast<unsigned long long>(__float_as_uint(FLT_MAX)) << 32,
                     [&](uint32_t slot, bool in) { return in ? __float_as_uint(pv(__ldg(adj + slot))) : 0u; },
-                    [&](uint32_t x, unsigned long long, uint32_t k, unsigned act) {
-                        const uint32_t k0 = __shfl_sync(act, k, 0);  // lane 0 always has an entry
-                        if (__all_sync(act, k == k0)) {  // one row: reduced across the warp
-                            const uint32_t mx = __reduce_max_sync(act, x), mn = __reduce_min_sync(act, x);
+                    [&](uint32_t x, unsigned long long, uint32_t k, bool in) {
+                        const uint32_t k0 = __shfl_sync(kFullMask, k, 0);  // lane 0 always has an entry
+                        if (__all_sync(kFullMask, !in || k == k0)) {  // one row: reduced across the warp
+                            const uint32_t mx = __reduce_max_sync(kFullMask, x);
+                            const uint32_t mn = __reduce_min_sync(kFullMask, in ? x : 0xffffffffu);
                             if (lane == 0) {
                                 atomicMax(ext + 2 * k, mx);
                                 atomicMin(ext + 2 * k + 1, mn);
                             }
-                        } else {
+                        } else if (in) {
                             atomicMax(ext + 2 * k, x);
                             atomicMin(ext + 2 * k + 1, x);
                         }
