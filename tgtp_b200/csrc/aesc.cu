@@ -3,7 +3,7 @@
 // Stages (all on the graph's stream, consecutive kernels joined by programmatic dependent launch):
 //   1. tau per undirected edge (u <= v): the omega-eigenvector walk-length bound (calculate_taus,
 //      :164-216), written to both CSR slots; rows with a slot of tau > 1 are listed.
-//        FP32 form           tau_kernel<float>: the reference's sequential sums, lane per edge.
+//        FP32 form           tau_kernel: the reference's sequential sums, lane per edge.
 //        FP64 / mixed forms  tau_sums_kernel (eight lanes per edge gather the rows) then
 //                            tau_bound_kernel (lane per edge evaluates the bound).
 //   2. the listed sources: push rounds until the push/walk cost test stops them (:456-503), the
@@ -51,7 +51,8 @@
 namespace tgtp {
 namespace {
 
-constexpr int kTauThreads = 32;
+constexpr int kTauThreads = 32;      // FP32 form's tau: one warp per block
+constexpr int kTauBlocks = 20;       // per SM: 96 registers (16 blocks: 78 us for 70; 24 spill: 70)
 // per-warp shared scratch of the chi step: 64 u64 max/min images + 33 + 32 u32 slot offsets
 constexpr size_t kAccBytes = 1280;
 constexpr int kTauTableRows = 64;    // rows of the eigen_t_1 power table (api.cu)
@@ -148,15 +149,14 @@ __device__ int get_tau(uint32_t p1, uint32_t p2, Real epsilon, double one_m_lam2
     return tau % 2 == 0 ? int(tau + 1) : int(tau);
 }
 
-// eigen_t_1[i] cast to the form's real type after k multiplications by lambda_i^2.
-template <class Real>
-__device__ __forceinline__ Real etab_value(const Real* tab, const double* tabd, uint32_t stride,
-                                           uint32_t k, uint32_t i) {
+// eigen_t_1[i] cast to float after k multiplications by lambda_i^2.
+__device__ __forceinline__ float etab_value(const float* tab, const double* tabd, uint32_t stride,
+                                            uint32_t k, uint32_t i) {
     if (k < uint32_t(kTauTableRows)) return __ldg(tab + size_t(k) * stride + i);
     double e = __ldg(tabd + size_t(kTauTableRows - 1) * stride + i);
     const double sq = __ldg(tabd + i);
     for (uint32_t r = kTauTableRows - 1; r < k; ++r) e = __dmul_rn(e, sq);
-    return from_f64<Real>(e);
+    return from_f64<float>(e);
 }
 
 // Rows whose every tau is at most 1 stop after their first push round: with ell = 1 every slot has
@@ -177,175 +177,191 @@ __device__ __forceinline__ void mark_row(const RowMarks& rm, uint32_t r) {
 }
 
 // ---- stage 1: tau per undirected edge ------------------------------------------------------------
-// A warp takes 32 forward slots (one lane each) and sweeps the eigen index i in chunks of 32.  For
-// each chunk the 32 edges' x_u and x_v pieces are copied into shared memory with asynchronous
-// copies (every copy of the chunk in flight at once, coalesced 128/256-byte rows), double buffered
-// so the next chunk streams in while the lanes consume the current one from odd-stride tiles
-// (conflict-free).  Each lane keeps its edge's sums in index order, exactly as the reference does:
-// the first sweep carries upsilon and the first delta term together (two independent chains), any
-// further delta iteration takes one more sweep.
-__device__ __forceinline__ void cp_async_elem(void* smem_dst, const void* gsrc, int bytes) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-    if (bytes == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gsrc) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// x / y for a positive divisor known in advance, correctly rounded (round to nearest even), with
-// Markstein's method (P. Markstein, IBM J. Res. Dev. 34(1), 1990): q0 = x * r with r = RN(1/y) and
-// one correction q1 = q0 + r * (x - q0 y), remainders exact by FMA.  The result is then checked:
-// with rho = x - q1 y exact, q1 = RN(x / y) when |rho| < y * (half the gap from q1 to its
-// neighbour on x / y's side): half an ulp of q1, a quarter ulp below a power of two.  Whenever the
-// check cannot prove it (x zero or negative, q1 out of the safe exponent range, a divisor the host
-// marked with r = NaN), the quotient comes from the correctly rounded division instead.
-__device__ __forceinline__ double div_fixed(double x, double y, double r) {
+// The FP32 form keeps the reference's sums: upsilon and the first delta term of an edge, each a chain
+// of dependent additions over the eigen index in order, and a delta per further sweep.  A warp takes
+// 16 forward slots.  The terms do not depend on one another, so all 32 lanes form them, one edge and
+// 32 consecutive indices at a time (coalesced row pieces, a lane's constants loaded once per 32
+// indices), and leave them in shared memory; then each lane adds up one chain, lanes 0 .. 15 the
+// edges' upsilon and lanes 16 .. 31 their delta.
+//
+// What bounds it: issue slots at many warps per SM, else the chains (an addition and two conversions
+// an index) and the divisions' latency, which is why four edges' terms are formed side by side and the
+// next pieces fetched before they are used.  One edge per lane, terms and sums (a sweep costs a warp
+// the same however few of its edges want it), took on the 88,234-edge graph 70 us at eps = 0.05 (one
+// sweep) and 133 us at 0.01 (1.15 sweeps an edge, two or more in most warps); this takes 49 and 70.
+// x / y for a divisor known in advance, 1e-150 < y <= 2^32, correctly rounded (round to nearest
+// even), with Markstein's method (P. Markstein, IBM J. Res. Dev. 34(1), 1990): from r = RN(1/y), q0 =
+// x * r is within 1.5 ulp, one correction q1 = q0 + r * (x - q0 y) within an ulp (remainders are exact
+// by FMA), and his theorem says that a correction of such a quotient by a correctly rounded
+// reciprocal is RN(x / y).  Nothing under- or overflows while 2^-913 <= x < 2^513 (known_range); any
+// other x (zero and negative ones too) takes the correctly rounded division.  With a check of
+// q1's remainder against half an ulp in place of the second correction a call on the 4,039-vertex
+// graph (FP64, eps = 0.005) took 0.98 ms, so 0.87.
+__device__ __forceinline__ double div_known(double x, double y, double r) {
     const double q0 = __dmul_rn(x, r);
     const double q1 = __fma_rn(__fma_rn(-q0, y, x), r, q0);
-    const double rho = __fma_rn(-q1, y, x);
-    const unsigned hi = unsigned(__double2hiint(q1));
-    const unsigned e = hi >> 20;  // sign bit clear for positive q1
-    double half = __hiloint2double(int((e - 53u) << 20), 0);
-    if (((hi & 0xfffffu) | unsigned(__double2loint(q1))) == 0u && rho < 0.0) half *= 0.5;
-    const bool ok = (e - 65u) < (0x600u - 65u) && fabs(rho) < __dmul_rn(y, half);
-    return ok ? q1 : __ddiv_rn(x, y);
+    return __fma_rn(__fma_rn(-q1, y, x), r, q1);
+}
+__device__ __forceinline__ bool known_range(double x) {
+    return (unsigned(__double2hiint(x)) >> 20) - 110u < 0x600u - 110u;  // the sign bit counts as large
+}
+__device__ __forceinline__ double div_fixed(double x, double y, double r) {
+    return known_range(x) ? div_known(x, y, r) : __ddiv_rn(x, y);
 }
 
-template <class Real>
-__global__ void __launch_bounds__(kTauThreads)
+constexpr uint32_t kTauEdges = 16;  // forward slots per warp: two chains each
+
+__global__ void __launch_bounds__(kTauThreads, kTauBlocks)
 tau_kernel(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ adj,
            const uint32_t* __restrict__ row_of, const uint32_t* __restrict__ rev,
            const uint32_t* __restrict__ forward, uint64_t num_forward,
-           const Real* __restrict__ vec, uint32_t stride, uint32_t omega,
-           const double* __restrict__ onep_g, const double* __restrict__ onem_g,
-           const Real* __restrict__ etab, const double* __restrict__ etabd, Real epsilon,
+           const float* __restrict__ vec, uint32_t stride, uint32_t omega,
+           const double* __restrict__ onep, const double* __restrict__ onem,
+           const float* __restrict__ etab, const double* __restrict__ etabd, float epsilon,
            uint64_t m, TauConst c, int* __restrict__ taus, RowMarks rm,
            unsigned long long* __restrict__ stats) {
-    constexpr uint32_t CH = 128 / sizeof(Real);  // chunk: one 128-byte row piece
-    constexpr uint32_t LD = CH + 1;              // odd tile stride: conflict-free own-row reads
-    extern __shared__ __align__(16) unsigned char tsm[];
+    __shared__ double terms[2][kTauEdges][33];  // upsilon's and delta's, of 32 indices
     pdl_launch_dependents();
-    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint32_t wpb = blockDim.x >> 5;
-    // per index: (1 + lambda_i, 1 - lambda_i) and (RN(1 / (1 - lambda_i)), eigen_t_1 row 0)
-    double2* cA = reinterpret_cast<double2*>(tsm);
-    double2* cB = cA + omega;
-    Real* tiles = reinterpret_cast<Real*>(cB + omega) + size_t(wib) * 4 * 32 * LD;  // [2][U,V][32][LD]
-    for (uint32_t i = threadIdx.x; i < omega; i += blockDim.x) {
-        const double y = onem_g[i];
-        const double r = (y > 1e-150 && y < 8.0) ? __drcp_rn(y) : __longlong_as_double(0x7ff8000000000000ull);
-        cA[i] = make_double2(onep_g[i], y);
-        cB[i] = make_double2(r, double(etab[i]));
-    }
-    __syncthreads();
+    const uint32_t lane = threadIdx.x;
+    const uint32_t half = lane / kTauEdges, mine = lane % kTauEdges;
+    const float mreal = from_u64<float>(m);
     unsigned long long iters = 0, ambiguous = 0;
-    const Real mreal = from_u64<Real>(m);
-    const uint64_t nw = uint64_t(gridDim.x) * wpb;
-    const uint32_t nchunks = (omega + CH - 1) / CH;
-    // lanes stage CH consecutive indices of 32 / CH edges per step
-    constexpr uint32_t EPS = 32 / CH;  // edges per staging step (1 for float, 2 for double)
-    const uint32_t sub = lane / CH, col = lane % CH;
-    for (uint64_t base = (uint64_t(blockIdx.x) * wpb + wib) * 32; base < num_forward; base += nw * 32) {
-        const uint64_t e = base + lane;
-        const bool act = e < num_forward;
-        uint32_t pos = 0, u = 0, v = 0, du = 0, dv = 0;
-        if (act) {
+    for (uint64_t base = uint64_t(blockIdx.x) * kTauEdges; base < num_forward; base += uint64_t(gridDim.x) * kTauEdges) {
+        // both halves of the warp hold the edges' state
+        const uint64_t e = base + mine;
+        uint32_t pos = 0, u = 0, v = 0, du = 1, dv = 1;
+        bool done = e >= num_forward;
+        if (!done) {
             pos = __ldg(forward + e);
             u = __ldg(row_of + pos);
             v = __ldg(adj + pos);
             du = __ldg(idx + u + 1) - __ldg(idx + u);
             dv = __ldg(idx + v + 1) - __ldg(idx + v);
         }
-        const uint32_t cnt = uint32_t(min(uint64_t(32), num_forward - base));
-        auto stage = [&](uint32_t chunk, uint32_t buf) {
-            Real* U = tiles + size_t(buf) * 2 * 32 * LD;
-            Real* V = U + 32 * LD;
-            const uint32_t i = chunk * CH + col;
-            for (uint32_t t0 = 0; t0 < cnt; t0 += EPS) {
-                const uint32_t t = t0 + sub;
-                const uint32_t ut = __shfl_sync(kFullMask, u, t & 31u);
-                const uint32_t vt = __shfl_sync(kFullMask, v, t & 31u);
-                if (t < cnt && i < omega) {
-                    cp_async_elem(U + t * LD + col, vec + size_t(ut) * stride + i, int(sizeof(Real)));
-                    cp_async_elem(V + t * LD + col, vec + size_t(vt) * stride + i, int(sizeof(Real)));
-                }
-            }
-            cp_async_commit();
-        };
-        Real ups = 0, del = 0;
+        float ups = 0.0f;
         int tau = 0, t = 1;
-        bool done = !act;
-        for (uint32_t k = 0; __any_sync(kFullMask, !done); ++k) {
-            del = Real(0);
-            stage(0, 0);
-            for (uint32_t ch = 0; ch < nchunks; ++ch) {
-                if (ch + 1 < nchunks) {
-                    stage(ch + 1, (ch + 1) & 1);
-                    cp_async_wait<1>();
+        for (uint32_t k = 0;; ++k) {
+            const unsigned left = __ballot_sync(kFullMask, !done) & ((1u << kTauEdges) - 1u);
+            if (!left) break;
+            // get_upsilon (:151-162) with get_delta (:137-150) at eigen_t_1 = lambda^2, or get_delta
+            // alone at lambda^(2(k+1)); indices 1 .. omega - 2
+            float acc = 0.0f;
+            const bool full = left == (1u << kTauEdges) - 1u;
+            auto inside = [&](uint32_t i) { return i > 0 && i < omega - 1; };
+            // one edge's row elements; a place that loads nothing divides 1
+            auto piece = [&](int slot, uint32_t i, float& xu, float& xv) {
+                const uint32_t uq = __shfl_sync(kFullMask, u, slot), vq = __shfl_sync(kFullMask, v, slot);
+                xu = inside(i) ? __ldg(vec + size_t(uq) * stride + i) : 1.0f;
+                xv = inside(i) ? __ldg(vec + size_t(vq) * stride + i) : 0.0f;
+            };
+            // the next indices' constants and first pieces are fetched before the sums of these
+            struct {
+                float et;
+                double w, y;
+            } next;
+            auto constants = [&](uint32_t i) {
+                next.et = inside(i) ? etab_value(etab, etabd, stride, k, i) : 1.0f;
+                next.w = inside(i) ? __ldg(onep + i) : 1.0;
+                next.y = inside(i) ? __ldg(onem + i) : 1.0;
+            };
+            float nu[4], nv[4];
+            constants(lane);
+            if (full) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) piece(q, lane, nu[q], nv[q]);
+            }
+            for (uint32_t i0 = 0; i0 < omega - 1; i0 += 32) {
+                const uint32_t i = i0 + lane;
+                const float et = next.et;
+                const double w = next.w, y = next.y;
+                const bool known = y > 1e-150 && y < 8.0;
+                const double r = __drcp_rn(y);
+                // the terms of four edges from their row pieces
+                auto form = [&](const float (&xu)[4], const float (&xv)[4], const int (&slot)[4]) {
+                    float d2[4];
+                    double x[4], z[4];
+                    bool ok = known;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float d = rsub(xu[q], xv[q]);
+                        d2[q] = rmul(d, d);
+                        x[q] = double(rmul(d2[q], et));
+                        ok = ok && known_range(x[q]);
+                        z[q] = div_known(x[q], y, r);
+                    }
+                    if (!ok) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) z[q] = __ddiv_rn(x[q], y);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (slot[q] >= 0) {
+                            if (k == 0) terms[0][slot[q]][lane] = __dmul_rn(double(d2[q]), w);
+                            terms[1][slot[q]][lane] = z[q];
+                        }
+                };
+                if (full) {
+#pragma unroll
+                    for (int g = 0; g < int(kTauEdges); g += 4) {
+                        float xu[4], xv[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            xu[q] = nu[q];
+                            xv[q] = nv[q];
+                            if (g + 4 < int(kTauEdges)) piece(g + 4 + q, i, nu[q], nv[q]);
+                            else piece(q, i + 32, nu[q], nv[q]);
+                        }
+                        if (g + 4 == int(kTauEdges)) constants(i + 32);
+                        const int slot[4] = {g, g + 1, g + 2, g + 3};
+                        form(xu, xv, slot);
+                    }
                 } else {
-                    cp_async_wait<0>();
+                    constants(i + 32);
+                    for (unsigned rest = left; rest;) {
+                        float xu[4], xv[4];
+                        int slot[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            slot[q] = __ffs(int(rest)) - 1;
+                            rest &= rest - 1;
+                            xu[q] = 1.0f;
+                            xv[q] = 0.0f;
+                            if (slot[q] >= 0) piece(slot[q], i, xu[q], xv[q]);
+                        }
+                        form(xu, xv, slot);
+                    }
                 }
                 __syncwarp();
-                if (!done) {
-                    const Real* U = tiles + size_t(ch & 1) * 2 * 32 * LD + lane * LD;
-                    const Real* V = U + 32 * LD;
-                    const uint32_t i0 = ch * CH;
-                    const uint32_t lo = i0 == 0 ? 1u : 0u;
-                    const uint32_t hi = min(CH, omega - 1 - i0);  // indices i < omega - 1
-                    // get_upsilon (:151-162) with get_delta (:137-150) at eigen_t_1 = lambda^2,
-                    // or get_delta alone at lambda^(2(k+1))
-                    auto term0 = [&](uint32_t j) {
-                        const uint32_t i = i0 + j;
-                        const Real d = rsub(U[j], V[j]);
-                        const Real d2 = rmul(d, d);
-                        const double2 a = cA[i], b = cB[i];
-                        ups = from_f64<Real>(__dadd_rn(double(ups), __dmul_rn(double(d2), a.x)));
-                        del = from_f64<Real>(__dadd_rn(
-                            double(del), div_fixed(double(rmul(d2, Real(b.y))), a.y, b.x)));
-                    };
-                    auto termk = [&](uint32_t j) {
-                        const uint32_t i = i0 + j;
-                        const Real d = rsub(U[j], V[j]);
-                        const Real et = etab_value<Real>(etab, etabd, stride, k, i);
-                        const double2 a = cA[i], b = cB[i];
-                        del = from_f64<Real>(__dadd_rn(
-                            double(del), div_fixed(double(rmul(rmul(d, d), et)), a.y, b.x)));
-                    };
-                    if (k == 0) {
-                        if (lo == 0 && hi == CH) {
-#pragma unroll
-                            for (uint32_t j = 0; j < CH; ++j) term0(j);
-                        } else {
-                            for (uint32_t j = lo; j < hi; ++j) term0(j);
-                        }
+                if (!done && (half || k == 0)) {
+                    const double* const mt = terms[half][mine];
+                    const uint32_t lo = i0 == 0 ? 1u : 0u, hi = min(32u, omega - 1 - i0);
+                    if (lo == 0 && hi == 32) {
+#pragma unroll 8
+                        for (uint32_t j = 0; j < 32; ++j) acc = from_f64<float>(__dadd_rn(double(acc), mt[j]));
                     } else {
-                        for (uint32_t j = lo; j < hi; ++j) termk(j);
+                        for (uint32_t j = lo; j < hi; ++j) acc = from_f64<float>(__dadd_rn(double(acc), mt[j]));
                     }
                 }
                 __syncwarp();
             }
+            acc = rdiv(acc, mreal);
+            if (k == 0) ups = __shfl_sync(kFullMask, acc, int(mine));
+            // lanes 16 .. 31: the bound of this delta; lanes 0 .. 15, first sweep: tau from lambda_1
+            int bound = 0;
+            if (!done && (half || k == 0))
+                bound = get_tau<float>(du, dv, epsilon, half ? c.one_m_l2sq : c.one_m_l1sq, half ? c.b2 : c.b1,
+                                       half ? acc : 0.0f, half ? ups : 0.0f, ambiguous);
+            if (k == 0) tau = __shfl_sync(kFullMask, bound, int(mine));
+            const int tp = __shfl_sync(kFullMask, bound, int(mine + kTauEdges));
             if (!done) {
-                if (k == 0) {
-                    ups = rdiv(ups, mreal);
-                    tau = get_tau<Real>(du, dv, epsilon, c.one_m_l1sq, c.b1, Real(0), Real(0), ambiguous);
-                }
-                del = rdiv(del, mreal);
-                ++iters;
-                const int tp = get_tau<Real>(du, dv, epsilon, c.one_m_l2sq, c.b2, del, ups, ambiguous);
+                iters += half;
                 if (t <= tp && tp < tau) {
                     tau = tp;
                     t += 2;
                 } else {
                     done = true;
-                    taus[pos] = tau;
-                    taus[__ldg(rev + pos)] = tau;
-                    if (tau > 1) {
-                        mark_row(rm, u);
-                        mark_row(rm, v);
-                    }
+                    taus[half ? __ldg(rev + pos) : pos] = tau;
+                    if (tau > 1) mark_row(rm, half ? v : u);
                 }
             }
         }
@@ -2593,20 +2609,13 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
         const Real* vec = (const Real*)g->vec_f32.ptr;
         const Real* etab = (const Real*)g->etab_f.ptr;
         const Real eps_half = Real(cfg.epsilon / 2.0);
-        // per block: two double2 constants per index; per warp: two buffers of (x_u, x_v) chunks
-        // of 32 edges x one 128-byte row piece, rows padded by one element
-        const size_t tau_smem = 2 * sizeof(double2) * omega +
-                                size_t(kTauThreads / 32) * 4 * 32 * (128 / sizeof(Real) + 1) * sizeof(Real);
-        if (tau_smem > size_t(227) * 1024)
+        // the largest omega taken: 32 bytes per index beside 16.5 KB
+        if (32 * size_t(omega) + 4 * 32 * 33 * sizeof(Real) > size_t(227) * 1024)
             fail(TGTP_ERR_UNSUPPORTED, "omega too large for the tau kernel tile");
-        const int tau_per_sm =
-            blocks_per_sm(reinterpret_cast<const void*>(tau_kernel<Real>), kTauThreads, tau_smem);
-        if (tau_per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "omega too large for the tau kernel tile");
-        const uint64_t groups = (g->num_forward + 31) / 32;
-        const uint64_t tau_blocks = std::max<uint64_t>(1, std::min<uint64_t>(
-            (groups + kTauThreads / 32 - 1) / (kTauThreads / 32), uint64_t(g->num_sms) * tau_per_sm));
+        const unsigned tau_blocks = unsigned(std::max<uint64_t>(
+            1, std::min<uint64_t>((g->num_forward + kTauEdges - 1) / kTauEdges, uint64_t(1) << 30)));
         ScopedKernel k(g->prof, s, "tau");
-        tau_kernel<Real><<<unsigned(tau_blocks), kTauThreads, tau_smem, s>>>(
+        tau_kernel<<<tau_blocks, kTauThreads, 0, s>>>(
             g->idx.as<uint32_t>(), g->adj.as<uint32_t>(), g->row_of.as<uint32_t>(),
             g->rev.as<uint32_t>(), g->forward.as<uint32_t>(), g->num_forward, vec, g->omega, omega,
             g->onep.as<double>(), g->onem.as<double>(), etab, g->etab.as<double>(), eps_half, m, c,

@@ -11,8 +11,8 @@
 // applied; r / deg(u) is formed from the vertex's reciprocal (div_fixed).
 //
 // Against one warp per source, half as many sources in flight and a flag array beside the residuals
-// (per call): FP64, n = 4,039, 44 neighbours, eps = 0.005, 1.55 -> 1.0 ms; FP32 there, eps = 0.01, 0.62
-// -> 0.42 ms; FP64, n = 25,860, 9 neighbours, eps = 0.05 (HBM tier), 290 -> 145 ms.  A step still waits
+// (per call): FP64, n = 4,039, 44 neighbours, eps = 0.005, 1.55 -> 0.87 ms; FP32 there, eps = 0.01, 0.62
+// -> 0.36 ms; FP64, n = 25,860, 9 neighbours, eps = 0.05 (HBM tier), 290 -> 145 ms.  A step still waits
 // on a shared-memory or L2 round trip: 0.14 (shared memory) and 0.22 (HBM) instructions per cycle and
 // scheduler, no unit above 26 % of its rate.
 
