@@ -209,6 +209,7 @@ __device__ __forceinline__ double div_fixed(double x, double y, double r) {
     return known_range(x) ? div_known(x, y, r) : __ddiv_rn(x, y);
 }
 
+constexpr int kSumsEdges = 2, kSumsThreads = 256, kSumsBlocks = 4, kSumsUnroll = 4;  // tau_sums_kernel
 constexpr uint32_t kTauEdges = 16;  // forward slots per warp: two chains each
 
 __global__ void __launch_bounds__(kTauThreads, kTauBlocks)
@@ -607,17 +608,57 @@ __device__ __forceinline__ void split_pass(const Vec* __restrict__ ur, const Vec
     }
 }
 
+// Both sums of N edges at a time by one 8-lane group: the weights are read once for all of them, and
+// one u row where the edges share it (SAME).
+template <class Vec, int N, bool SAME>
+__device__ __forceinline__ void split_pass_n(const Vec* const (&ur)[SAME ? 1 : N], const Vec* const (&vr)[N],
+                                             uint32_t omega, bool vec_ok, uint32_t sl,
+                                             const typename Split<Vec>::Part* wa,
+                                             const typename Split<Vec>::Part* wb,
+                                             typename Split<Vec>::Part (&sa)[N],
+                                             typename Split<Vec>::Part (&sb)[N]) {
+    using Part = typename Split<Vec>::Part;
+    constexpr uint32_t P = Split<Vec>::P, C = 8 * P;
+#pragma unroll kSumsUnroll
+    for (uint32_t i0 = sl * P; i0 < omega; i0 += C) {
+        Part xu[SAME ? 1 : N][P], xv[N][P];
+#pragma unroll
+        for (int q = 0; q < (SAME ? 1 : N); ++q) load_piece(ur[q], i0, omega, vec_ok, xu[q]);
+#pragma unroll
+        for (int q = 0; q < N; ++q) load_piece(vr[q], i0, omega, vec_ok, xv[q]);
+#pragma unroll
+        for (uint32_t j = 0; j < P; ++j) {
+            const Part a = wa[i0 + j], b = wb[i0 + j];
+#pragma unroll
+            for (int q = 0; q < N; ++q) {
+                const Part d = split_sub(xu[SAME ? 0 : q][j], xv[q][j]);
+                sa[q] = split_fma(d, a, sa[q]);
+                sb[q] = split_fma(d, b, sb[q]);
+            }
+        }
+    }
+}
+
 // Stage 1a: the first sweep of every forward edge (upsilon and delta_0 sums), a pure gather.  A
-// warp takes eight edges at a time, two per group; the edge records of the next step are fetched
-// one step ahead.
+// group takes two consecutive edges at a time (slots are in row order, so they mostly share their u);
+// the next ones' vertices are fetched one step ahead.
+//
+// What bounds it: the rows come from L2, half of them from L1, and half of the L1's cycles went to
+// the weights, read from shared memory for every edge.  Two edges per read and one u row for both took
+// (with the launch) 21 -> 17 us on 88,234 edges in FP64, 249 -> 177 us on 2,000,000 in F32 rows.  Four edges
+// a group need 80 registers, so 24 warps an SM: 20 us, 182 us; five blocks an SM spill: 18 us.
 template <class Vec>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(kSumsThreads, kSumsBlocks)
 tau_sums_kernel(const uint4* __restrict__ fedge, uint64_t num_forward, const Vec* __restrict__ vec,
                 uint32_t stride, uint32_t omega, const typename Split<Vec>::Part* __restrict__ wtab,
-                uint32_t wpad, double2* __restrict__ sums) {
+                uint32_t wpad, double2* __restrict__ sums, uint32_t* __restrict__ zero, uint64_t zero_words) {
     using Part = typename Split<Vec>::Part;
+    constexpr int N = kSumsEdges;
     extern __shared__ __align__(16) unsigned char ssm[];
     pdl_launch_dependents();
+    // the run's counters, work words and row marks, which the later kernels use
+    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < zero_words; i += uint64_t(gridDim.x) * blockDim.x)
+        zero[i] = 0u;
     Part* wu = reinterpret_cast<Part*>(ssm);  // upsilon weights, then delta_0 weights
     Part* wd = wu + wpad;
     for (uint32_t i = threadIdx.x; i < 2 * wpad; i += blockDim.x) wu[i] = __ldg(wtab + i);
@@ -626,25 +667,50 @@ tau_sums_kernel(const uint4* __restrict__ fedge, uint64_t num_forward, const Vec
     const uint64_t gw = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nw = (uint64_t(gridDim.x) * blockDim.x) >> 5;
     const bool vec_ok = stride % Split<Vec>::P == 0;
-    uint4 n0 = make_uint4(0, 0, 0, 0), n1 = n0;
-    if (gw * 8 + grp < num_forward) n0 = __ldg(fedge + gw * 8 + grp);
-    if (gw * 8 + 4 + grp < num_forward) n1 = __ldg(fedge + gw * 8 + 4 + grp);
-    for (uint64_t base = gw * 8; base < num_forward; base += nw * 8) {
-        const uint64_t e0 = base + grp, e1 = e0 + 4;
-        const uint4 r0 = n0, r1 = n1;
-        if (e0 + nw * 8 < num_forward) n0 = __ldg(fedge + e0 + nw * 8);
-        if (e1 + nw * 8 < num_forward) n1 = __ldg(fedge + e1 + nw * 8);
-        Part su0 = Part(0), sd0 = Part(0), su1 = Part(0), sd1 = Part(0);
-        if (e0 < num_forward)
-            split_pass<Vec, 2>(vec + size_t(r0.x) * stride, vec + size_t(r0.y) * stride, omega,
-                               vec_ok, sl, wu, wd, su0, sd0);
-        if (e1 < num_forward)
-            split_pass<Vec, 2>(vec + size_t(r1.x) * stride, vec + size_t(r1.y) * stride, omega,
-                               vec_ok, sl, wu, wd, su1, sd1);
-        const double u0 = split_reduce(su0), d0 = split_reduce(sd0);
-        const double u1 = split_reduce(su1), d1 = split_reduce(sd1);
-        if (sl == 0 && e0 < num_forward) sums[e0] = make_double2(u0, d0);
-        if (sl == 0 && e1 < num_forward) sums[e1] = make_double2(u1, d1);
+    // the N edges from e on (past the end: the last edge again)
+    uint2 next[N];
+    auto fetch = [&](uint64_t e) {
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+            next[q] = __ldg(reinterpret_cast<const uint2*>(fedge + min(e + q, num_forward - 1)));
+    };
+    if (gw * 4 * N < num_forward) fetch(gw * 4 * N + grp * N);
+    for (uint64_t base = gw * 4 * N; base < num_forward; base += nw * 4 * N) {
+        const uint64_t e = base + grp * N;
+        const Vec* vr[N];
+        uint32_t u[N];
+        bool one = true;
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            u[q] = next[q].x;
+            vr[q] = vec + size_t(next[q].y) * stride;
+            one = one && u[q] == u[0];
+        }
+        if (base + nw * 4 * N < num_forward) fetch(e + nw * 4 * N);
+        Part su[N], sd[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) su[q] = sd[q] = Part(0);
+        if (__all_sync(kFullMask, one)) {
+            const Vec* const ur[1] = {vec + size_t(u[0]) * stride};
+            split_pass_n<Vec, N, true>(ur, vr, omega, vec_ok, sl, wu, wd, su, sd);
+        } else {
+#pragma unroll
+            for (int h = 0; h < N; h += 2) {
+                const Vec* const ur[2] = {vec + size_t(u[h]) * stride, vec + size_t(u[h + 1]) * stride};
+                const Vec* const v2[2] = {vr[h], vr[h + 1]};
+                Part a[2] = {Part(0), Part(0)}, b[2] = {Part(0), Part(0)};
+                split_pass_n<Vec, 2, false>(ur, v2, omega, vec_ok, sl, wu, wd, a, b);
+                su[h] = a[0];
+                su[h + 1] = a[1];
+                sd[h] = b[0];
+                sd[h + 1] = b[1];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < N; ++q) {
+            const double x = split_reduce(su[q]), y = split_reduce(sd[q]);
+            if (sl == 0 && e + q < num_forward) sums[e + q] = make_double2(x, y);
+        }
     }
 }
 
@@ -938,7 +1004,7 @@ __device__ __forceinline__ void flush_tau_stats(unsigned long long iters, unsign
 template <class Vec>
 __global__ void __launch_bounds__(256)
 tau_bound_kernel(const uint4* __restrict__ fedge, uint64_t num_forward,
-                 const double2* __restrict__ sums, BoundArgs<Vec> A,
+                 const double2* __restrict__ sums, BoundArgs<Vec> A, uint32_t per_warp,
                  unsigned long long* __restrict__ stats) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t gw = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -946,9 +1012,9 @@ tau_bound_kernel(const uint4* __restrict__ fedge, uint64_t num_forward,
     unsigned long long iters = 0, ambiguous = 0;
     pdl_launch_dependents();
     pdl_wait();  // the sums of tau_sums_kernel
-    for (uint64_t base = gw * 32; base < num_forward; base += nw * 32) {
+    for (uint64_t base = gw * per_warp; base < num_forward; base += nw * per_warp) {
         const uint64_t e = base + lane;
-        const bool act = e < num_forward;
+        const bool act = lane < per_warp && e < num_forward;
         uint4 rec = make_uint4(0, 0, 0, 0);
         double2 sm = make_double2(0.0, 0.0);
         if (act) {
@@ -2524,10 +2590,15 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
     grow(g, g->stats, zero_bytes);
     auto* stats = g->stats.as<unsigned long long>();
     auto* work = run_work(g);
-    TGTP_CUDA(cudaMemsetAsync(stats, 0, zero_bytes, s));
+    const bool multi = !MIXED && g->has_multi_edges;
+    const char* bulk_env = std::getenv("TGTP_TAU_BULK");
+    const bool want_bulk = bulk_env && std::atoi(bulk_env) == 1;
+    // tau_sums_kernel, where it runs first, zeroes them on its way (a launch less: 30.5 -> 27 us for
+    // a call on the 4,039-vertex graph, FP64, eps = 0.05)
+    const bool zero_in_sums = (MIXED || std::is_same<Real, double>::value) && !multi && !want_bulk;
+    if (!zero_in_sums) TGTP_CUDA(cudaMemsetAsync(stats, 0, zero_bytes, s));
 
     const RowMarks rm = begin_row_marks(g);
-    const bool multi = !MIXED && g->has_multi_edges;
     if (multi) {
         // the reference leaves tau = 0 in the slots no forward edge writes (the later repeats of
         // a neighbour u < v in row v, src/aesc.h:179-209), and every row goes to the source kernel
@@ -2562,10 +2633,11 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
         ba.rm = rm;
         {
             const int per_sm =
-                blocks_per_sm(reinterpret_cast<const void*>(tau_sums_kernel<Vec>), 256, ssmem);
+                blocks_per_sm(reinterpret_cast<const void*>(tau_sums_kernel<Vec>), kSumsThreads, ssmem);
             if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "omega too large for the tau kernel");
             grow(g, g->tau_sums, sizeof(double2) * (g->num_forward + 1));
-            const uint64_t need = (g->num_forward + 63) / 64;  // 64 edges per block and step
+            constexpr uint64_t kStep = kSumsThreads / 8 * kSumsEdges;  // edges per block and step
+            const uint64_t need = (g->num_forward + kStep - 1) / kStep;
             const unsigned blocks = unsigned(std::max<uint64_t>(
                 1, std::min<uint64_t>(need, uint64_t(g->num_sms) * per_sm)));
             // TGTP_TAU_BULK=1: the bulk-copy pipeline instead of the gather (rows whose bytes are a
@@ -2573,8 +2645,7 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
             // it measured 0.056 ms per FP64 step against the gather's 0.046: the rows are
             // L2-resident, so the gather's 32 warps per SM hide the latency better than six
             // pipelined warps, and the bulk copies fetch each edge's u row again.
-            const char* bulk_env = std::getenv("TGTP_TAU_BULK");
-            const bool bulk = (bulk_env && std::atoi(bulk_env) == 1) &&
+            const bool bulk = want_bulk &&
                               (size_t(omega) * sizeof(Vec)) % 16 == 0 &&
                               (size_t(g->omega) * sizeof(Vec)) % 16 == 0;
             constexpr int WPB = BulkShape<Vec>::WPB;
@@ -2593,15 +2664,22 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
                 TGTP_LAUNCH_CHECK("tau_sums_bulk_kernel");
             } else {
                 ScopedKernel k(g->prof, s, "tau_sums");
-                launch(tau_sums_kernel<Vec>, blocks, 256u, ssmem, s, false,
+                launch(tau_sums_kernel<Vec>, blocks, unsigned(kSumsThreads), ssmem, s, false,
                     g->fedge.as<uint4>(), g->num_forward, vec, g->omega, omega, wtab, wpad,
-                    g->tau_sums.as<double2>());
+                    g->tau_sums.as<double2>(), reinterpret_cast<uint32_t*>(stats),
+                    zero_in_sums ? uint64_t(zero_bytes / sizeof(uint32_t)) : uint64_t(0));
                 TGTP_LAUNCH_CHECK("tau_sums_kernel");
             }
             ScopedKernel k(g->prof, s, "tau_bound");
-            launch(tau_bound_kernel<Vec>, grid_cap(g->num_forward, 256, g->num_sms, 8), 256u,
+            // Edges per warp: a further delta sweep serves four of a warp's edges at a time, one round
+            // after another, so graphs with few edges spread them over more warps (12,000 edges, most
+            // with a second sweep: 32 a warp 29 us, 16 19, 8 16, 4 15; 29,700: 23, 21, 17, 19; 88,234 with
+            // one sweep: 10.7, 12.7, 16.5, 25; 2,000,000: 88, 123, 184, 299).
+            const uint64_t at_once = uint64_t(g->num_sms) * 32;
+            const uint32_t per_warp = g->num_forward <= 8 * at_once ? 8u : g->num_forward <= 16 * at_once ? 16u : 32u;
+            launch(tau_bound_kernel<Vec>, grid_cap(g->num_forward * (32 / per_warp), 256, g->num_sms, 8), 256u,
                    size_t(0), s, true, g->fedge.as<uint4>(), g->num_forward,
-                   static_cast<const double2*>(g->tau_sums.as<double2>()), ba, stats);
+                   static_cast<const double2*>(g->tau_sums.as<double2>()), ba, per_warp, stats);
             TGTP_LAUNCH_CHECK("tau_bound_kernel");
         }
     } else {
