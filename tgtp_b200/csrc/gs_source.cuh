@@ -521,12 +521,14 @@ struct SourcePack {
 constexpr int kBatchPack = 64;  // graphs per persistent batch launch
 
 // Threads per block and the blocks per SM its registers are limited for: in shared memory four warps
-// share the stages after the push (two where many small vectors fit, see gs_layout); in HBM, where the push is nearly all of the time, two, so that
-// more sources are in flight.
+// share the stages after the push (two where many small vectors fit, see gs_layout); in HBM, where
+// the push is nearly all of the time, two, and as many blocks as the vectors' way through L1 and L2
+// stands (FP64, n = 10,000, 10 neighbours: 6, 8, 10, 12, 16 blocks 19.6, 17.3, 16.6, 18.3, 18.6 ms; n = 25,860:
+// 179, 156, 145, 147, 150; FP32 there, 8 .. 20 blocks: 127, 118 (10), 117 (12), 114 (16), 118 (20)).
 template <class Real, bool SMEM>
 struct GsShape {
     static constexpr int kThreads = SMEM ? 128 : 64;
-    static constexpr int kBlocks = SMEM ? (sizeof(Real) == 8 ? 6 : 8) : (sizeof(Real) == 8 ? 12 : 16);
+    static constexpr int kBlocks = SMEM ? (sizeof(Real) == 8 ? 6 : 8) : (sizeof(Real) == 8 ? 10 : 16);
 };
 
 template <class Real, bool SMEM, class Pack>
