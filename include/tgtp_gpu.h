@@ -150,12 +150,12 @@ tgtp_status tgtp_last_run_stats(tgtp_graph* g, tgtp_run_stats* out);
 /* Per-slot tau of the last run (m int32, host). */
 tgtp_status tgtp_last_taus(tgtp_graph* g, int32_t* host_taus);
 
-/* Times the candidate layouts of the source kernel (per-source residual vectors in shared memory
- * or in HBM, warps per block; for the mixed form also the multi-source block push at four
- * push-frontier thresholds) for cfg's precision form on this graph, `trials` runs each after a
+/* Times the candidate layouts of the source kernels (per-source residual vectors in shared memory
+ * or in HBM; for the FP32 and FP64 forms the windowed or the one-vertex push; for the mixed form
+ * also the one-source and the multi-source block push, the latter at four frontier thresholds) for cfg's precision form on this graph, `trials` runs each after a
  * warm-up, and keeps the fastest on the handle for later runs of that form.  Scores are identical
  * under every layout.  *layout (may be NULL) receives the choice: 0x100 bit = shared memory, low
- * byte = warps per block, 0x200 = block push, bits 12-13 = its compaction threshold (a round is
+ * byte = nominal warps per block, 0x200 = block push, bits 12-13 = its compaction threshold (a round is
  * compacted to the rows next to the live ones when their degree sum is below m / 4, m / 2,
  * m / 16, or never); for the FP32 and FP64 forms 0x400 = the windowed sequential push, 0x800 =
  * one frontier vertex at a time.  The reference has no counterpart (its OpenMP loop has one

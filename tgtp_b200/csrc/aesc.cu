@@ -3,13 +3,14 @@
 // Stages (all on the graph's stream, consecutive kernels joined by programmatic dependent launch):
 //   1. tau per undirected edge (u <= v): the omega-eigenvector walk-length bound (calculate_taus,
 //      :164-216), written to both CSR slots; rows with a slot of tau > 1 are listed.
-//        FP32 form           tau_kernel: the reference's sequential sums, lane per edge.
+//        FP32 form           tau_kernel: the reference's sequential sums, two lanes per edge.
 //        FP64 / mixed forms  tau_sums_kernel (eight lanes per edge gather the rows) then
 //                            tau_bound_kernel (lane per edge evaluates the bound).
 //   2. the listed sources: push rounds until the push/walk cost test stops them (:456-503), the
 //      top-gamma edge bound (:414-442), the per-edge chi and walk count (:392-412, :508-521) and
 //      the 2-way bouquet walks (:241-391), accumulating each source's CSR row (:524-525).
-//        source_kernel        FP32 / FP64 forms: persistent warps, one source at a time per warp;
+//        source_kernel        FP32 / FP64 forms: one source at a time per block, pushed by one of
+//                             its warps (gs_source.cuh);
 //        mixed_source_kernel  mixed form: one source at a time per block (mixed_source.cuh);
 //        push_shared_kernel, push_block_kernel  mixed form, deep pushes: the push alone, one source
 //                             per block in shared memory, or 32 sources per CTA as a pull product;
@@ -53,7 +54,7 @@ namespace {
 
 constexpr int kTauThreads = 32;      // FP32 form's tau: one warp per block
 constexpr int kTauBlocks = 20;       // per SM: 96 registers (16 blocks: 78 us for 70; 24 spill: 70)
-// per-warp shared scratch of the chi step: 64 u64 max/min images + 33 + 32 u32 slot offsets
+// scratch counted beside a residual vector where the size rule of the mixed form's pushes is stated
 constexpr size_t kAccBytes = 1280;
 constexpr int kTauTableRows = 64;    // rows of the eigen_t_1 power table (api.cu)
 constexpr uint64_t kMaxWalks = 0xffffffffull;  // nr beyond the 32-bit grid is not supported
