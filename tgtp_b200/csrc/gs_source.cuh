@@ -68,7 +68,9 @@ struct GsScratch {
     uint32_t set_v[kSetMax];
     double rw[4];
     alignas(8) uint32_t filter[kGsFilter];
-    uint32_t k, graph, late, picost, found, nitems, next_item, set_count, cand_count, bin, rest;
+    // late: past the deadline at the claim, round_late: at a round's start.  Two words: a warp may read
+    // the one after thread 0 has written the other, and every warp must leave the loops with the rest.
+    uint32_t k, graph, late, round_late, picost, found, nitems, next_item, set_count, cand_count, bin, rest;
 };
 static_assert(sizeof(unsigned long long) * kGsRows == 4 * kGsFilter, "the chi step keeps its minima in the filter");
 template <class Real>
@@ -734,7 +736,7 @@ source_kernel(const Pack pk) {
             // ---- the push/walk cost test (:483-502) ----
             // The walk counts are whole numbers, so their sum does not depend on the order while it
             // is below 2^53; beyond that it exceeds any push cost either way.
-            if (tid == 0) s.late = globaltimer_ns() > deadline;
+            if (tid == 0) s.round_late = globaltimer_ns() > deadline;
             __syncthreads();
             gmax = from_ord<Real>(s.gmax);
             gmin = qs < n ? Real(0) : from_ord<Real>(s.gmin);
@@ -757,7 +759,7 @@ source_kernel(const Pack pk) {
             rw = 0;
             for (uint32_t w = 0; w < nw; ++w) rw += s.rw[w];
             const bool stop = picost >= __dmul_rn(25.0, rw);
-            timed_out = s.late != 0 && !stop;
+            timed_out = s.round_late != 0 && !stop;
             lap(3);
             if (stop || timed_out) break;
             if (warp == 0) {

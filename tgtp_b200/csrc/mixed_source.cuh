@@ -68,6 +68,7 @@ struct SourceScratch {
     uint32_t cand_v[kCandMax];
     uint32_t set_v[kSetMax], set_r[kSetMax];  // set_r: first the groups' maxima
     uint32_t set_count, cand_count, nth, best, nitems, next_item, smax, smin, bin, rest, graph;
+    uint32_t late;  // past the deadline at the claim (push.late: at a round's start; see GsScratch)
 };
 inline size_t mixed_words(uint64_t n) { return (n + 31) / 32; }
 inline size_t mixed_shared_bytes(int mode, uint64_t n) {
@@ -336,7 +337,7 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
             }
             s.k = k;
             S.graph = gi;
-            s.late = globaltimer_ns() > deadline;
+            S.late = globaltimer_ns() > deadline;
             reset_sums(s);
             S.nitems = S.next_item = S.set_count = S.cand_count = 0;
             S.smax = S.best = 0;
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
             if (last_gi != 0xffffffffu) flush_stats(pk.g[last_gi].stats);
             last_gi = gi;
         }
-        if (s.late) {
+        if (S.late) {
             if (tid == 0) atomicOr(p.work + 1, kErrDeadline);
             break;
         }
