@@ -351,7 +351,8 @@ __device__ __forceinline__ unsigned long long warp_nth_largest_u64(unsigned long
 }
 
 // The rg-th largest key (counting repeats) of value(i), i < count, by digits of eight bits (see
-// block_nth_largest).  At least rg keys are positive.
+// block_nth_largest); 0 when fewer than rg keys are positive (a vertex that is drained after its last
+// visit of the round stays in the frontier with residual 0).
 template <int BITS, class Value>
 __device__ __forceinline__ unsigned long long gs_nth_largest(GsScratch& s, uint32_t count, uint32_t rg, Value value) {
     unsigned long long prefix = 0;
@@ -382,6 +383,7 @@ __device__ __forceinline__ unsigned long long gs_nth_largest(GsScratch& s, uint3
                 if (lane >= uint32_t(o)) incl += y;
             }
             const unsigned reach = __ballot_sync(kFullMask, incl >= rest);
+            if (!reach && lane == 0) s.rest = 0;  // too few (seen at the first digit)
             if (lane == uint32_t(__ffs(int(reach)) - 1)) {
                 uint32_t left = rest - (incl - sum);
                 int k = 0;
@@ -393,6 +395,7 @@ __device__ __forceinline__ unsigned long long gs_nth_largest(GsScratch& s, uint3
         __syncthreads();
         prefix = (prefix << 8) | s.bin;
         rest = s.rest;
+        if (rest == 0) return 0;
     }
     return prefix;
 }
