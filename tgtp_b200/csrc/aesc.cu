@@ -2150,7 +2150,8 @@ MixedLayout mixed_layout(int mode, uint64_t n, uint64_t max_degree, uint64_t row
     l.item_bytes = align(sizeof(WalkItem) * std::max<uint64_t>(max_degree, 1) * l.blocks);
     l.sum_bytes = mode == kGlobal ? align(sizeof(unsigned long long) * size_t(n) * l.blocks) : 0;
     l.touched_bytes = mode == kGlobal ? align(sizeof(uint32_t) * size_t(n) * l.blocks) : 0;
-    l.bit_bytes = mode == kGlobal && 4 * mixed_words(n) > kBitsInSmem ? align(4 * mixed_words(n) * l.blocks) : 0;
+    const bool gbits = mode == kShared || (mode == kGlobal && 4 * mixed_words(n) > kBitsInSmem);
+    l.bit_bytes = gbits ? align(4 * mixed_words(n) * l.blocks) : 0;
     return l;
 }
 void carve_mixed(MixedParams& p, const MixedLayout& l, unsigned char* base, uint64_t n, uint64_t max_degree) {

@@ -169,12 +169,13 @@ struct Frontier {
     uint32_t cap;
 };
 
-// Appends the lanes' vertices with r > 0 (K of them per lane) to the frontier and adds up what the
-// cost test needs.  All lanes of a warp call it.
+// Appends the lanes' vertices with r > 0 (K of them per lane; REACHED: those with a number, also where
+// r is 0) to the frontier and adds up what the cost test needs.  All lanes of a warp call it.
 struct FrontierSums {
     uint32_t pc = 0, mx = 0, mn = 0x3f800000u;  // degree sum, bits of the largest and smallest residual
 };
-template <int K>
+constexpr uint32_t kNoVertex = 0xffffffffu;
+template <int K, bool REACHED = false>
 __device__ __forceinline__ void append_frontier(PushScratch& s, const Frontier& f, FrontierSums& t,
                                                 const uint32_t (&u)[K], const uint32_t (&beg)[K],
                                                 const uint32_t (&deg)[K], const float (&r)[K]) {
@@ -184,7 +185,7 @@ __device__ __forceinline__ void append_frontier(PushScratch& s, const Frontier& 
     uint32_t nl = 0, nh = 0;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        const bool live = r[k] > 0.f, big = live && deg[k] > kHeavyRow;
+        const bool live = REACHED ? u[k] != kNoVertex : r[k] > 0.f, big = live && deg[k] > kHeavyRow;
         bl[k] = __ballot_sync(kFullMask, live && !big);
         bh[k] = __ballot_sync(kFullMask, big);
         nl += __popc(bl[k]);
@@ -200,7 +201,7 @@ __device__ __forceinline__ void append_frontier(PushScratch& s, const Frontier& 
     if (nh) hat = __shfl_sync(kFullMask, hat, 0);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        if (r[k] > 0.f) {
+        if (REACHED ? u[k] != kNoVertex : r[k] > 0.f) {
             const bool big = (bh[k] >> lane) & 1u;
             f.list[big ? f.cap - 1u - (hat + uint32_t(__popc(bh[k] & below)))
                        : at + uint32_t(__popc(bl[k] & below))] =

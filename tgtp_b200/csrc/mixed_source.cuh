@@ -42,7 +42,7 @@ struct MixedParams {
     WalkItem* items;
     unsigned long long* sums;  // kGlobal: scratch_n words, all zero between sources
     uint32_t* touched;         // kGlobal: scratch_n vertices
-    uint32_t* gbits;           // kGlobal: the bitmap when it is not in shared memory
+    uint32_t* gbits;           // kGlobal: the bitmap when it is not in shared memory; kShared: see round_with_zeros
     unsigned char* clean;      // kGlobal, per block: 1 = its sums and bitmap are all zero
     // kColumn
     uint32_t list_base, list_cap;
@@ -82,7 +82,7 @@ inline bool mixed_fits_shared(uint64_t n) { return mixed_shared_bytes(kShared, n
 
 // The rg-th largest (counting repeats) of the positive values value(i), i < count, as FP32 bits:
 // the digits are fixed eight bits at a time from a histogram of the values that share the digits
-// fixed so far.  At least rg values are positive.  All threads of the block call it.
+// fixed so far; 0 when fewer than rg values are positive.  All threads of the block call it.
 template <class Value>
 __device__ __forceinline__ uint32_t block_nth_largest(SourceScratch& s, uint32_t count, uint32_t rg, Value value) {
     uint32_t prefix = 0, rest = rg;
@@ -109,6 +109,7 @@ __device__ __forceinline__ uint32_t block_nth_largest(SourceScratch& s, uint32_t
                 if (lane >= uint32_t(o)) incl += y;
             }
             const unsigned reach = __ballot_sync(kFullMask, incl >= rest);
+            if (!reach && lane == 0) s.rest = 0;  // too few (seen at the first digit)
             if (lane == uint32_t(__ffs(int(reach)) - 1)) {
                 uint32_t left = rest - (incl - sum);
                 int k = 0;
@@ -120,6 +121,7 @@ __device__ __forceinline__ uint32_t block_nth_largest(SourceScratch& s, uint32_t
         __syncthreads();
         prefix = (prefix << 8) | s.bin;
         rest = s.rest;
+        if (rest == 0) return 0;
     }
     return prefix;
 }
@@ -241,6 +243,53 @@ __device__ __forceinline__ uint32_t drain_bits(PushScratch& s, uint32_t* bits, u
     return s.chunk.total;
 }
 
+// A round of kShared in which a residual may be 0.  Every vertex a frontier vertex reaches is in the
+// next frontier, also one whose residual rounds to 0 (below 2^-62) or is a sum of such.  A vertex's sum
+// is at least one frontier residual, so its residual is above 0 while the smallest of them is at least
+// the largest degree in 2^-62; the other rounds (far vertices of grids and the like, after 30 rounds
+// and more) come here, where the neighbours of the frontier's zeros have bits of their own (all clear
+// between rounds).  The block pushes leave vertices with residual 0 out, so where there are some a
+// source may stop at another round than here.
+__device__ __noinline__ void round_with_zeros(PushScratch& s, uint32_t* lo, uint32_t* hi, uint32_t* bits,
+                                              const uint32_t* __restrict__ idx, const uint32_t* __restrict__ adj,
+                                              const double* __restrict__ dinv, uint32_t n, const Frontier& f,
+                                              uint32_t nl, uint32_t nh) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    push_frontier(s, f, nl, nh, adj, [&](uint32_t u, unsigned long long v) { add_fixed(lo, hi, u, v); });
+    for (uint32_t i = warp; i < nl + nh; i += nw) {
+        const uint4 v = f.list[i < nl ? i : f.cap - 1u - (i - nl)];
+        if (v.z) continue;
+        for (uint32_t o = lane; o < v.y; o += 32) {
+            const uint32_t u = __ldg(adj + v.x + o);
+            atomicOr(bits + (u >> 5), 1u << (u & 31u));
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) reset_sums(s);
+    __syncthreads();
+    FrontierSums t;
+    for (uint32_t w = warp; w < (n + 31u) / 32u; w += nw) {
+        const uint32_t x = __ldcg(bits + w);
+        const uint32_t v = w * 32u + lane;
+        uint32_t u[1] = {kNoVertex}, b[1] = {0u}, d[1] = {1u};
+        float r[1] = {0.f};
+        if (v < n) {
+            const uint32_t sl = lo[v], sh = hi[v];
+            b[0] = __ldg(idx + v);
+            d[0] = __ldg(idx + v + 1) - b[0];
+            if (sl | sh) {
+                r[0] = from_fixed(sh, sl, d[0], __ldg(dinv + v));
+                lo[v] = __float_as_uint(r[0]);
+                hi[v] = 0u;
+            }
+            if ((sl | sh) || ((x >> lane) & 1u)) u[0] = v;
+        }
+        append_frontier<1, true>(s, f, t, u, b, d, r);
+        if (lane == 0 && x) bits[w] = 0u;
+    }
+    add_sums(s, t);
+}
+
 template <int MODE, class Pack>
 __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
     extern __shared__ __align__(16) unsigned char mixed_smem[];
@@ -255,7 +304,7 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
     uint32_t* const hi = smem_words + pad;  // kShared
     const uint32_t bwords = (sn + 31u) / 32u;
     const bool bits_here = MODE == kGlobal && size_t(4) * bwords <= kBitsInSmem;
-    uint32_t* const gbits = MODE == kGlobal && !bits_here ? p0.gbits + size_t(blockIdx.x) * bwords : nullptr;
+    uint32_t* const gbits = MODE == kShared || (MODE == kGlobal && !bits_here) ? p0.gbits + size_t(blockIdx.x) * bwords : nullptr;
     unsigned long long* const sums = MODE == kGlobal ? p0.sums + size_t(blockIdx.x) * sn : nullptr;
     uint32_t* const touched = MODE == kGlobal ? p0.touched + size_t(blockIdx.x) * sn : nullptr;
     const Frontier f{p0.lists + size_t(blockIdx.x) * sn, sn};
@@ -266,6 +315,8 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
         for (uint32_t w = tid; w < bwords; w += blockDim.x) smem_words[w] = 0u;
     pdl_launch_dependents();
     pdl_wait();  // taus and row lists of the tau kernels; the columns of a block push
+    if (MODE == kShared)
+        for (uint32_t w = tid; w < bwords; w += blockDim.x) gbits[w] = 0u;
     if (MODE == kGlobal && !p0.clean[blockIdx.x]) {
         for (uint32_t u = tid; u < sn; u += blockDim.x) sums[u] = 0ull;
         if (gbits)
@@ -419,60 +470,64 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
                     }
                 }
                 __syncthreads();
-                push_frontier(s, f, nl, nh, adj, [&](uint32_t u, unsigned long long v) {
-                    if (MODE == kShared) {
-                        add_fixed(lo, hi, u, v);
-                    } else {
-                        atomicAdd(sums + u, v);
-                        if (bits_here) atomicOr(smem_words + (u >> 5), 1u << (u & 31u));
-                        else atomicOr(gbits + (u >> 5), 1u << (u & 31u));
-                    }
-                });
-                __syncthreads();
-                if (tid == 0) reset_sums(s);
-                __syncthreads();
-                if (MODE == kShared) {
-                    take_residuals(s, lo, hi, idx, p.dinv, n, f);
+                if (MODE == kShared && to_fixed(__uint_as_float(s.gmin)) < p0.max_degree) {
+                    round_with_zeros(s, lo, hi, gbits, idx, adj, p.dinv, n, f, nl, nh);
                 } else {
-                    const uint32_t count = drain_bits(s, bits_here ? smem_words : gbits, (n + 31u) / 32u, touched);
+                    push_frontier(s, f, nl, nh, adj, [&](uint32_t u, unsigned long long v) {
+                        if (MODE == kShared) {
+                            add_fixed(lo, hi, u, v);
+                        } else {
+                            atomicAdd(sums + u, v);
+                            if (bits_here) atomicOr(smem_words + (u >> 5), 1u << (u & 31u));
+                            else atomicOr(gbits + (u >> 5), 1u << (u & 31u));
+                        }
+                    });
                     __syncthreads();
-                    constexpr int K = 4;
-                    FrontierSums t;
-                    for (uint32_t i0 = tid - lane; i0 < count; i0 += K * blockDim.x) {
-                        uint32_t u[K], b[K], d[K];
-                        float r[K];
-                        unsigned long long sum[K];
-                        double inv[K];
+                    if (tid == 0) reset_sums(s);
+                    __syncthreads();
+                    if (MODE == kShared) {
+                        take_residuals(s, lo, hi, idx, p.dinv, n, f);
+                    } else {
+                        const uint32_t count = drain_bits(s, bits_here ? smem_words : gbits, (n + 31u) / 32u, touched);
+                        __syncthreads();
+                        constexpr int K = 4;
+                        FrontierSums t;
+                        for (uint32_t i0 = tid - lane; i0 < count; i0 += K * blockDim.x) {
+                            uint32_t u[K], b[K], d[K];
+                            float r[K];
+                            unsigned long long sum[K];
+                            double inv[K];
 #pragma unroll
-                        for (int k = 0; k < K; ++k) {
-                            const uint32_t i = i0 + k * blockDim.x + lane;
-                            u[k] = i < count ? touched[i] : 0xffffffffu;
-                        }
-#pragma unroll
-                        for (int k = 0; k < K; ++k) {
-                            sum[k] = 0;
-                            b[k] = 0;
-                            d[k] = 1;
-                            inv[k] = 1.0;
-                            if (u[k] != 0xffffffffu) {
-                                sum[k] = __ldcg(sums + u[k]);
-                                b[k] = __ldg(idx + u[k]);
-                                d[k] = __ldg(idx + u[k] + 1);
-                                inv[k] = __ldg(p.dinv + u[k]);
+                            for (int k = 0; k < K; ++k) {
+                                const uint32_t i = i0 + k * blockDim.x + lane;
+                                u[k] = i < count ? touched[i] : kNoVertex;
                             }
-                        }
 #pragma unroll
-                        for (int k = 0; k < K; ++k) {
-                            r[k] = 0.f;
-                            d[k] -= b[k];
-                            if (sum[k]) {
-                                r[k] = from_fixed(uint32_t(sum[k] >> 32), uint32_t(sum[k]), d[k], inv[k]);
-                                sums[u[k]] = __float_as_uint(r[k]);
+                            for (int k = 0; k < K; ++k) {
+                                sum[k] = 0;
+                                b[k] = 0;
+                                d[k] = 1;
+                                inv[k] = 1.0;
+                                if (u[k] != kNoVertex) {
+                                    sum[k] = __ldcg(sums + u[k]);
+                                    b[k] = __ldg(idx + u[k]);
+                                    d[k] = __ldg(idx + u[k] + 1);
+                                    inv[k] = __ldg(p.dinv + u[k]);
+                                }
                             }
+#pragma unroll
+                            for (int k = 0; k < K; ++k) {
+                                r[k] = 0.f;
+                                d[k] -= b[k];
+                                if (sum[k]) {
+                                    r[k] = from_fixed(uint32_t(sum[k] >> 32), uint32_t(sum[k]), d[k], inv[k]);
+                                    sums[u[k]] = __float_as_uint(r[k]);
+                                }
+                            }
+                            append_frontier<K, true>(s, f, t, u, b, d, r);
                         }
-                        append_frontier<K>(s, f, t, u, b, d, r);
+                        add_sums(s, t);
                     }
-                    add_sums(s, t);
                 }
                 __syncthreads();
                 lap(1);
