@@ -2118,6 +2118,24 @@ MixedPlan plan_mixed(tgtp_graph* g, const tgtp_config& cfg) {
     return p;
 }
 
+// The per-block "vector is all zero" marks of a run that carves the handle's scratch as `kind` says.
+// They hold while the same carving of the same scratch runs again; a run that reads them after
+// another one clears them first.  A captured run can be replayed between any two later runs, which
+// the host does not see, so it clears them inside the capture, and from then on every run on the
+// handle does.
+unsigned char* clean_marks(tgtp_graph* g, uint64_t kind, unsigned blocks, bool reads) {
+    const uint64_t sig[5] = {kind, blocks, g->n, uint64_t(reinterpret_cast<uintptr_t>(g->scratch.ptr)),
+                             uint64_t(g->scratch.bytes)};
+    grow(g, g->wclean, blocks + 16);
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    TGTP_CUDA(cudaStreamIsCapturing(g->stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) g->captured = true;
+    if (reads && (g->captured || std::memcmp(sig, g->wclean_sig, sizeof(sig)) != 0))
+        TGTP_CUDA(cudaMemsetAsync(g->wclean.ptr, 0, blocks + 16, g->stream));
+    std::memcpy(g->wclean_sig, sig, sizeof(sig));
+    return g->wclean.as<unsigned char>();
+}
+
 // Blocks of the mixed form's per-source kernel in one of its modes over up to n vertices.
 struct MixedLayout {
     unsigned blocks, threads;
@@ -2216,23 +2234,14 @@ bool run_mixed(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMarks
         p.trace_ell = p.trace_nr + m;
         g->trace_valid = true;
     }
-    // the per-block "sums are zero" marks hold only for the same carving of the same scratch
-    {
-        const uint64_t sig[5] = {uint64_t(key) | (uint64_t(mode) << 8) | (uint64_t(1) << 63), lay.blocks, uint64_t(n),
-                                 uint64_t(reinterpret_cast<uintptr_t>(g->scratch.ptr)),
-                                 uint64_t(g->scratch.bytes)};
-        grow(g, g->wclean, lay.blocks + 16);
-        if (std::memcmp(sig, g->wclean_sig, sizeof(sig)) != 0) {
-            TGTP_CUDA(cudaMemsetAsync(g->wclean.ptr, 0, lay.blocks + 16, s));
-            std::memcpy(g->wclean_sig, sig, sizeof(sig));
-        }
-        p.clean = g->wclean.as<unsigned char>();
-    }
     MixedPack<1> pk;
     pk.count = 1;
     if (!mp.block_mode) {
         p.claim = work;
         if (defer_to_batch(g, cfg, out, mode == kShared, p)) return false;
+    }
+    p.clean = clean_marks(g, uint64_t(key) | (uint64_t(mode) << 8) | (uint64_t(1) << 63), lay.blocks, mode == kGlobal);
+    if (!mp.block_mode) {
         pk.g[0] = p;
         ScopedKernel k(g->prof, s, "source");
         launch_mixed(mode, lay, s, true, pk);
@@ -2527,18 +2536,6 @@ bool run_sources(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMar
         p.trace_ell = p.trace_nr + m;
         g->trace_valid = true;
     }
-    // the per-block "vector is zero" marks hold only for the same carving of the same scratch
-    {
-        const uint64_t sig[5] = {uint64_t(key) | (uint64_t(use_smem) << 8) | (uint64_t(1) << 62), l.blocks, uint64_t(n),
-                                 uint64_t(reinterpret_cast<uintptr_t>(g->scratch.ptr)),
-                                 uint64_t(g->scratch.bytes)};
-        grow(g, g->wclean, l.blocks + 16);
-        if (std::memcmp(sig, g->wclean_sig, sizeof(sig)) != 0) {
-            TGTP_CUDA(cudaMemsetAsync(g->wclean.ptr, 0, l.blocks + 16, s));
-            std::memcpy(g->wclean_sig, sig, sizeof(sig));
-        }
-        p.clean = g->wclean.as<unsigned char>();
-    }
     {
         // The windowed push pays off when rows are short: several frontier vertices share a 32-entry
         // step.  With long rows each vertex fills its steps anyway and adjacent frontier vertices cut
@@ -2554,6 +2551,7 @@ bool run_sources(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMar
     }
     p.claim = run_work(g);
     if (defer_to_batch(g, cfg, out, use_smem, p)) return false;
+    p.clean = clean_marks(g, uint64_t(key) | (uint64_t(use_smem) << 8) | (uint64_t(1) << 62), l.blocks, !use_smem);
     Pack1 pk;
     pk.count = 1;
     pk.g[0] = p;
