@@ -33,7 +33,7 @@ CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-Wextra", "-I" + INCLUDE, "
              "-I" + os.path.join(CUDA_HOME, "include")]
 
 CU_SOURCES = ["api.cu", "saba.cu", "aesc.cu", "batch.cu", "exact_sc.cu", "mt_walk.cu"]
-CPP_SOURCES = ["host_io.cpp"]
+CPP_SOURCES = ["host_io.cpp", "occupancy.cpp"]
 # executable -> (source under csrc/host, extra flags)
 RUNNERS = {"tgtp": ("tgtp_main.cpp", []), "benchmark": ("benchmark_main.cpp", []),
            "rw_experiment_saba": ("rw_experiment_saba_main.cpp", []),

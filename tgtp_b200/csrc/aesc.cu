@@ -37,11 +37,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
-#include <map>
 #include <memory>
 #include <vector>
-#include <mutex>
-#include <tuple>
 #include <type_traits>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -1980,30 +1977,6 @@ void launch(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem, 
     cfg.numAttrs = (pdl && pdl_enabled()) ? 1 : 0;
     TGTP_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
 }
-
-}  // namespace
-
-int blocks_per_sm(const void* kern, int threads, size_t smem) {
-    static std::mutex mu;
-    static std::map<std::tuple<const void*, int, size_t, int>, int> cache;
-    static std::map<const void*, size_t> limit;
-    int dev = 0;
-    TGTP_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lock(mu);
-    const auto key = std::make_tuple(kern, threads, smem, dev);
-    auto it = cache.find(key);
-    if (it != cache.end()) return it->second;
-    if (smem > limit[kern]) {
-        TGTP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        limit[kern] = smem;
-    }
-    int per_sm = 0;
-    TGTP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-    cache[key] = per_sm;
-    return per_sm;
-}
-
-namespace {
 
 // Symmetrisation of one run (stage 3) on the graph's stream.
 template <class Real, class Acc>
