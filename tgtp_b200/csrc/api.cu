@@ -38,7 +38,16 @@ size_t size_class(size_t bytes) {
 }
 }  // namespace
 
+// TGTP_ALLOC_LIMIT: the largest device block, in bytes, that is granted (as on a device with no more
+// room; the tests of the smaller forms set it).
+size_t alloc_limit() {
+    const char* e = std::getenv("TGTP_ALLOC_LIMIT");
+    const unsigned long long v = e ? std::strtoull(e, nullptr, 10) : 0ull;
+    return v ? size_t(v) : SIZE_MAX;
+}
+
 void* cache_alloc(size_t bytes, size_t* granted) {
+    if (bytes > alloc_limit()) fail(TGTP_ERR_OUT_OF_MEMORY, "device block above TGTP_ALLOC_LIMIT");
     int dev = 0;
     TGTP_CUDA(cudaGetDevice(&dev));
     const size_t c = size_class(bytes);

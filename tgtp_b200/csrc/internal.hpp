@@ -67,6 +67,7 @@ tgtp_status guarded(F&& f) {
 // device after release; a release first waits for the device to be idle, so no queued kernel can
 // still be using the block when it is handed out again.  tgtp_release_cached_memory() returns the
 // cached blocks to the driver.
+size_t alloc_limit();
 void* cache_alloc(size_t bytes, size_t* granted);
 void cache_free(void* p, size_t granted);
 void cache_trim();
@@ -209,6 +210,7 @@ struct tgtp_graph {
     uint32_t saba_ncls = 0;
     tgtp::DeviceBuffer mt_seeds;  // per warp of the MT19937 walks: the states of its next sources
     bool saba_ready = false, saba_plain_ready = false, saba_packed_ready = false;
+    bool saba_no_packed = false;  // the device had no room for the packed copy
     // the walk layout saba_tune chose: walkers per lane (low byte: 1, 2 or 4, so 4, 8 or 16
     // bouquets per warp) and 0x100 for the packed copy; 0 = not tuned
     uint16_t saba_choice = 0;
@@ -239,6 +241,7 @@ void saba_prepare(tgtp_graph* g);
 void saba_prepare_plain(tgtp_graph* g);
 bool saba_packable(const tgtp_graph* g);
 PackedWalk saba_prepare_packed(tgtp_graph* g);
+bool saba_prepare_copy(tgtp_graph* g, bool packed);
 // Visit counters of the renumbered vertices in global memory.  Numbers are in order of degree, so
 // neighbouring numbers take visits at similar rates and the first ones the most: sectors of eight
 // counters are dealt out to 64 runs of the array, so that the busy ones spread over the L2 slices.

@@ -238,14 +238,10 @@ void mt_walk_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, bool simd,
         return;
     }
     saba_prepare(g);
-    const bool packed = saba_packable(g);
+    const bool packed = saba_prepare_copy(g, saba_packable(g));
     PackedWalk w{};
-    if (packed) {
-        w = saba_prepare_packed(g);
-    } else {
-        saba_prepare_plain(g);
-        w.info = g->saba_info.as<uint4>();
-    }
+    if (packed) w = saba_prepare_packed(g);
+    else w.info = g->saba_info.as<uint4>();
     auto kern = simd ? (packed ? mt_walk_kernel<true, true> : mt_walk_kernel<true, false>)
                      : (packed ? mt_walk_kernel<false, true> : mt_walk_kernel<false, false>);
     // shared memory: the rings, the classes (12 bytes each), and counters in what is left of it
@@ -254,9 +250,17 @@ void mt_walk_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, bool simd,
     const uint32_t hot = uint32_t(std::min<uint64_t>({g->n, kMtHot, room / sizeof(uint32_t)}));
     const size_t smem = fixed + sizeof(uint32_t) * hot;
     const int per_sm = std::max(1, blocks_per_sm(reinterpret_cast<const void*>(kern), kMtThreads, smem));
-    const uint64_t blocks =
-        std::min<uint64_t>(uint64_t(g->num_sms) * per_sm, (g->n + kMtWarps - 1) / kMtWarps);
-    g->mt_seeds.reserve(blocks * kMtWarps * kSeedAhead * kMtWords * sizeof(uint32_t));
+    uint64_t blocks = std::min<uint64_t>(uint64_t(g->num_sms) * per_sm, (g->n + kMtWarps - 1) / kMtWarps);
+    // the generators' states (320 KB a block); fewer blocks where the device has no room for all
+    for (bool there = false; !there;) {
+        try {
+            g->mt_seeds.reserve(blocks * kMtWarps * kSeedAhead * kMtWords * sizeof(uint32_t));
+            there = true;
+        } catch (const Error& e) {
+            if (e.code != TGTP_ERR_OUT_OF_MEMORY || blocks <= 1) throw;
+            blocks /= 2;
+        }
+    }
     {
         ScopedKernel k(g->prof, s, "mt_walk");
         kern<<<unsigned(blocks), kMtThreads, smem, s>>>(w, g->saba_adj.as<uint32_t>(), g->n, depth, n_walks,

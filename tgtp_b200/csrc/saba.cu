@@ -548,9 +548,10 @@ uint32_t saba_pbits(const tgtp_graph* g) {
 }
 
 // Whether the graph's numbers and classes fit in a packed slot's 32 bits and the class table in
-// its shared memory, and the copy takes at most 4 GiB (needs saba_prepare).
+// its shared memory, and the copy takes at most 4 GiB and did not fail to fit on the device (needs
+// saba_prepare).
 bool saba_packable(const tgtp_graph* g) {
-    return saba_pbits(g) < 32 && g->saba_ncls <= kMaxClasses &&
+    return !g->saba_no_packed && saba_pbits(g) < 32 && g->saba_ncls <= kMaxClasses &&
            g->saba_ncls <= (uint64_t(1) << (32 - saba_pbits(g))) &&
            g->m * sizeof(uint2) <= (uint64_t(4) << 30);
 }
@@ -577,6 +578,22 @@ PackedWalk saba_prepare_packed(tgtp_graph* g) {
     w.classes = g->saba_classes.as<uint2>();
     w.info = g->saba_info.as<uint4>();
     return w;
+}
+
+// The packed copy if `packed` and the device has room for its 8 bytes per slot, else the plain one (4);
+// returns which (needs saba_prepare).
+bool saba_prepare_copy(tgtp_graph* g, bool packed) {
+    if (packed) {
+        try {
+            (void)saba_prepare_packed(g);
+            return true;
+        } catch (const Error& e) {
+            if (e.code != TGTP_ERR_OUT_OF_MEMORY) throw;
+            g->saba_no_packed = true;
+        }
+    }
+    saba_prepare_plain(g);
+    return false;
 }
 
 // Whether saba_count walks the packed copy (one dependent 8-byte load per hop) or the plain
@@ -608,16 +625,15 @@ template <int WPL>
 void saba_launch(tgtp_graph* g, uint32_t depth, uint32_t bps, uint32_t grid_step, uint64_t total,
                  WalkCounters cnt, unsigned long long* fb) {
     cudaStream_t s = g->stream;
-    uint32_t cap = saba_use_packed(g) ? kPackedHotCap : kSabaHotCap;
+    const bool packed = saba_use_packed(g);  // the copy is there (saba_run)
+    uint32_t cap = packed ? kPackedHotCap : kSabaHotCap;
     if (const char* e = std::getenv("TGTP_SABA_HOT")) cap = uint32_t(std::atoi(e));
     cap = std::max<uint32_t>(1024u, std::min<uint32_t>(cap, 53248u));
-    const bool packed = saba_use_packed(g);
     if (packed) cap = std::min<uint32_t>(cap, 53248u - 2 * g->saba_ncls);  // beside the class table
     const uint32_t hot = uint32_t(g->n < cap ? g->n : cap);
     const uint32_t hot_rec = packed ? 0u : std::min(hot, saba_hot_records(g));
     PackedWalk pw{};
     if (packed) pw = saba_prepare_packed(g);
-    else saba_prepare_plain(g);
     const size_t smem = sizeof(uint32_t) * (hot + 3 * size_t(hot_rec)) + sizeof(uint2) * pw.ncls;
     const void* kern = packed ? reinterpret_cast<const void*>(saba_walk_packed_kernel<WPL>)
                               : reinterpret_cast<const void*>(saba_walk_perm_kernel<WPL>);
@@ -676,7 +692,7 @@ void saba_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, uint32_t* device_
     // walkers per lane: the tuned choice, else TGTP_SABA_WPL, else 1 over the packed copy (2: within
     // 2 % on large graphs, 6 % slower on the 4,039-vertex one) and 2 over the plain one (its two
     // dependent loads per hop want more chains in flight)
-    int wpl = saba_use_packed(g) ? 1 : 2;
+    int wpl = saba_prepare_copy(g, saba_use_packed(g)) ? 1 : 2;
     if (g->saba_choice) wpl = g->saba_choice & 0xff;
     else if (const char* e = std::getenv("TGTP_SABA_WPL")) wpl = std::atoi(e);
     switch (wpl) {
