@@ -2064,15 +2064,28 @@ MixedPlan plan_mixed(tgtp_graph* g, const tgtp_config& cfg) {
         p.block_mode = g->push_hint[key] == 2;
     else p.block_mode = mixed_beyond_smem(n) && cfg.epsilon <= 0.01;
     // Graphs whose sums fit in shared memory push one source per block (push_shared_kernel), all
-    // listed sources in waves of at most 4 GiB of residual vectors; a knob of the 32-source block
-    // push asks for that one.  Sparse Chung-Lu graph (n = 25,860), eps = 0.005 / 0.05: push 208 / 109 ms
+    // listed sources in waves of at most 4 GiB of residual vectors, or of half the device memory free
+    // now (beside what the columns already hold) where that is less, but not below what the 32-source
+    // push takes; in a live batch, which pins the columns, of what they hold.  A knob of the 32-source
+    // block push asks for that one.  Sparse Chung-Lu graph (n = 25,860), eps = 0.005 / 0.05: push 208 / 109 ms
     // with the 32-source block push (six waves), 79 / 19 ms with this one (its inner loop takes 55 ms of the 79:
     // 21.6e9 additions of two shared atomics each).
     const bool block_knob = std::getenv("TGTP_BLOCK_CTAS") || std::getenv("TGTP_BLOCK_ROUNDS") ||
                             std::getenv("TGTP_BLOCK_MASKS") || std::getenv("TGTP_BLOCK_LIST_DIV");
     p.shared_push = p.block_mode && push_shared_bytes(n) <= size_t(227) * 1024 && !block_knob;
-    const uint32_t shared_wave =
+    uint32_t shared_wave =
         uint32_t(std::min<uint64_t>(n, std::max<uint64_t>(1, (uint64_t(4) << 30) / (sizeof(float) * n))));
+    const uint64_t held_wave = g->block_cols.bytes / (sizeof(float) * n);
+    if (p.shared_push && held_wave < shared_wave) {
+        uint64_t wave = held_wave;
+        if (g->batch_refs == 0 || wave == 0) {
+            size_t free_b = 0, total_b = 0;
+            TGTP_CUDA(cudaMemGetInfo(&free_b, &total_b));
+            const uint64_t budget = (std::min(free_b, alloc_limit()) + g->block_cols.bytes) / 2;
+            wave = std::max<uint64_t>({wave, budget / (sizeof(float) * n), 2 * kBlockCols * uint64_t(g->num_sms)});
+        }
+        shared_wave = uint32_t(std::min<uint64_t>(shared_wave, wave));
+    }
     // CTAs of the 32-source block push: one per SM, within a budget for their residual blocks of 24 GB or
     // half the device memory free now (beside what the blocks already hold), whichever is larger
     // (TGTP_BLOCK_CTAS lowers the count, e.g. to exercise many waves on small graphs)
