@@ -2154,7 +2154,10 @@ MixedLayout mixed_layout(int mode, uint64_t n, uint64_t max_degree, uint64_t row
     l.item_bytes = align(sizeof(WalkItem) * std::max<uint64_t>(max_degree, 1) * l.blocks);
     l.sum_bytes = mode == kGlobal ? align(sizeof(unsigned long long) * size_t(n) * l.blocks) : 0;
     l.touched_bytes = mode == kGlobal ? align(sizeof(uint32_t) * size_t(n) * l.blocks) : 0;
-    const bool gbits = mode == kShared || (mode == kGlobal && 4 * mixed_words(n) > kBitsInSmem);
+    // the bitmap in HBM: beyond kBitsInSmem, or as TGTP_BLOCK_MASKS=global asks (kShared: always)
+    const char* masks = std::getenv("TGTP_BLOCK_MASKS");
+    const bool gbits = mode == kShared || (mode == kGlobal && (4 * mixed_words(n) > kBitsInSmem ||
+                                                               (masks && std::string(masks) == "global")));
     l.bit_bytes = gbits ? align(4 * mixed_words(n) * l.blocks) : 0;
     return l;
 }
@@ -2226,7 +2229,8 @@ bool run_mixed(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMarks
         p.claim = work;
         if (defer_to_batch(g, cfg, out, mode == kShared, p)) return false;
     }
-    p.clean = clean_marks(g, uint64_t(key) | (uint64_t(mode) << 8) | (uint64_t(1) << 63), lay.blocks, mode == kGlobal);
+    p.clean = clean_marks(g, uint64_t(key) | (uint64_t(mode) << 8) | (uint64_t(lay.bit_bytes != 0) << 16) | (uint64_t(1) << 63),
+                          lay.blocks, mode == kGlobal);
     if (!mp.block_mode) {
         pk.g[0] = p;
         ScopedKernel k(g->prof, s, "source");

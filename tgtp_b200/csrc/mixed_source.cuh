@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
     uint32_t* const lo = smem_words;        // kShared
     uint32_t* const hi = smem_words + pad;  // kShared
     const uint32_t bwords = (sn + 31u) / 32u;
-    const bool bits_here = MODE == kGlobal && size_t(4) * bwords <= kBitsInSmem;
+    const bool bits_here = MODE == kGlobal && !p0.gbits;
     uint32_t* const gbits = MODE == kShared || (MODE == kGlobal && !bits_here) ? p0.gbits + size_t(blockIdx.x) * bwords : nullptr;
     unsigned long long* const sums = MODE == kGlobal ? p0.sums + size_t(blockIdx.x) * sn : nullptr;
     uint32_t* const touched = MODE == kGlobal ? p0.touched + size_t(blockIdx.x) * sn : nullptr;
