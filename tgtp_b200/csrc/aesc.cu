@@ -2432,9 +2432,11 @@ GsLayout gs_layout(bool use_smem, uint64_t n, uint64_t max_degree, uint64_t rows
     if (per_sm < 1) fail(TGTP_ERR_UNSUPPORTED, "source kernel does not fit on an SM");
     // Small vectors: where registers and not shared memory limit the 128-thread blocks and there are
     // sources for more than one round of them, blocks of half the threads, so that more sources push
-    // at a time (FP64, n = 2,000, 20 neighbours, eps = 0.005: 2.81 ms against 3.13; at n = 600, one
-    // round, 0.626 against 0.610; at n = 5,500, shared memory the limit, 17.3 against 16.7).
-    if (use_smem && rows * 4 > uint64_t(num_sms) * per_sm * 5) {
+    // at a time (FP64, eps = 0.005: n = 2,000, 20 neighbours 2.81 ms against 3.13; n = 1,000, 14 and 6
+    // neighbours, 888 blocks of 128 threads or all sources at once, 1.13 against 1.39 and 4.27 against
+    // 6.03; n = 600, one round, 0.626 against 0.610; at n = 5,500, shared memory the limit, 17.3 against
+    // 16.7).
+    if (use_smem && rows > uint64_t(num_sms) * per_sm) {
         const int half = blocks_per_sm(kern, int(l.threads) / 2, l.smem);
         if (half > per_sm) {
             l.threads /= 2;
