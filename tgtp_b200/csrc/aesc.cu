@@ -2534,12 +2534,16 @@ bool run_sources(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMar
         // windows often.  In shared memory the line is at 15 neighbours (one vertex at a time /
         // windowed, ms: 9.5 neighbours 2.96 / 2.02; 14: 3.04 / 2.78; 16: 2.37 / 2.39; 20: 2.81 / 3.17;
         // 44: 0.73 / 1.42), in HBM, where a step waits for its words, at 32 (20: 18.7 / 12.8; 30:
-        // 5.18 / 4.94; 44: 1.73 / 2.44).  The tuned layout, then TGTP_GS_WINDOW=0/1, override the rule.
+        // 5.18 / 4.94; 44: 1.73 / 2.44).  Where two vertices are neighbours with a chance of 1 in 25 or
+        // more, half of the windows of eight are cut and it does not pay (n = 150, 6 neighbours: FP64
+        // 0.305 / 0.336, FP32 0.289 / 0.346; n = 150, 12: FP64 0.187 / 0.324; n = 300, 12: FP64 0.63 / 0.84,
+        // FP32 0.59 / 0.85; at 1 in 50, n = 300, 6 neighbours: FP64 1.05 / 0.88, FP32 0.96 / 0.88).  The tuned
+        // layout, then TGTP_GS_WINDOW=0/1, override the rule.
         const char* e = std::getenv("TGTP_GS_WINDOW");
         if (lay & kLayoutWindow) p.gs_window = true;
         else if (lay & kLayoutNoWindow) p.gs_window = false;
         else if (e) p.gs_window = std::string(e) != "0";
-        else p.gs_window = m < (use_smem ? 15 : 32) * n;
+        else p.gs_window = m < (use_smem ? 15 : 32) * n && 25 * m < n * n;
     }
     p.claim = run_work(g);
     if (defer_to_batch(g, cfg, out, use_smem, p)) return false;
