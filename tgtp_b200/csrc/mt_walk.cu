@@ -36,7 +36,6 @@ namespace {
 constexpr uint32_t kMtWords = 624;
 constexpr uint32_t kMtShift = 397;
 constexpr int kMtThreads = 1024;
-constexpr int kMtWarps = kMtThreads / 32;
 constexpr int kSlots = 4;       // walks (bouquets) in flight per lane (8 lanes)
 constexpr int kSeedAhead = 4;   // sources a warp seeds at once
 constexpr uint32_t kMtHot = 12288;
@@ -111,7 +110,7 @@ mt_walk_kernel(const PackedWalk g, const uint32_t* __restrict__ adjp, uint64_t n
     extern __shared__ __align__(16) uint32_t s_mt[];
     const uint32_t lane = threadIdx.x & 31;
     uint32_t* ring = s_mt + size_t(threadIdx.x >> 5) * 2 * kMtWords;
-    uint2* s_cls = reinterpret_cast<uint2*>(s_mt + size_t(kMtWarps) * 2 * kMtWords);
+    uint2* s_cls = reinterpret_cast<uint2*>(s_mt + size_t(blockDim.x >> 5) * 2 * kMtWords);
     uint32_t* s_inv = reinterpret_cast<uint32_t*>(s_cls + (PACKED ? g.ncls : 0u));
     uint32_t* s_cnt = s_inv + (PACKED ? g.ncls : 0u);
     if (PACKED)
@@ -245,16 +244,19 @@ void mt_walk_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, bool simd,
     auto kern = simd ? (packed ? mt_walk_kernel<true, true> : mt_walk_kernel<true, false>)
                      : (packed ? mt_walk_kernel<false, true> : mt_walk_kernel<false, false>);
     // shared memory: the rings, the classes (12 bytes each), and counters in what is left of it
-    const size_t fixed = size_t(kMtWarps) * 2 * kMtWords * sizeof(uint32_t) + size_t(w.ncls) * 12;
+    // Warps per block: a source each on graphs too small for 32 on every SM (n = 1,000, depth 700, 8
+    // walks: 3.36 ms with 32 on each of 32 SMs, 2.39 with seven on each of 143).
+    const int warps = int(std::min<uint64_t>(kMtThreads / 32, (g->n + g->num_sms - 1) / g->num_sms));
+    const size_t fixed = size_t(warps) * 2 * kMtWords * sizeof(uint32_t) + size_t(w.ncls) * 12;
     const size_t room = size_t(227) * 1024 - fixed;
     const uint32_t hot = uint32_t(std::min<uint64_t>({g->n, kMtHot, room / sizeof(uint32_t)}));
     const size_t smem = fixed + sizeof(uint32_t) * hot;
-    const int per_sm = std::max(1, blocks_per_sm(reinterpret_cast<const void*>(kern), kMtThreads, smem));
-    uint64_t blocks = std::min<uint64_t>(uint64_t(g->num_sms) * per_sm, (g->n + kMtWarps - 1) / kMtWarps);
-    // the generators' states (320 KB a block); fewer blocks where the device has no room for all
+    const int per_sm = std::max(1, blocks_per_sm(reinterpret_cast<const void*>(kern), warps * 32, smem));
+    uint64_t blocks = std::min<uint64_t>(uint64_t(g->num_sms) * per_sm, (g->n + warps - 1) / warps);
+    // the generators' states (10 KB a warp); fewer blocks where the device has no room for all
     for (bool there = false; !there;) {
         try {
-            g->mt_seeds.reserve(blocks * kMtWarps * kSeedAhead * kMtWords * sizeof(uint32_t));
+            g->mt_seeds.reserve(blocks * warps * kSeedAhead * kMtWords * sizeof(uint32_t));
             there = true;
         } catch (const Error& e) {
             if (e.code != TGTP_ERR_OUT_OF_MEMORY || blocks <= 1) throw;
@@ -263,7 +265,7 @@ void mt_walk_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, bool simd,
     }
     {
         ScopedKernel k(g->prof, s, "mt_walk");
-        kern<<<unsigned(blocks), kMtThreads, smem, s>>>(w, g->saba_adj.as<uint32_t>(), g->n, depth, n_walks,
+        kern<<<unsigned(blocks), unsigned(warps * 32), smem, s>>>(w, g->saba_adj.as<uint32_t>(), g->n, depth, n_walks,
                                                         cnt, hot, g->mt_seeds.as<uint32_t>());
         TGTP_LAUNCH_CHECK("mt_walk_kernel");
     }
