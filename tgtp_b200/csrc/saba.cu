@@ -640,8 +640,8 @@ void saba_launch(tgtp_graph* g, uint32_t depth, uint32_t bps, uint32_t grid_step
     const int threads = packed ? kPackedThreads : kSabaThreads;
     const int per_sm = std::max(1, blocks_per_sm(kern, threads, smem));
     uint64_t blocks = uint64_t(g->num_sms) * per_sm;
-    const uint64_t need = (total + 4 * WPL - 1) / (4 * WPL) / (threads / 32) + 1;
-    if (blocks > need) blocks = need;
+    const uint64_t steps = (total + 4 * WPL - 1) / (4 * WPL);
+    blocks = std::min(blocks, std::max<uint64_t>(steps / (threads / 32) + 1, std::min<uint64_t>(steps, g->num_sms)));
     ScopedKernel k(g->prof, s, "saba_walk");
     if (packed) {
         saba_walk_packed_kernel<WPL><<<unsigned(blocks), unsigned(threads), smem, s>>>(
