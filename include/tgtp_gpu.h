@@ -57,7 +57,10 @@ typedef enum {
     /* Every float of the reference held in double (needs F64 vectors). */
     TGTP_PRECISION_FP64 = 1,
     /* FP32 residuals, lane-parallel compensated FP32 eigen projections over F32 or BF16 vectors,
-     * FP64 tau bounds, stop test and per-edge score accumulation; reductions in parallel order. */
+     * FP64 tau bounds, stop test and per-edge score accumulation; reductions in parallel order.
+     * What a vertex is sent in one push round is added up modulo 4: it passes 4 at hubs of many
+     * low-degree neighbours, whose scores then carry an error of their own (on a sparse power-law
+     * graph 8e-4 on average next to such rows, 3.6e-4 in the FP64 form, at epsilon = 0.005). */
     TGTP_PRECISION_MIXED = 2
 } tgtp_precision;
 
@@ -152,9 +155,12 @@ tgtp_status tgtp_last_taus(tgtp_graph* g, int32_t* host_taus);
 
 /* Times the candidate layouts of the source kernels (per-source residual vectors in shared memory
  * or in HBM; for the FP32 and FP64 forms the windowed or the one-vertex push; for the mixed form
- * also the one-source and the multi-source block push, the latter at four frontier thresholds) for cfg's precision form on this graph, `trials` runs each after a
- * warm-up, and keeps the fastest on the handle for later runs of that form.  Scores are identical
- * under every layout.  *layout (may be NULL) receives the choice: 0x100 bit = shared memory, low
+ * also the one-source and the multi-source block push, the latter at four frontier thresholds) for
+ * cfg's precision form on this graph, `trials` runs each after a warm-up, and keeps the fastest on the
+ * handle for later runs of that form.  Scores are identical under every layout, but for this: the
+ * mixed form's block pushes leave out vertices whose residual has rounded to 0 (below 2^-62; on grids
+ * after 31 rounds), so there a source may stop at another round than in the per-source kernel.
+ * *layout (may be NULL) receives the choice: 0x100 bit = shared memory, low
  * byte = nominal warps per block, 0x200 = block push, bits 12-13 = its compaction threshold (a round is
  * compacted to the rows next to the live ones when their degree sum is below m / 4, m / 2,
  * m / 16, or never); for the FP32 and FP64 forms 0x400 = the windowed sequential push, 0x800 =
@@ -240,8 +246,8 @@ tgtp_status saba_count_static(const uint32_t* device_idx, const uint32_t* device
  * every slot iterates until its residual norm is at most tol * ||e_u - e_v|| (TGTP_ERR_TIMEOUT when
  * max_iter iterations do not get there).  host_iterations (may be NULL) receives the iteration count
  * of each batch of 32 slots (ceil(count / 32) entries).  Synchronous; scratch is allocated per call
- * (four blocks of n x 32 doubles per batch;
- * several batches run side by side while their blocks stay within 80 MB). */
+ * (four blocks of n x 32 doubles per batch; several batches run side by side while their blocks stay
+ * within 80 MB). */
 tgtp_status tgtp_exact_sc_slots(tgtp_graph* g, const uint32_t* host_slots, uint32_t count,
                                 double tol, uint32_t max_iter, double* host_resistance,
                                 uint32_t* host_iterations);

@@ -51,8 +51,6 @@ namespace {
 
 constexpr int kTauThreads = 32;      // FP32 form's tau: one warp per block
 constexpr int kTauBlocks = 20;       // per SM: 96 registers (16 blocks: 78 us for 70; 24 spill: 70)
-// scratch counted beside a residual vector where the size rule of the mixed form's pushes is stated
-constexpr size_t kAccBytes = 1280;
 constexpr int kTauTableRows = 64;    // rows of the eigen_t_1 power table (api.cu)
 constexpr uint64_t kMaxWalks = 0xffffffffull;  // nr beyond the 32-bit grid is not supported
 
@@ -390,8 +388,13 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 // Residual arithmetic of the mixed form's push: the residual a vertex u receives in a round is the
 // exact integer sum of its frontier neighbours' residuals in 2^-62 fixed point, divided (rounding
 // down) by deg(u), then rounded once to FP32.  The sum does not depend on the order of the
-// additions, so the per-warp push and the multi-source block push give the same bits.  Residuals
-// never exceed 1 and a round conserves their total, so no sum exceeds 2^62.
+// additions, so the per-source push and the block pushes add up the same bits.
+// Sums are 64 bits wide, so they are taken modulo 4.  A round conserves the sum of deg(u) r(u), not
+// that of r(u): a vertex whose neighbours have few others (a hub with leaves) can be sent up to the
+// source's degree, and where that passes 4 its residual becomes (sum mod 4) / deg(u).  All pushes do
+// so alike and the scores of this form are defined with it; the FP32 and FP64 forms have no such
+// limit.  Sparse Chung-Lu graph (n = 25,860, exponent 2.1): 723 sources are sent more than 4 in round
+// 2; scores next to them are 8e-4 off the exact values on average, 3.6e-4 in the FP64 form (eps = 0.005).
 constexpr unsigned long long kFixOne = 1ull << 62;
 __device__ __forceinline__ unsigned long long to_fixed(float r) {
     return __float2ull_rn(__fmul_rn(r, 0x1p62f));
@@ -1030,12 +1033,6 @@ struct WalkItem {
     unsigned long long nr;
 };
 
-// The final residual vector (n contiguous floats) of list entry list_base + slot after the block
-// push: with finals, a column of its 32-source CTA's spare block (finals[cta] tells which of the
-// two blocks is the spare), else the entry's own.
-__device__ __forceinline__ const float* pre_column(const float* cols, const uint32_t* finals,
-                                                   uint32_t slot, uint32_t n);
-
 // Outcome of the push of one listed source in push_block_kernel or push_shared_kernel.
 struct PrePush {
     int ell;           // rounds pushed
@@ -1098,9 +1095,14 @@ template <> __device__ __forceinline__ double from_ord<double>(unsigned long lon
 // and divides by deg(u).  The same pass accumulates each column's frontier statistics (degree sum,
 // max, min, size of the support), so the stop test of src/aesc.h:483-502 needs no further pass.
 // Columns whose source has stopped are carried over unchanged, so when the last one stops every
-// column holds its source's final residual vector; the edge bound, chi and walks of those sources
-// then run in source_kernel (PrePush mode), which copies the column into its own residual vector.
+// column holds its source's final residual vector; the edge bound, chi and walk counts of those
+// sources then run in mixed_source_kernel<kColumn>, which reads the column in place, and their walks
+// in kernels of their own.
 constexpr int kBlockCols = 32;
+
+// The final residual vector (n contiguous floats) of list entry list_base + slot after a block push:
+// with finals, a column of its 32-source CTA's spare block (finals[cta] tells which of the two
+// blocks is the spare), else the entry's own.
 __device__ __forceinline__ const float* pre_column(const float* cols, const uint32_t* finals,
                                                    uint32_t slot, uint32_t n) {
     if (!finals) return cols + size_t(slot) * n;
@@ -1992,12 +1994,12 @@ void launch_finish(tgtp_graph* g, float* out) {
 }  // namespace
 
 // ---- batched runs: one persistent source kernel over the rows of many graphs --------------------
-// While a batch is captured (batch.cu), each run_form of a graph whose per-source stage runs as
-// per-warp pushes stops after its tau kernels and leaves that stage and the symmetrisation to the
+// While a batch is captured (batch.cu), each run_form of a graph whose per-source stage is one kernel
+// (no block push) stops after its tau kernels and leaves that stage and the symmetrisation to the
 // batch: the batch joins every graph's branch, launches one persistent source kernel per
 // (arithmetic form, residual-vector tier) over the listed rows of all its graphs, then launches
 // each graph's finish kernel on the graph's own stream again.  The graphs of a group share one
-// per-warp scratch laid out for the group's largest graph.
+// per-block scratch laid out for the group's largest graph.
 struct BatchEntry {
     tgtp_graph* g;
     float* out;
@@ -2032,10 +2034,11 @@ bool defer_to_batch(tgtp_graph* g, const tgtp_config& cfg, float* out, bool smem
     return true;
 }
 
-// Whether a warp's FP32 residual vector and flags (the mixed form's) exceed the 112 KB of the
-// shared-memory tier the mixed form's pushes had per warp; the learned push choice keeps to it.
-bool mixed_beyond_smem(uint64_t n) {
-    return ((n * 4 + 15) & ~uint64_t(15)) + ((n + 15) & ~uint64_t(15)) + kAccBytes > uint64_t(112) * 1024;
+// Graphs of more than 22,680 vertices (five bytes a vertex and 1,280 beyond 112 KB, what a warp had
+// for its vector when pushes were made by single warps): those whose mixed push is chosen by
+// measurement, see learn_push_hint.
+bool mixed_push_chosen(uint64_t n) {
+    return ((n * 4 + 15) & ~uint64_t(15)) + ((n + 15) & ~uint64_t(15)) + 1280 > uint64_t(112) * 1024;
 }
 void poll_push_hint(tgtp_graph* g);
 void post_push_hint(tgtp_graph* g, int key, double eps);
@@ -2050,19 +2053,17 @@ MixedPlan plan_mixed(tgtp_graph* g, const tgtp_config& cfg) {
     const int key = form_key(cfg);
     MixedPlan p;
     poll_push_hint(g);
-    // mixed form, residual vectors too large for shared memory: multi-source push in waves of
-    // block_ctas x kBlockCols listed sources (each wave has its own claim counter)
-    // The block push gives the same bits as the per-warp push (fixed-point residual sums), so the
-    // choice is only about speed: the handle's tuned layout, else TGTP_MIXED_BLOCK, else what the
-    // last completed mixed run on this graph at this epsilon measured (push_hint), else the block
-    // push for
-    // vectors beyond shared memory at eps <= 0.01 (deep pushes: the block push was the faster one
-    // on every such graph measured) and the per-warp push otherwise.
+    // A block push (the push alone, in waves of listed sources with a claim counter each, then the
+    // other stages) or the per-source kernel for all of it: the handle's tuned layout, else
+    // TGTP_MIXED_BLOCK, else what the last completed mixed run on this graph at this epsilon showed
+    // (push_hint), else the block push on graphs of more than 22,680 vertices at eps <= 0.01.  Scores
+    // are the same while no residual rounds to 0 (see round_with_zeros).  learn_push_hint has the
+    // figures: the line is the former kernels'.
     if (g->src_layout[key]) p.block_mode = (g->src_layout[key] & kLayoutBlock) != 0;
     else if (const char* e = std::getenv("TGTP_MIXED_BLOCK")) p.block_mode = std::atoi(e) != 0;
     else if (g->push_hint[key] && g->push_hint_eps[key] == cfg.epsilon)
         p.block_mode = g->push_hint[key] == 2;
-    else p.block_mode = mixed_beyond_smem(n) && cfg.epsilon <= 0.01;
+    else p.block_mode = mixed_push_chosen(n) && cfg.epsilon <= 0.01;
     // Graphs whose sums fit in shared memory push one source per block (push_shared_kernel), all
     // listed sources in waves of at most 4 GiB of residual vectors, or of half the device memory free
     // now (beside what the columns already hold) where that is less, but not below what the 32-source
@@ -2683,9 +2684,9 @@ void run_form(tgtp_graph* g, const tgtp_config& cfg, float* out) {
         const Real* vec = (const Real*)g->vec_f32.ptr;
         const Real* etab = (const Real*)g->etab_f.ptr;
         const Real eps_half = Real(cfg.epsilon / 2.0);
-        // the largest omega taken: 32 bytes per index beside 16.5 KB
+        // the largest omega this form takes (6,736); the kernel itself keeps 32 indices at a time
         if (32 * size_t(omega) + 4 * 32 * 33 * sizeof(Real) > size_t(227) * 1024)
-            fail(TGTP_ERR_UNSUPPORTED, "omega too large for the tau kernel tile");
+            fail(TGTP_ERR_UNSUPPORTED, "omega too large for the FP32 form");
         const unsigned tau_blocks = unsigned(std::max<uint64_t>(
             1, std::min<uint64_t>((g->num_forward + kTauEdges - 1) / kTauEdges, uint64_t(1) << 30)));
         ScopedKernel k(g->prof, s, "tau");
@@ -2882,18 +2883,26 @@ void aesc_check_flags(tgtp_graph* g) {
 
 namespace {
 
-// Mixed form: a dense round of the block push reads every slot once per 32 sources, about 40
-// times cheaper per slot than a per-warp push reads a frontier entry (scattered residual updates in
-// HBM).  So the block push pays off when a round's frontier averages more than m / 40 traversals
-// -- for graphs whose residual vectors do not fit in shared memory (smaller ones push per warp in
-// shared memory).  Measured on the sparse Chung-Lu graph (n = 25,860) at eps 0.05 / 0.01 / 0.005,
-// R-MAT (n = 143,522) at 0.05 / 0.01 and Chung-Lu (n = 199,772) at 0.05 / 0.01 / 0.005, the rule
-// picks the faster push every time (or one within 3 %).
+// Mixed form, graphs of more than 22,680 vertices: the block push when a run's rounds average more than
+// m / 40 traversals.  That line was drawn where a dense round of the 32-source push, which reads
+// every slot once per 32 sources, became cheaper than pushes made by single warps.  With the present
+// kernels, ms, per-source kernel / block push at eps = 0.05, 0.01, 0.005 (Chung-Lu, neighbours and
+// exponent; * where the rule takes the block push):
+//   one-source block push, up to 27,900 vertices
+//     9.3, 2.1   n = 9,000 4.2/3.2, 11/8.3, 16/11; 16,000 23/11, 60/30, 81/40; 20,000 36/17, 100/47, 135/63;
+//                23,000 44/21*, 128/58*, 178/78*; 25,860 55/24*, 160/68*, 222/92*
+//     20, 2.3    16,000 3.7/3.1, 11/8.3, 17/13; 27,800 4.1/6.8, 24/18*, 48/31*
+//   32-source block push
+//     9.3, 2.1   28,500 62/143*, 196/253*, 272/307*; 60,000 355/710*, 1,068/1,258*
+//     20, 2.3    28,500 4.4/36, 25/70*, 50/83*; 60,000 16/127, 99/256*; 200,000 137/1,125
+//     R-MAT, n = 90,000   101/808, 717/1,578*
+// So up to 27,900 vertices the block push is the faster one from about 9,000 on unless the pushes are
+// shallow, and above that the per-source kernel everywhere; the rule is still the former one.
 void learn_push_hint(tgtp_graph* g, int key, double eps, unsigned long long rounds,
                      unsigned long long traversals) {
     if (key < 2 || rounds == 0) return;
     const double per_round = double(traversals) / double(rounds);
-    g->push_hint[key] = (mixed_beyond_smem(g->n) && per_round * 40.0 > double(g->m)) ? 2 : 1;
+    g->push_hint[key] = (mixed_push_chosen(g->n) && per_round * 40.0 > double(g->m)) ? 2 : 1;
     g->push_hint_eps[key] = eps;
 }
 
@@ -2916,11 +2925,10 @@ void poll_push_hint(tgtp_graph* g) {
     g->hint_key = -1;
 }
 
-// After a mixed run on the handle's stream (not while capturing) on a graph whose vectors exceed
-// shared memory (smaller ones always push per warp): copy its counters to pinned memory and
-// record the event poll_push_hint looks at.
+// After a mixed run on the handle's stream (not while capturing) on a graph whose push is chosen by
+// measurement: copy its counters to pinned memory and record the event poll_push_hint looks at.
 void post_push_hint(tgtp_graph* g, int key, double eps) {
-    if (!mixed_beyond_smem(g->n)) return;
+    if (!mixed_push_chosen(g->n)) return;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     TGTP_CUDA(cudaStreamIsCapturing(g->stream, &cs));
     if (cs != cudaStreamCaptureStatusNone) return;

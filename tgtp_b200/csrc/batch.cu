@@ -3,8 +3,8 @@
 // A batch is built once: every run is executed once on its graph handle (which sizes all of the
 // handle's buffers and weight tables, and optionally times the candidate source-kernel layouts and
 // keeps the fastest), then all runs are captured from one origin stream that forks to each handle's
-// stream.  Each graph's branch runs its tau kernels; the per-source stage of every run that pushes
-// per warp is left to the batch (aesc.cu, BatchPlan): the branches join, one persistent source
+// stream.  Each graph's branch runs its tau kernels; the per-source stage of every run without a
+// block push is left to the batch (aesc.cu, BatchPlan): the branches join, one persistent source
 // kernel per (arithmetic form, residual-vector tier) works through the listed rows of all those
 // graphs as one queue of (graph, row) items, so the rows of small graphs fill the SMs that a large
 // graph leaves idle, and the branches fork again for each graph's symmetrisation.  Runs whose push

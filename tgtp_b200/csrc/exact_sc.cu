@@ -23,9 +23,9 @@
 // What bounds a pass is the latency of the gathered 256-byte rows, not their bytes (the blocks of a
 // batch stay in L2 up to n of about 10^5), so the work is cut to keep loads in flight: a warp has
 // eight neighbour rows in flight, rows of more than kSeg slots are cut into segments for different
-// warps (a hub row held the whole pass before), and several batches run side by side while their
-// blocks fit in L2 together.  256 slots of the Chung-Lu graph with n = 25,860, m = 239,944: 373 ms
-// with one batch at a time, whole rows per warp and one neighbour row in flight, 9.8 ms now.
+// warps (a hub row would hold the whole pass), and several batches run side by side while their
+// blocks fit in L2 together.  256 slots of the Chung-Lu graph with n = 25,860, m = 239,944: 9.7 ms;
+// with one batch at a time, whole rows per warp and one neighbour row in flight 373.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -44,8 +44,8 @@ constexpr int kScWarps = kScThreads / 32;
 // with 256.
 constexpr uint32_t kSeg = 64;
 // Bytes of the blocks (x, r, p, lp) of the batches that run side by side, and their largest number
-// (their sums and flags).  n = 25,860 / 4,039, 256 slots: one batch after another 16.3 / 4.4 ms,
-// 40 MB 16.4 / 1.2, 80 MB 10.2 / 1.2, 160 MB (beyond L2) 9.8 / 1.2.
+// (their sums and flags).  n = 25,860 / 4,039, 256 slots: one batch after another 14.6 / 3.7 ms,
+// 40 MB 14.6 / 1.13, 80 MB 9.7 / 1.13, 160 MB (beyond L2) 9.5 / 1.13.
 constexpr uint64_t kSideBySide = uint64_t(80) << 20;
 constexpr uint64_t kMostSide = 256;
 constexpr int kCheck = 8;       // iterations between two looks at the residuals from the host

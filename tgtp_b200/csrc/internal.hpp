@@ -279,7 +279,7 @@ constexpr int kRunStatSlots = 32;
 void aesc_read_stats(tgtp_graph* g, unsigned long long* st);
 void graph_prepare(tgtp_graph* g);
 // Batched runs (aesc.cu): while collection is on for this thread (batch_plan_collect(plan)),
-// aesc_run leaves the per-source stage and the symmetrisation of per-warp-push runs to the plan;
+// aesc_run leaves the per-source stage and the symmetrisation of runs without a block push to the plan;
 // batch_plan_launch then runs one persistent source kernel per (form, tier) group over all the
 // deferred graphs' rows on stream s, and batch_plan_finish each deferred graph's finish kernel on
 // the graph's own stream.  batch_plan_collect(nullptr) ends collection.

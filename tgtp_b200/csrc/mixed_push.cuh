@@ -50,8 +50,8 @@ __device__ __forceinline__ uint32_t find_segment(const uint32_t* offs, uint32_t 
 // Concatenates the rows of up to C vertices: thread i < cnt passes vertex i's row start, its
 // degree (at least 1) and a value.  Every entry is loaded, load(slot, whether there is an entry), and
 // then used, use(loaded, value of its vertex, the vertex's index in the chunk, whether there is an
-// entry), by all lanes of a warp together, on consecutive entries.  All threads of the block call it; the scratch is free again after
-// the caller's next __syncthreads.
+// entry), by all lanes of a warp together, on consecutive entries.  All threads of the block call it;
+// the scratch is free again after the caller's next __syncthreads.
 template <int C, class Load, class Use>
 __device__ __forceinline__ uint32_t for_entries(ChunkScratchOf<C>& s, uint32_t cnt, uint32_t beg, uint32_t deg,
                                                 unsigned long long val, Load load, Use use) {
