@@ -106,13 +106,13 @@ template <bool SIMD, bool PACKED>
 __global__ void __launch_bounds__(kMtThreads)
 mt_walk_kernel(const PackedWalk g, const uint32_t* __restrict__ adjp, uint64_t n, uint32_t depth,
                uint32_t n_walks, WalkCounters cnt, uint32_t hot, uint32_t* seeds) {
-    // per warp the ring, then the class table (8 bytes a class), its inverses, the counters
+    // the class table (8 bytes a class), its inverses, the counters, then per warp the ring
     extern __shared__ __align__(16) uint32_t s_mt[];
     const uint32_t lane = threadIdx.x & 31;
-    uint32_t* ring = s_mt + size_t(threadIdx.x >> 5) * 2 * kMtWords;
-    uint2* s_cls = reinterpret_cast<uint2*>(s_mt + size_t(blockDim.x >> 5) * 2 * kMtWords);
+    uint2* s_cls = reinterpret_cast<uint2*>(s_mt);
     uint32_t* s_inv = reinterpret_cast<uint32_t*>(s_cls + (PACKED ? g.ncls : 0u));
     uint32_t* s_cnt = s_inv + (PACKED ? g.ncls : 0u);
+    uint32_t* ring = s_mt + (((PACKED ? 3u * g.ncls : 0u) + hot + 3u) & ~3u) + size_t(threadIdx.x >> 5) * 2 * kMtWords;
     if (PACKED)
         for (uint32_t i = threadIdx.x; i < g.ncls; i += blockDim.x) {
             s_cls[i] = __ldg(g.classes + i);
@@ -247,10 +247,10 @@ void mt_walk_run(tgtp_graph* g, uint32_t depth, uint32_t n_walks, bool simd,
     // Warps per block: a source each on graphs too small for 32 on every SM (n = 1,000, depth 700, 8
     // walks: 3.36 ms with 32 on each of 32 SMs, 2.39 with seven on each of 143).
     const int warps = int(std::min<uint64_t>(kMtThreads / 32, (g->n + g->num_sms - 1) / g->num_sms));
-    const size_t fixed = size_t(warps) * 2 * kMtWords * sizeof(uint32_t) + size_t(w.ncls) * 12;
-    const size_t room = size_t(227) * 1024 - fixed;
-    const uint32_t hot = uint32_t(std::min<uint64_t>({g->n, kMtHot, room / sizeof(uint32_t)}));
-    const size_t smem = fixed + sizeof(uint32_t) * hot;
+    const size_t rings = size_t(warps) * 2 * kMtWords;  // words, as are the next two
+    const size_t room = size_t(227) * 256 - rings - 3 * size_t(w.ncls) - 4;
+    const uint32_t hot = uint32_t(std::min<uint64_t>({g->n, kMtHot, room}));
+    const size_t smem = sizeof(uint32_t) * (((3 * size_t(w.ncls) + hot + 3) & ~size_t(3)) + rings);
     const int per_sm = std::max(1, blocks_per_sm(reinterpret_cast<const void*>(kern), warps * 32, smem));
     uint64_t blocks = std::min<uint64_t>(uint64_t(g->num_sms) * per_sm, (g->n + warps - 1) / warps);
     // the generators' states (10 KB a warp); fewer blocks where the device has no room for all
