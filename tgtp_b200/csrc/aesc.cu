@@ -2144,7 +2144,10 @@ MixedLayout mixed_layout(int mode, uint64_t n, uint64_t max_degree, uint64_t row
     // eps = 0.05, ms: 128 166 / 12.6, 256 143.9 / 11.6, 512 143.5 / 10.9, 1,024 158 / 15.2 (fewer
     // sources at once wait for each other's barriers, more push each other's words out of L2)
     if (mode == kShared)
-        l.threads = l.smem > size_t(113) * 1024 ? 1024u : (l.smem > size_t(56) * 1024 ? 512u : (l.smem > size_t(28) * 1024 ? 256u : 128u));
+        l.threads = l.smem > size_t(113) * 1024  ? 1024u
+                    : l.smem > size_t(56) * 1024 ? 512u
+                    : l.smem > size_t(28) * 1024 ? 256u
+                                                 : 128u;
     else
         l.threads = mode == kGlobal ? 512u : 256u;
     const int per_sm = blocks_per_sm(mixed_kernel<Pack>(mode), int(l.threads), l.smem);
@@ -2230,8 +2233,8 @@ bool run_mixed(tgtp_graph* g, const tgtp_config& cfg, float* out, const RowMarks
         p.claim = work;
         if (defer_to_batch(g, cfg, out, mode == kShared, p)) return false;
     }
-    p.clean = clean_marks(g, uint64_t(key) | (uint64_t(mode) << 8) | (uint64_t(lay.bit_bytes != 0) << 16) | (uint64_t(1) << 63),
-                          lay.blocks, mode == kGlobal);
+    const uint64_t carving = uint64_t(key) | (uint64_t(mode) << 8) | (uint64_t(lay.bit_bytes != 0) << 16);
+    p.clean = clean_marks(g, carving | (uint64_t(1) << 63), lay.blocks, mode == kGlobal);
     if (!mp.block_mode) {
         pk.g[0] = p;
         ScopedKernel k(g->prof, s, "source");

@@ -11,8 +11,8 @@
 // block's threads too: with one warp per source the largest source of the 4,039-vertex graph (2,055
 // neighbours) alone took as long as the whole kernel.  Against one source per warp (four warps per
 // SM in shared memory, twelve with their vectors in HBM), ms: 4,039-vertex graph, eps = 0.005,
-// 1.92 -> 0.57; Chung-Lu n = 200,000, m = 4e6, eps = 0.05, 287 -> 139; 16 graphs of 1,000-3,500
-// vertices as one batch 9.1 -> 2.7.
+// 1.92 -> 0.49; Chung-Lu n = 200,000, m = 4e6, eps = 0.05, 287 -> 133; 16 graphs of 1,000-3,500
+// vertices as one batch 9.1 -> 2.25.
 
 enum MixedMode { kShared, kGlobal, kColumn };
 constexpr uint32_t kSetMax = 64;              // members of the top-gamma set compared pair by pair
@@ -249,7 +249,9 @@ __device__ __forceinline__ uint32_t drain_bits(PushScratch& s, uint32_t* bits, u
 // the largest degree in 2^-62; the other rounds (far vertices of grids and the like, after 30 rounds
 // and more) come here, where the neighbours of the frontier's zeros have bits of their own (all clear
 // between rounds).  The block pushes leave vertices with residual 0 out, so where there are some a
-// source may stop at another round than here.
+// source may stop at another round than here.  A function of its own, because the other rounds pay
+// for code around them: 4,039-vertex graph, eps = 0.005, 484 us without it, 490 so, 487 to 503 with the
+// marking inside take_residuals or the push; batch of 16 graphs 2.18 ms, 2.21, 2.23 to 2.33.
 __device__ __noinline__ void round_with_zeros(PushScratch& s, uint32_t* lo, uint32_t* hi, uint32_t* bits,
                                               const uint32_t* __restrict__ idx, const uint32_t* __restrict__ adj,
                                               const double* __restrict__ dinv, uint32_t n, const Frontier& f,
@@ -304,7 +306,9 @@ __global__ void __launch_bounds__(1024, 1) mixed_source_kernel(const Pack pk) {
     uint32_t* const hi = smem_words + pad;  // kShared
     const uint32_t bwords = (sn + 31u) / 32u;
     const bool bits_here = MODE == kGlobal && !p0.gbits;
-    uint32_t* const gbits = MODE == kShared || (MODE == kGlobal && !bits_here) ? p0.gbits + size_t(blockIdx.x) * bwords : nullptr;
+    uint32_t* const gbits = MODE == kShared || (MODE == kGlobal && !bits_here)
+                                ? p0.gbits + size_t(blockIdx.x) * bwords
+                                : nullptr;
     unsigned long long* const sums = MODE == kGlobal ? p0.sums + size_t(blockIdx.x) * sn : nullptr;
     uint32_t* const touched = MODE == kGlobal ? p0.touched + size_t(blockIdx.x) * sn : nullptr;
     const Frontier f{p0.lists + size_t(blockIdx.x) * sn, sn};
